@@ -79,12 +79,15 @@ __device__ __forceinline__ float minmod_d(float a, float b)
     const float m = fmaxf(0.0f, fminf(fabsf(a), __uint_as_float(__float_as_uint(b) ^ sa)));
     return __uint_as_float(__float_as_uint(m) | sa);
 }
+// FP64: minimum, maximum and signs on the bit patterns (section "FP64
+// arithmetic for a narrow pipe" below)
 __device__ __forceinline__ double minmod_d(double a, double b)
 {
-    const unsigned long long sa = (unsigned long long)__double_as_longlong(a) & 0x8000000000000000ull;
-    const double bs = __longlong_as_double((long long)((unsigned long long)__double_as_longlong(b) ^ sa));
-    const double m = fmax(0.0, fmin(fabs(a), bs));
-    return __longlong_as_double((long long)((unsigned long long)__double_as_longlong(m) | sa));
+    const long long ia = __double_as_longlong(a);
+    const long long sa = ia & (long long)0x8000000000000000ull;
+    const long long ma = ia & 0x7fffffffffffffffll, bs = __double_as_longlong(b) ^ sa;
+    const long long m = (ma < bs) ? ma : bs;   // negative: opposite signs
+    return __longlong_as_double(((m < 0) ? 0ll : m) | sa);
 }
 
 // left / right face values of a cell from its three-point stencil; the
@@ -92,14 +95,91 @@ __device__ __forceinline__ double minmod_d(double a, double b)
 template <typename R>
 __device__ __forceinline__ void recon_pair(R tm, R t0, R tp, R& left, R& right)
 {
-    R d = minmod_d(t0 - tm, tp - t0) * R(0.5);
-    left = t0 - d;
-    right = t0 + d;
+    if constexpr (sizeof(R) == 8) {
+        // half the slope in the multiply-add: one FP64 operation per value
+        const R m = minmod_d(t0 - tm, tp - t0);
+        left = fma(m, R(-0.5), t0);
+        right = fma(m, R(0.5), t0);
+    } else {
+        R d = minmod_d(t0 - tm, tp - t0) * R(0.5);
+        left = t0 - d;
+        right = t0 + d;
+    }
 }
 
+// ------------------------------------------------------------------ FP64 arithmetic for a narrow pipe
+// GB300 issues one FP64 warp instruction per SM every 17-20 cycles (measured:
+// fma 17, add and mul 20, a compare-and-select 20, fmin 40; each waits 92
+// cycles for its operands) and four instructions of every other kind per
+// cycle.  The FP64 kernels are therefore bound by the count of their FP64
+// operations, and what is not a sum or a product goes elsewhere: signs,
+// comparisons, minima and maxima are integer operations on the bit patterns
+// (64-bit integer minimum: 0.4 cycles), and reciprocals and sound speeds
+// start from the approximation instructions (20 bits, 2 cycles) and take one
+// third-order step of the binomial series (Householder's iteration) instead
+// of a division (150 cycles) and a square root (150).  Written with explicit
+// roundings (fma, __dadd_rn, __dmul_rn) so that every kernel that inlines
+// them gives the same bits.
+namespace d64 {
+constexpr long long kSign = (long long)0x8000000000000000ull;
+__device__ __forceinline__ long long bits(double a) { return __double_as_longlong(a); }
+__device__ __forceinline__ double from(long long a) { return __longlong_as_double(a); }
+__device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
+__device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double abs(double a) { return from(bits(a) & ~kSign); }
+__device__ __forceinline__ bool neg(double a) { return __double2hiint(a) < 0; }   // the sign bit
+__device__ __forceinline__ double sel(bool c, double a, double b) { return from(c ? bits(a) : bits(b)); }
+// an integer that orders as the numbers do (no NaN)
+__device__ __forceinline__ long long key(double a)
+{
+    const long long i = bits(a);
+    return i ^ ((i >> 63) & 0x7fffffffffffffffll);
+}
+__device__ __forceinline__ double min(double a, double b) { return sel(key(a) < key(b), a, b); }
+__device__ __forceinline__ double max(double a, double b) { return sel(key(a) < key(b), b, a); }
+// the larger magnitude of two numbers, and the larger of two numbers >= 0
+__device__ __forceinline__ double max_abs(double a, double b)
+{
+    const long long x = bits(a) & ~kSign, y = bits(b) & ~kSign;
+    return from(x < y ? y : x);
+}
+__device__ __forceinline__ double max_pos(double a, double b) { return from(bits(a) < bits(b) ? bits(b) : bits(a)); }
+__device__ __forceinline__ bool finite(double a) { return (__double2hiint(a) & 0x7ff00000) != 0x7ff00000; }
+// The ranges the short forms take: positive with 2^-150 <= a < 2^150, and
+// |a| < 2^150 (so that no product or quotient of theirs leaves the normal
+// range); NaN and infinities are outside.
+constexpr int kLo = (1023 - 150) << 20, kHi = (1023 + 150) << 20;
+__device__ __forceinline__ bool tame_pos(double a) { return (unsigned)(__double2hiint(a) - kLo) < (unsigned)(kHi - kLo); }
+__device__ __forceinline__ bool tame(double a) { return (__double2hiint(a) & 0x7fffffff) < kHi; }
+
+// 1/x of a normal number well inside the range: with y0 = (1 + d)/x and
+// e = 1 - x y0, 1/x = y0 (1 + e + e^2 + ...), cut after e^2 (|e| < 2^-19)
+__device__ __forceinline__ double rcp(double x)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
+// sqrt(a / r) of tame a and r as a (a r)^(-1/2): with y0 the approximate
+// inverse root of x = a r and e = 1 - x y0^2, x^(-1/2) = y0 (1 + e/2 +
+// 3 e^2/8 + ...), cut after e^2
+__device__ __forceinline__ double sqrt_ratio(double a, double r)
+{
+    const double x = mul(a, r);
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-mul(x, y), y, 1.0);
+    const double w = mul(a, y);
+    return fma(w, mul(e, fma(e, 0.375, 0.5)), w);
+}
+}  // namespace d64
+
 // ------------------------------------------------------------------ HLL
+// the reference's formula (FP32, and FP64 states outside the short form's range)
 template <typename R>
-__device__ __forceinline__ R flux_hll(const Gas<R>& g, R rL, R pL, R unL, R utL, R rR, R pR, R unR, R utR,
+__device__ __forceinline__ R flux_hll_ref(const Gas<R>& g, R rL, R pL, R unL, R utL, R rR, R pR, R unR, R utR,
                                       R F[4])
 {
     R cL = (rL <= R(0)) ? R(0) : sqrt(g.ga * pL / rL);
@@ -131,6 +211,79 @@ __device__ __forceinline__ R flux_hll(const Gas<R>& g, R rL, R pL, R unL, R utL,
     return S;
 }
 
+template <typename R>
+__device__ __forceinline__ R flux_hll(const Gas<R>& g, R rL, R pL, R unL, R utL, R rR, R pR, R unR, R utR,
+                                      R F[4])
+{
+    return flux_hll_ref(g, rL, pL, unL, utL, rR, pR, unR, utR, F);
+}
+
+// a face's flux and wave speed from an out-of-line call (by value, so that
+// the caller's flux stays in registers on its own path)
+struct WildFlux {
+    double F[4], S;
+    __device__ __forceinline__ double get(double o[4]) const
+    {
+        for (int k = 0; k < 4; k++) o[k] = F[k];
+        return S;
+    }
+};
+// FP64: both sides' densities and pressures positive and everything inside
+// the short forms' range
+__device__ __forceinline__ bool face_tame(double rL, double pL, double unL, double utL, double rR, double pR,
+                                          double unR, double utR)
+{
+    using namespace d64;
+    return tame_pos(rL) && tame_pos(pL) && tame_pos(rR) && tame_pos(pR) && tame(unL) && tame(utL) && tame(unR) &&
+           tame(utR);
+}
+// the larger sound speed of the two sides: of p/r the larger (compared as
+// cross products), then one root
+__device__ __forceinline__ double sound_max(const Gas<double>& g, double rL, double pL, double rR, double pR)
+{
+    using namespace d64;
+    const bool l = bits(mul(pL, rR)) >= bits(mul(pR, rL));
+    return sqrt_ratio(mul(g.ga, sel(l, pL, pR)), sel(l, rL, rR));
+}
+static __device__ __noinline__ WildFlux flux_hll_wild(const Gas<double>& g, double rL, double pL, double unL, double utL,
+                                                       double rR, double pR, double unR, double utR)
+{
+    WildFlux w;
+    w.S = flux_hll_ref(g, rL, pL, unL, utL, rR, pR, unR, utR, w.F);
+    return w;
+}
+// The HLL flux in 46 FP64 operations (the formula above compiles to about
+// 100).  With the bounds S_L = min(D_L, 0) <= 0 <= S_R = max(D_R, 0),
+// a = S_R/(S_R - S_L), b = -S_L/(S_R - S_L) and the side's weights
+// A = a (u_L - S_L), B = b (u_R - S_R):
+//   F = A U_L + B U_R + (0, P, 0, a p_L u_L + b p_R u_R),  P = a p_L + b p_R,
+// which is (S_R F_L - S_L F_R + S_L S_R (U_R - U_L))/(S_R - S_L) with the
+// terms of each side collected; a supersonic face has a or b = 1 and the
+// other 0, the upwind side's flux.
+__device__ __forceinline__ double flux_hll(const Gas<double>& g, double rL, double pL, double unL, double utL,
+                                           double rR, double pR, double unR, double utR, double F[4])
+{
+    using namespace d64;
+    if (!face_tame(rL, pL, unL, utL, rR, pR, unR, utR))
+        return flux_hll_wild(g, rL, pL, unL, utL, rR, pR, unR, utR).get(F);
+    const double c = sound_max(g, rL, pL, rR, pR);
+    const double DL = sub(min(unL, unR), c), DR = add(max(unL, unR), c);
+    const double SL = sel(neg(DL), DL, 0.0), SR = sel(neg(DR), 0.0, DR);
+    const double inv = rcp(sub(SR, SL));
+    const double a = sel(neg(DL), mul(SR, inv), 1.0), b = sel(neg(DR), 1.0, mul(-SL, inv));
+    const double A = mul(a, sub(unL, SL)), B = mul(b, sub(unR, SR));
+    const double mL = mul(A, rL), mR = mul(B, rR);
+    const double PL = mul(a, pL), PR = mul(b, pR);
+    F[0] = add(mL, mR);
+    F[1] = fma(mL, unL, fma(mR, unR, add(PL, PR)));
+    F[2] = fma(mL, utL, mul(mR, utR));
+    const double qL = fma(unL, unL, mul(utL, utL)), qR = fma(unR, unR, mul(utR, utR));
+    const double k = fma(mL, qL, mul(mR, qR));
+    const double h = fma(mul(A, pL), g.inv_g1, mul(PL, unL));
+    F[3] = fma(0.5, k, fma(mul(B, pR), g.inv_g1, fma(PR, unR, h)));
+    return max_abs(DL, DR);
+}
+
 // ------------------------------------------------------------------ identical states
 // The HLL and HLLC fluxes of a face whose two sides hold one state (r, p,
 // un, ut), r > 0, p > 0: the physical flux of that state, which their
@@ -138,7 +291,7 @@ __device__ __forceinline__ R flux_hll(const Gas<R>& g, R rL, R pL, R unL, R utL,
 // expressions), and the wave speed they return, max(|un - c|, |un + c|)
 // with c = sqrt(ga p / r), formed as they form it.
 template <typename R>
-__device__ __forceinline__ R flux_physical(const Gas<R>& g, R r, R p, R un, R ut, R F[4])
+__device__ __forceinline__ R flux_physical_ref(const Gas<R>& g, R r, R p, R un, R ut, R F[4])
 {
     const R c = sqrt(g.ga * p / r);
     const R SL = un - c, SR = un + c;
@@ -149,6 +302,35 @@ __device__ __forceinline__ R flux_physical(const Gas<R>& g, R r, R p, R un, R ut
     F[2] = m * ut;
     F[3] = (e + p) * un;
     return fmax(fabs(SL), fabs(SR));
+}
+
+template <typename R>
+__device__ __forceinline__ R flux_physical(const Gas<R>& g, R r, R p, R un, R ut, R F[4])
+{
+    return flux_physical_ref(g, r, p, un, ut, F);
+}
+static __device__ __noinline__ WildFlux flux_physical_wild(const Gas<double>& g, double r, double p, double un, double ut)
+{
+    WildFlux w;
+    w.S = flux_physical_ref(g, r, p, un, ut, w.F);
+    return w;
+}
+// FP64, with the sound speed as the short HLL and HLLC forms find it
+__device__ __forceinline__ double flux_physical(const Gas<double>& g, double r, double p, double un, double ut,
+                                                double F[4])
+{
+    using namespace d64;
+    if (!(tame_pos(r) && tame_pos(p) && tame(un) && tame(ut)))
+        return flux_physical_wild(g, r, p, un, ut).get(F);
+    const double c = sqrt_ratio(mul(g.ga, p), r);
+    const double m = mul(r, un);
+    F[0] = m;
+    F[1] = fma(m, un, p);
+    F[2] = mul(m, ut);
+    // (e + p) un, e + p = ga p/(ga - 1) + r q/2
+    const double q = fma(un, un, mul(ut, ut));
+    F[3] = fma(mul(0.5, m), q, mul(mul(mul(g.ga, p), g.inv_g1), un));
+    return max_abs(sub(un, c), add(un, c));
 }
 
 // ------------------------------------------------------------------ HLL, two faces in packed FP32
@@ -250,7 +432,7 @@ __device__ __forceinline__ R flux_hllc_a(const Gas<R>& g, R r1, R p1, R un1, R u
 
 // ------------------------------------------------------------------ HLLC
 template <typename R>
-__device__ __forceinline__ R flux_hllc(const Gas<R>& g, R rL, R pL, R u1, R v1, R rR, R pR, R u2, R v2, R F[4])
+__device__ __forceinline__ R flux_hllc_ref(const Gas<R>& g, R rL, R pL, R u1, R v1, R rR, R pR, R u2, R v2, R F[4])
 {
     R cL = sqrt(g.ga * pL / rL);
     R cR = sqrt(g.ga * pR / rR);
@@ -294,6 +476,54 @@ __device__ __forceinline__ R flux_hllc(const Gas<R>& g, R rL, R pL, R u1, R v1, 
         F[3] = (eR + pR) * u2 + SR * (es - eR);
     }
     return S;
+}
+
+template <typename R>
+__device__ __forceinline__ R flux_hllc(const Gas<R>& g, R rL, R pL, R u1, R v1, R rR, R pR, R u2, R v2, R F[4])
+{
+    return flux_hllc_ref(g, rL, pL, u1, v1, rR, pR, u2, v2, F);
+}
+static __device__ __noinline__ WildFlux flux_hllc_wild(const Gas<double>& g, double rL, double pL, double u1, double v1,
+                                                        double rR, double pR, double u2, double v2)
+{
+    WildFlux w;
+    w.S = flux_hllc_ref(g, rL, pL, u1, v1, rR, pR, u2, v2, w.F);
+    return w;
+}
+// The HLLC flux in 46 FP64 operations (the formula above compiles to about
+// 110).  The side K that the contact leaves behind is selected before its
+// star state is formed, and the flux is taken as the star state's own,
+//   rho* SM (1, SM, v_K, .) + p* (0, 1, 0, .),  (E* + p*) SM,
+// rho* = rho_K (S_K - u_K)/(S_K - SM), which equals F_K + S_K (U* - U_K);
+// a supersonic face is its upwind side with SM = u_K and rho* = rho_K.
+__device__ __forceinline__ double flux_hllc(const Gas<double>& g, double rL, double pL, double u1, double v1,
+                                            double rR, double pR, double u2, double v2, double F[4])
+{
+    using namespace d64;
+    if (!face_tame(rL, pL, u1, v1, rR, pR, u2, v2))
+        return flux_hllc_wild(g, rL, pL, u1, v1, rR, pR, u2, v2).get(F);
+    const double c = sound_max(g, rL, pL, rR, pR);
+    const double SL = sub(min(u1, u2), c), SR = add(max(u1, u2), c);
+    const double wL = sub(SL, u1), wR = sub(SR, u2);
+    const double aL = mul(rL, wL), aR = mul(rR, wR);     // aL < 0 < aR
+    const double num = fma(aR, u2, fma(-aL, u1, sub(pL, pR)));
+    const double SM = mul(num, rcp(sub(aR, aL)));
+    const double ptz = mul(0.5, add(fma(aR, sub(SM, u2), pR), fma(aL, sub(SM, u1), pL)));
+    // SL >= 0, then SR <= 0, then the side of the contact
+    const bool supL = bits(SL) >= 0, supR = bits(SR) <= 0;
+    const bool left = supL || (!supR && bits(SM) >= 0), sup = supL || supR;
+    const double r = sel(left, rL, rR), p = sel(left, pL, pR), u = sel(left, u1, u2), v = sel(left, v1, v2);
+    const double S = sel(left, SL, SR), w = sel(left, wL, wR), a = sel(left, aL, aR);
+    const double inv = rcp(sub(S, SM));
+    const double q = fma(u, u, mul(v, v));
+    const double e = fma(p, g.inv_g1, mul(mul(0.5, r), q));
+    const double es = mul(fma(e, w, fma(ptz, SM, -mul(p, u))), inv);
+    const double um = sel(sup, u, SM), pm = sel(sup, p, ptz);
+    F[0] = mul(sel(sup, r, mul(a, inv)), um);
+    F[1] = fma(F[0], um, pm);
+    F[2] = mul(F[0], v);
+    F[3] = mul(add(sel(sup, e, es), pm), um);
+    return max_abs(SL, SR);
 }
 
 // The passive-scalar flux of the HLLC solver above (the Q channel of

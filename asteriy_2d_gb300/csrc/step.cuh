@@ -264,10 +264,13 @@ __device__ __forceinline__ bool cell_fixed(const StepParams& P, double x, double
 }
 
 // ------------------------------------------------------------------ reductions
+// the larger of two wave speeds >= 0 (not NaN)
+__device__ __forceinline__ float larger_speed(float a, float b) { return fmaxf(a, b); }
+__device__ __forceinline__ double larger_speed(double a, double b) { return d64::max_pos(a, b); }
 template <typename T>
 __device__ __forceinline__ T warp_max(T v)
 {
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    for (int o = 16; o > 0; o >>= 1) v = larger_speed(v, __shfl_xor_sync(0xffffffffu, v, o));
     return v;
 }
 
@@ -388,52 +391,104 @@ __device__ __forceinline__ S& tile_smem()
     return *reinterpret_cast<S*>(smem_raw + ((128 - (a & 127)) & 127));
 }
 
+// ------------------------------------------------------------------ sign and NaN tests
+// a <= 0, and whether a is a NaN, for values that seldom are: FP64 on the bit
+// pattern (an FP64 comparison only where the pattern says it may be so)
+__device__ __forceinline__ bool le_zero(float a) { return a <= 0.0f; }
+__device__ __forceinline__ bool le_zero(double a) { return __double_as_longlong(a) <= 0 && a <= 0.0; }
+__device__ __forceinline__ bool is_nan(float a) { return !(a == a); }
+__device__ __forceinline__ bool is_nan(double a) { return !d64::finite(a) && !(a == a); }
 // ------------------------------------------------------------------ cell update
-// Conservative update of one cell in arithmetic C from its state `in`
+// Conservative update of one cell in FP32 from its state `in`
 // (rho, p, vz, vr) and its four face fluxes f[k][face] (k = mass, mom_z,
 // mom_r, energy; face = right, left, bottom, top, all oriented along +z/+r).
 // tdv = T_do/(dx dy), ty = T_do/r.  Planar: Kernel_TVD, kernel.cu:3027-3073;
 // axisymmetric with the cylindrical source: add_MK, kernel.cu:2480-2509.
-template <typename C, typename R>
-__device__ __forceinline__ void update_cell(const StepParams& P, C ga, C g1, C inv_g1, const R in[4],
-                                            const R f[4][4], C T_do, C tdv, C ty, C dx, C dy, C Q2, C Sz, C Sr,
-                                            int& nrho, int& np, unsigned& status, R out[4], C* E2o = nullptr,
-                                            C* KE2o = nullptr)
+__device__ __forceinline__ void update_cell(const StepParams& P, float ga, float g1, float inv_g1, const float in[4],
+                                            const float f[4][4], float T_do, float tdv, float ty, float dx, float dy,
+                                            float Q2, int& nrho, int& np, unsigned& status, float out[4], float& E2o,
+                                            float& KE2o)
 {
-    const C r1 = (C)in[0], p1 = (C)in[1], vz1 = (C)in[2], vr1 = (C)in[3];
-    C ps[4];
+    const float r1 = in[0], p1 = in[1], vz1 = in[2], vr1 = in[3];
+    float ps[4];
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        const C f12 = (C)f[k][0], f14 = -(C)f[k][1], f13 = -(C)f[k][2], f15 = (C)f[k][3];
+        const float f12 = f[k][0], f14 = -f[k][1], f13 = -f[k][2], f15 = f[k][3];
         if (P.geom == 1) ps[k] = (f12 + f14) * dy + (f13 + f15) * dx;
         else ps[k] = f12 * dy + f13 * dx + f14 * dy + f15 * dx;
     }
-    const C Q3 = Q2 * vr1;
-    const C ke1 = r1 * (vz1 * vz1 + vr1 * vr1) * C(0.5);
-    C rho2, mz, mr, E2;
+    const float Q3 = Q2 * vr1;
+    const float ke1 = r1 * (vz1 * vz1 + vr1 * vr1) * 0.5f;
+    float rho2, mz, mr, E2;
     if (P.geom == 1) {
         rho2 = r1 - tdv * ps[0] - ty * r1 * vr1;
-        if (rho2 <= C(0)) { nrho++; rho2 = r1; }
-        mz = r1 * vz1 - tdv * ps[1] - ty * r1 * vr1 * vz1 + Sz;
-        mr = r1 * vr1 - tdv * ps[2] - ty * r1 * vr1 * vr1 + T_do * Q2 + Sr;
+        if (rho2 <= 0.0f) { nrho++; rho2 = r1; }
+        mz = r1 * vz1 - tdv * ps[1] - ty * r1 * vr1 * vz1;
+        mr = r1 * vr1 - tdv * ps[2] - ty * r1 * vr1 * vr1 + T_do * Q2;
         E2 = (p1 * inv_g1 + ke1) - tdv * ps[3] - ty * vr1 * (ga * p1 * inv_g1 + ke1) + T_do * Q3;
     } else {
         rho2 = r1 - tdv * ps[0];
-        if (rho2 <= C(0)) { nrho++; rho2 = r1; }
-        mz = r1 * vz1 - tdv * ps[1] + Sz;
-        mr = r1 * vr1 - tdv * ps[2] + T_do * Q2 + Sr;
+        if (rho2 <= 0.0f) { nrho++; rho2 = r1; }
+        mz = r1 * vz1 - tdv * ps[1];
+        mr = r1 * vr1 - tdv * ps[2] + T_do * Q2;
         E2 = (p1 * inv_g1 + ke1) - tdv * ps[3] + T_do * Q3;
     }
-    const C irho = C(1) / rho2;
-    const C vz2 = mz * irho, vr2 = mr * irho;
-    const C KE2 = C(0.5) * rho2 * (vz2 * vz2 + vr2 * vr2);
-    C p2 = (E2 - KE2) * g1;
-    if (p2 <= C(0)) { np++; p2 = sizeof(C) == 4 ? (C)P.p_floorf : (C)P.p_floor; }
+    const float irho = 1.0f / rho2;
+    const float vz2 = mz * irho, vr2 = mr * irho;
+    const float KE2 = 0.5f * rho2 * (vz2 * vz2 + vr2 * vr2);
+    float p2 = (E2 - KE2) * g1;
+    if (p2 <= 0.0f) { np++; p2 = P.p_floorf; }
     // a non-finite flux or state reaches p2 through the energy or 1/rho
     // (a NaN sound speed can leave the wave speed finite: fmax drops NaN)
     if (!(p2 == p2)) status |= 0x10u;
+    out[0] = rho2; out[1] = p2; out[2] = vz2; out[3] = vr2;
+    E2o = E2;
+    KE2o = KE2;
+}
+
+// The same update in FP64, in 38 operations (the expressions above compile
+// to about 65): tz = T_do/dx and tr = T_do/dy multiply the flux differences
+// themselves, the momenta serve the energies (rho v^2 = (rho v) v), and the
+// signs are read off the bit patterns.  `body`, `source`: whether Q2, and
+// Sz and Sr, are to be added.
+template <typename R>
+__device__ __forceinline__ void update_cell64(const StepParams& P, const R in[4], const R f[4][4], double T_do,
+                                              double tz, double tr, double ty, bool body, double Q2, bool source,
+                                              double Sz, double Sr, int& nrho, int& np, unsigned& status, R out[4])
+{
+    using namespace d64;
+    const double r1 = (double)in[0], p1 = (double)in[1], vz1 = (double)in[2], vr1 = (double)in[3];
+    const double mz1 = mul(r1, vz1), mr1 = mul(r1, vr1);
+    const double E1 = fma(0.5, fma(mz1, vz1, mul(mr1, vr1)), mul(p1, P.gd.inv_g1));
+    double U[4] = {r1, mz1, mr1, E1};
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const double fz = sub((double)f[k][0], (double)f[k][1]), fr = sub((double)f[k][3], (double)f[k][2]);
+        U[k] = fma(-tr, fr, fma(-tz, fz, U[k]));
+    }
+    if (P.geom == 1) {
+        const double w = mul(ty, mr1);
+        U[0] = sub(U[0], w);
+        U[1] = fma(-w, vz1, U[1]);
+        U[2] = fma(-w, vr1, U[2]);
+        U[3] = fma(-mul(ty, vr1), add(E1, p1), U[3]);
+    }
+    if (body) {
+        U[2] = fma(T_do, Q2, U[2]);
+        U[3] = fma(T_do, mul(Q2, vr1), U[3]);
+    }
+    if (source) {
+        U[1] = add(U[1], Sz);
+        U[2] = add(U[2], Sr);
+    }
+    double rho2 = U[0];
+    if (le_zero(rho2)) { nrho++; rho2 = r1; }
+    const double irho = tame_pos(rho2) ? rcp(rho2) : 1.0 / rho2;
+    const double vz2 = mul(U[1], irho), vr2 = mul(U[2], irho);
+    double p2 = mul(fma(-0.5, fma(U[1], vz2, mul(U[2], vr2)), U[3]), P.gd.g1);
+    if (le_zero(p2)) { np++; p2 = P.p_floor; }
+    if (is_nan(p2)) status |= 0x10u;
     out[0] = (R)rho2; out[1] = (R)p2; out[2] = (R)vz2; out[3] = (R)vr2;
-    if (E2o) { *E2o = E2; *KE2o = KE2; }
 }
 
 // The neutral-coupling source of cell (n, m): SoA planes of the state's
@@ -626,8 +681,8 @@ __device__ __forceinline__ bool face_states(const StepParams& P, const S& sm, in
 #pragma unroll
             for (int k = 0; k < 4; k++) L[k] = tl[k] + R(0);
             // (the positivity rule below leaves equal sides equal)
-            if (L[0] <= R(0)) L[0] = tl[0];
-            if (L[1] <= R(0) || !P.grad_p) L[1] = tl[1];
+            if (le_zero(L[0])) L[0] = tl[0];
+            if (le_zero(L[1]) || !P.grad_p) L[1] = tl[1];
             return true;
         } else {
 #pragma unroll
@@ -640,10 +695,10 @@ __device__ __forceinline__ bool face_states(const StepParams& P, const S& sm, in
             }
         }
         // positivity of the reconstructed rho and p (kernel.cu:2706-2743)
-        if (L[0] <= R(0)) L[0] = tl[0];
-        if (U[0] <= R(0)) U[0] = tu[0];
-        if (L[1] <= R(0) || !P.grad_p) L[1] = tl[1];
-        if (U[1] <= R(0) || !P.grad_p) U[1] = tu[1];
+        if (le_zero(L[0])) L[0] = tl[0];
+        if (le_zero(U[0])) U[0] = tu[0];
+        if (le_zero(L[1]) || !P.grad_p) L[1] = tl[1];
+        if (le_zero(U[1]) || !P.grad_p) U[1] = tu[1];
     }
     return false;
 }
@@ -735,7 +790,7 @@ __device__ __forceinline__ void face_flux(const StepParams& P, S& sm, const Gas<
             // test for one
             if (ZF) put4(sm.Fz[a][c], F[0], F[1], F[2], F[3]);
             else put4(sm.Fr[a][c], F[0], F[2], F[1], F[3]);
-            if (active) smax = fmax(smax, Sp);
+            if (active) smax = larger_speed(smax, Sp);
             return;
         } else if (hi) {
             const RPre<R> q = godunov_pre(g, L[0], L[1], L[NN], L[TT], U[0], U[1], U[NN], U[TT]);
@@ -767,14 +822,14 @@ __device__ __forceinline__ void face_flux(const StepParams& P, S& sm, const Gas<
     } else {
         Sp = flux_hll(g, L[0], L[1], L[NN], L[TT], U[0], U[1], U[NN], U[TT], F);
     }
-    if (!(Sp == Sp)) { rc.status |= 0x10u; Sp = R(0); }
+    if (is_nan(Sp)) { rc.status |= 0x10u; Sp = R(0); }
     if (ZF) {
         put4(sm.Fz[a][c], F[0], F[1], F[2], F[3]);
     } else {
         // r face: the normal momentum is mom_r, the tangential one mom_z
         put4(sm.Fr[a][c], F[0], F[2], F[1], F[3]);
     }
-    if (active) smax = fmax(smax, Sp);
+    if (active) smax = larger_speed(smax, Sp);
 }
 
 // Two adjacent faces of orientation ZF in one thread: (a, c) and the next
@@ -816,10 +871,10 @@ __device__ __forceinline__ void face_two(const StepParams& P, S& sm, int b, cons
         }
     };
     auto store = [&](int fa, int fc, bool act, R f0, R f1, R f2, R f3, R sp) {
-        if (!(sp == sp)) { rc.status |= 0x10u; sp = R(0); }
+        if (is_nan(sp)) { rc.status |= 0x10u; sp = R(0); }
         if (ZF) put4(sm.Fz[fa][fc], f0, f1, f2, f3);
         else put4(sm.Fr[fa][fc], f0, f2, f1, f3);
-        if (act) smax = fmax(smax, sp);
+        if (act) smax = larger_speed(smax, sp);
     };
     // FF (kernels with the skip_uniform code, when it is set): HLL in FP32,
     // a face pair in the high-order region.  When the five staged cells of
@@ -894,15 +949,15 @@ __device__ __forceinline__ void face_two(const StepParams& P, S& sm, int b, cons
             if (hi1) { L1[k] = y1; U1[k] = z0; }
             // positivity of the reconstructed rho and p (kernel.cu:2706-2743)
             if (k == 0) {
-                if (L0[0] <= R(0)) L0[0] = v[1];
-                if (U0[0] <= R(0)) U0[0] = v[2];
-                if (L1[0] <= R(0)) L1[0] = v[2];
-                if (U1[0] <= R(0)) U1[0] = v[3];
+                if (le_zero(L0[0])) L0[0] = v[1];
+                if (le_zero(U0[0])) U0[0] = v[2];
+                if (le_zero(L1[0])) L1[0] = v[2];
+                if (le_zero(U1[0])) U1[0] = v[3];
             } else if (k == 1) {
-                if (L0[1] <= R(0) || !P.grad_p) L0[1] = v[1];
-                if (U0[1] <= R(0) || !P.grad_p) U0[1] = v[2];
-                if (L1[1] <= R(0) || !P.grad_p) L1[1] = v[2];
-                if (U1[1] <= R(0) || !P.grad_p) U1[1] = v[3];
+                if (le_zero(L0[1]) || !P.grad_p) L0[1] = v[1];
+                if (le_zero(U0[1]) || !P.grad_p) U0[1] = v[2];
+                if (le_zero(L1[1]) || !P.grad_p) L1[1] = v[2];
+                if (le_zero(U1[1]) || !P.grad_p) U1[1] = v[3];
             }
         }
     }
@@ -1126,13 +1181,13 @@ __device__ __forceinline__ void queue_pass(const StepParams& P, S& sm, int b, co
         const R p = solve_queued(P, g, q, strong, p0, rc, fallback);
         R F[4];
         R Sp = godunov_sample<R, kSampleIterative>(g, q, p, F, rc);
-        if (!(Sp == Sp)) { rc.status |= 0x10u; Sp = R(0); }
+        if (is_nan(Sp)) { rc.status |= 0x10u; Sp = R(0); }
         if (zf) {
             put4(sm.Fz[a][c], F[0], F[1], F[2], F[3]);
-            if (active) smz = fmax(smz, Sp);
+            if (active) smz = larger_speed(smz, Sp);
         } else {
             put4(sm.Fr[a][c], F[0], F[2], F[1], F[3]);
-            if (active) smr = fmax(smr, Sp);
+            if (active) smr = larger_speed(smr, Sp);
         }
         // the recorder runs on the FP64 solver only (its records are training
         // targets; the FP32 kernels are smaller without it)
@@ -1161,8 +1216,8 @@ struct TileAcc {
 // constants of the step every tile shares (set by thread 0, read after a barrier)
 struct StepConsts {
     double T_do;           // the step's dt
-    double tdv;            // T_do / (dx dy)
-    float tdv_f, T_f;
+    double tz, tr;         // T_do / dx, T_do / dy
+    float tdv_f, T_f;      // T_do / (dx dy), T_do
     int step;
 };
 
@@ -1170,8 +1225,9 @@ __device__ __forceinline__ void step_consts_of(const StepParams& P, double T_do,
 {
     K.T_do = T_do;
     K.step = step;
-    K.tdv = K.T_do / (P.dx * P.dy);
-    K.tdv_f = (float)K.tdv;
+    K.tz = K.T_do / P.dx;
+    K.tr = K.T_do / P.dy;
+    K.tdv_f = (float)(K.T_do / (P.dx * P.dy));
     K.T_f = (float)K.T_do;
 }
 
@@ -1437,7 +1493,7 @@ __device__ __forceinline__ void tile_body(const StepParams& P, S& sm, int b, con
     // FP64 constants read where they are used (not held in registers
     // through the FP32 form's loop)
     auto update_fp64 = [&](int row, int n, const R in[4], const R f[4][4], R o[4]) {
-        const double T_do = K.T_do, tdv_d = K.tdv;
+        const double T_do = K.T_do;
         const double y = sm.ydrow[row];
         double Q2 = 0.0, Sz = 0.0, Sr = 0.0;
         if (P.body_force) {
@@ -1455,8 +1511,8 @@ __device__ __forceinline__ void tile_body(const StepParams& P, S& sm, int b, con
             Sr = w * ar;
         }
         const double ty = (sizeof(R) == 8) ? sm.tydrow[row] : ((P.geom == 1) ? T_do / y : 0.0);
-        update_cell<double>(P, P.gd.ga, P.gd.g1, P.gd.inv_g1, in, f, T_do, tdv_d, ty, P.dx, P.dy, Q2, Sz, Sr,
-                            acc.nrho, acc.np, acc.rc.status, o);
+        update_cell64(P, in, f, T_do, K.tz, K.tr, ty, P.body_force != 0, Q2, sizeof(R) == 8 && P.nsrc != nullptr, Sz,
+                      Sr, acc.nrho, acc.np, acc.rc.status, o);
     };
     // the FP32 form's source terms of a cell: ty = T_do/r and the body force
     auto sources_fp32 = [&](int row, int n, const R in[4], float& ty, float& Q2) {
@@ -1514,8 +1570,8 @@ __device__ __forceinline__ void tile_body(const StepParams& P, S& sm, int b, con
                 float ty, Q2;
                 sources_fp32(row, n, in, ty, Q2);
                 float E2, KE2;
-                update_cell<float>(P, gaf, g1f, ig1f, in, f, Tf, tdv_f, ty, dxf, dyf, Q2, 0.0f, 0.0f, acc.nrho, acc.np,
-                                   acc.rc.status, o, &E2, &KE2);
+                update_cell(P, gaf, g1f, ig1f, in, f, Tf, tdv_f, ty, dxf, dyf, Q2, acc.nrho, acc.np, acc.rc.status, o,
+                            E2, KE2);
                 // pressure recovery p = (g-1)(E - rho v^2/2) in FP64 where
                 // the kinetic energy is more than 99% of the total
                 if (KE2 > 0.99f * E2) deferred |= 2u << (2 * it);
@@ -1599,7 +1655,7 @@ __device__ __forceinline__ void cta_epilogue(const StepParams& P, TileAcc<R>& ac
         int c0 = 0, c1 = 0, c2 = 0;
         unsigned st = 0;
         for (int w = 0; w < kThreads / 32; w++) {
-            ar = fmax(ar, red_r[0][w]); br = fmax(br, red_r[1][w]);
+            ar = larger_speed(ar, red_r[0][w]); br = larger_speed(br, red_r[1][w]);
             c0 += red_i[0][w]; c1 += red_i[1][w]; st |= (unsigned)red_i[2][w]; c2 += red_i[3][w];
         }
         if (c0) st |= 0x01u;

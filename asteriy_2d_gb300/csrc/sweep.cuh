@@ -415,8 +415,8 @@ __device__ __forceinline__ void sweep_strip(const StepParams& P, const StepConst
                         if (x > P.body_lo && x < P.body_hi)
                             Q2 = (y >= P.body_rsplit) ? -P.body_amp * (double)w0[0] : P.body_amp * (double)w0[0];
                     }
-                    update_cell<double>(P, P.gd.ga, P.gd.g1, P.gd.inv_g1, w0, f, T_do, K.tdv, T_do / y, P.dx, P.dy,
-                                        Q2, 0.0, 0.0, acc.nrho, acc.np, acc.rc.status, o);
+                    update_cell64(P, w0, f, T_do, K.tz, K.tr, T_do / y, P.body_force != 0, Q2, false, 0.0, 0.0,
+                                  acc.nrho, acc.np, acc.rc.status, o);
                 } else {
                     const float y = P.y_minf + (float)m * P.dyf;
                     float Q2 = 0.0f;
@@ -427,8 +427,8 @@ __device__ __forceinline__ void sweep_strip(const StepParams& P, const StepConst
                     }
                     const float ty = (P.geom == 1) ? K.T_f / y : 0.0f;
                     float E2, KE2;
-                    update_cell<float>(P, gaf, g1f, ig1f, w0, f, K.T_f, K.tdv_f, ty, P.dxf, P.dyf, Q2, 0.0f, 0.0f,
-                                       acc.nrho, acc.np, acc.rc.status, o, &E2, &KE2);
+                    update_cell(P, gaf, g1f, ig1f, w0, f, K.T_f, K.tdv_f, ty, P.dxf, P.dyf, Q2, acc.nrho, acc.np,
+                                acc.rc.status, o, E2, KE2);
                     // pressure recovery in FP64 where the kinetic energy is
                     // more than 99% of the total
                     if (KE2 > 0.99f * E2)
