@@ -260,13 +260,10 @@ static __device__ __noinline__ WildFlux flux_hll_wild(const Gas<double>& g, doub
 // which is (S_R F_L - S_L F_R + S_L S_R (U_R - U_L))/(S_R - S_L) with the
 // terms of each side collected; a supersonic face has a or b = 1 and the
 // other 0, the upwind side's flux.
-__device__ __forceinline__ double flux_hll(const Gas<double>& g, double rL, double pL, double unL, double utL,
-                                           double rR, double pR, double unR, double utR, double F[4])
+__device__ __forceinline__ double flux_hll_of(const Gas<double>& g, double c, double rL, double pL, double unL,
+                                              double utL, double rR, double pR, double unR, double utR, double F[4])
 {
     using namespace d64;
-    if (!face_tame(rL, pL, unL, utL, rR, pR, unR, utR))
-        return flux_hll_wild(g, rL, pL, unL, utL, rR, pR, unR, utR).get(F);
-    const double c = sound_max(g, rL, pL, rR, pR);
     const double DL = sub(min(unL, unR), c), DR = add(max(unL, unR), c);
     const double SL = sel(neg(DL), DL, 0.0), SR = sel(neg(DR), 0.0, DR);
     const double inv = rcp(sub(SR, SL));
@@ -282,6 +279,13 @@ __device__ __forceinline__ double flux_hll(const Gas<double>& g, double rL, doub
     const double h = fma(mul(A, pL), g.inv_g1, mul(PL, unL));
     F[3] = fma(0.5, k, fma(mul(B, pR), g.inv_g1, fma(PR, unR, h)));
     return max_abs(DL, DR);
+}
+__device__ __forceinline__ double flux_hll(const Gas<double>& g, double rL, double pL, double unL, double utL,
+                                           double rR, double pR, double unR, double utR, double F[4])
+{
+    if (!face_tame(rL, pL, unL, utL, rR, pR, unR, utR))
+        return flux_hll_wild(g, rL, pL, unL, utL, rR, pR, unR, utR).get(F);
+    return flux_hll_of(g, sound_max(g, rL, pL, rR, pR), rL, pL, unL, utL, rR, pR, unR, utR, F);
 }
 
 // ------------------------------------------------------------------ identical states
@@ -496,13 +500,10 @@ static __device__ __noinline__ WildFlux flux_hllc_wild(const Gas<double>& g, dou
 //   rho* SM (1, SM, v_K, .) + p* (0, 1, 0, .),  (E* + p*) SM,
 // rho* = rho_K (S_K - u_K)/(S_K - SM), which equals F_K + S_K (U* - U_K);
 // a supersonic face is its upwind side with SM = u_K and rho* = rho_K.
-__device__ __forceinline__ double flux_hllc(const Gas<double>& g, double rL, double pL, double u1, double v1,
-                                            double rR, double pR, double u2, double v2, double F[4])
+__device__ __forceinline__ double flux_hllc_of(const Gas<double>& g, double c, double rL, double pL, double u1,
+                                               double v1, double rR, double pR, double u2, double v2, double F[4])
 {
     using namespace d64;
-    if (!face_tame(rL, pL, u1, v1, rR, pR, u2, v2))
-        return flux_hllc_wild(g, rL, pL, u1, v1, rR, pR, u2, v2).get(F);
-    const double c = sound_max(g, rL, pL, rR, pR);
     const double SL = sub(min(u1, u2), c), SR = add(max(u1, u2), c);
     const double wL = sub(SL, u1), wR = sub(SR, u2);
     const double aL = mul(rL, wL), aR = mul(rR, wR);     // aL < 0 < aR
@@ -524,6 +525,13 @@ __device__ __forceinline__ double flux_hllc(const Gas<double>& g, double rL, dou
     F[2] = mul(F[0], v);
     F[3] = mul(add(sel(sup, e, es), pm), um);
     return max_abs(SL, SR);
+}
+__device__ __forceinline__ double flux_hllc(const Gas<double>& g, double rL, double pL, double u1, double v1,
+                                            double rR, double pR, double u2, double v2, double F[4])
+{
+    if (!face_tame(rL, pL, u1, v1, rR, pR, u2, v2))
+        return flux_hllc_wild(g, rL, pL, u1, v1, rR, pR, u2, v2).get(F);
+    return flux_hllc_of(g, sound_max(g, rL, pL, rR, pR), rL, pL, u1, v1, rR, pR, u2, v2, F);
 }
 
 // The passive-scalar flux of the HLLC solver above (the Q channel of

@@ -452,21 +452,22 @@ __device__ __forceinline__ void update_cell(const StepParams& P, float ga, float
 // signs are read off the bit patterns.  `body`, `source`: whether Q2, and
 // Sz and Sr, are to be added.
 template <typename R>
-__device__ __forceinline__ void update_cell64(const StepParams& P, const R in[4], const R f[4][4], double T_do,
-                                              double tz, double tr, double ty, bool body, double Q2, bool source,
-                                              double Sz, double Sr, int& nrho, int& np, unsigned& status, R out[4])
+__device__ __forceinline__ void update_cell64(const Gas<double>& g, double p_floor, bool axisym, const R in[4],
+                                              const R f[4][4], double T_do, double tz, double tr, double ty,
+                                              bool body, double Q2, bool source, double Sz, double Sr, int& nrho,
+                                              int& np, unsigned& status, R out[4])
 {
     using namespace d64;
     const double r1 = (double)in[0], p1 = (double)in[1], vz1 = (double)in[2], vr1 = (double)in[3];
     const double mz1 = mul(r1, vz1), mr1 = mul(r1, vr1);
-    const double E1 = fma(0.5, fma(mz1, vz1, mul(mr1, vr1)), mul(p1, P.gd.inv_g1));
+    const double E1 = fma(0.5, fma(mz1, vz1, mul(mr1, vr1)), mul(p1, g.inv_g1));
     double U[4] = {r1, mz1, mr1, E1};
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         const double fz = sub((double)f[k][0], (double)f[k][1]), fr = sub((double)f[k][3], (double)f[k][2]);
         U[k] = fma(-tr, fr, fma(-tz, fz, U[k]));
     }
-    if (P.geom == 1) {
+    if (axisym) {
         const double w = mul(ty, mr1);
         U[0] = sub(U[0], w);
         U[1] = fma(-w, vz1, U[1]);
@@ -485,8 +486,8 @@ __device__ __forceinline__ void update_cell64(const StepParams& P, const R in[4]
     if (le_zero(rho2)) { nrho++; rho2 = r1; }
     const double irho = tame_pos(rho2) ? rcp(rho2) : 1.0 / rho2;
     const double vz2 = mul(U[1], irho), vr2 = mul(U[2], irho);
-    double p2 = mul(fma(-0.5, fma(U[1], vz2, mul(U[2], vr2)), U[3]), P.gd.g1);
-    if (le_zero(p2)) { np++; p2 = P.p_floor; }
+    double p2 = mul(fma(-0.5, fma(U[1], vz2, mul(U[2], vr2)), U[3]), g.g1);
+    if (le_zero(p2)) { np++; p2 = p_floor; }
     if (is_nan(p2)) status |= 0x10u;
     out[0] = (R)rho2; out[1] = (R)p2; out[2] = (R)vz2; out[3] = (R)vr2;
 }
@@ -1511,8 +1512,8 @@ __device__ __forceinline__ void tile_body(const StepParams& P, S& sm, int b, con
             Sr = w * ar;
         }
         const double ty = (sizeof(R) == 8) ? sm.tydrow[row] : ((P.geom == 1) ? T_do / y : 0.0);
-        update_cell64(P, in, f, T_do, K.tz, K.tr, ty, P.body_force != 0, Q2, sizeof(R) == 8 && P.nsrc != nullptr, Sz,
-                      Sr, acc.nrho, acc.np, acc.rc.status, o);
+        update_cell64(P.gd, P.p_floor, P.geom == 1, in, f, T_do, K.tz, K.tr, ty, P.body_force != 0, Q2,
+                      sizeof(R) == 8 && P.nsrc != nullptr, Sz, Sr, acc.nrho, acc.np, acc.rc.status, o);
     };
     // the FP32 form's source terms of a cell: ty = T_do/r and the body force
     auto sources_fp32 = [&](int row, int n, const R in[4], float& ty, float& Q2) {
