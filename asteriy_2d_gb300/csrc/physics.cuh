@@ -33,7 +33,9 @@ struct Gas {
     R tol;                    // Newton / bisection tolerance
     R eps;                    // 10e-10: degenerate rarefaction test (Header.h:62)
     R eps8;                   // 10e-8: smallest wave speed for dt (Header.h:63)
+    R hg1, hg2;               // (gamma-1)/2, (gamma+1)/2
     int max_iter;
+    int n;                    // 1/gm when it is a whole number from 2 to 16, else 0
 };
 
 template <typename R>
@@ -50,7 +52,12 @@ __host__ __device__ inline Gas<R> make_gas(double gamma, double tol, int max_ite
     g.tol = (R)tol;
     g.eps = (R)10e-10;
     g.eps8 = (R)10e-8;
+    g.hg1 = (R)(0.5 * g1);
+    g.hg2 = (R)(0.5 * g2);
     g.max_iter = max_iter;
+    const double n = 2.0 * gamma / g1;
+    const int ni = (n > 1.5 && n < 16.5) ? (int)(n + 0.5) : 0;
+    g.n = (ni > 0 && n - ni < 1e-14 * n && ni - n < 1e-14 * n) ? ni : 0;
     return g;
 }
 

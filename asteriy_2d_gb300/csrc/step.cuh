@@ -21,6 +21,7 @@
 #include <cstddef>
 #include <type_traits>
 
+#include "godunov64.cuh"
 #include "mlp.cuh"
 #include "physics.cuh"
 #include "tma.cuh"
@@ -583,7 +584,7 @@ __device__ __forceinline__ R solve_queued(const StepParams& P, const Gas<R>& g, 
     // the reference's own iteration (FP64 only: the FP32 form always runs
     // the safeguarded Newton, and its kernels leave this code out)
     if constexpr (sizeof(R) == 8) {
-        if (!P.riemann_newton) return solve_p_reference(g, q, rc);
+        if (!P.riemann_newton) return face_solve(g, q, rc);
     }
     R p0;
     if (P.guess == 1 && strong) {
@@ -704,6 +705,34 @@ __device__ __forceinline__ bool face_states(const StepParams& P, const S& sm, in
     return false;
 }
 
+// the exact solver's flux and wave speed of a face whose sides hold one state
+__device__ __forceinline__ float exact_same_state(const Gas<float>& g, float r, float p, float un, float ut, float F[4])
+{
+    const float cs = sqrt(g.ga * p / r);
+    const float m = r * un;
+    F[0] = m;
+    F[1] = m * un + p;
+    F[2] = m * ut;
+    F[3] = un * (p * g.inv_g1 + 0.5f * r * (un * un + ut * ut) + p);
+    return fmax(fabs(un) + cs, g.eps8);
+}
+__device__ __forceinline__ double exact_same_state(const Gas<double>& g, double r, double p, double un, double ut,
+                                                   double F[4])
+{
+    const double S = flux_physical(g, r, p, un, ut, F);
+    return is_nan(S) ? g.eps8 : larger_speed(S, g.eps8);
+}
+
+// whether the two sides of a face hold equal values (FP64: the same bits)
+__device__ __forceinline__ bool same_state(const float L[4], const float U[4])
+{
+    return L[0] == U[0] && L[1] == U[1] && L[2] == U[2] && L[3] == U[3];
+}
+__device__ __forceinline__ bool same_state(const double L[4], const double U[4])
+{
+    return same_bits(L[0], U[0]) && same_bits(L[1], U[1]) && same_bits(L[2], U[2]) && same_bits(L[3], U[3]);
+}
+
 // Whether face (a, c) of orientation ZF belongs to an updated cell
 // (active: its wave speed counts for dt) and lies in the high-order region
 // (hi).  ZF: z faces (between tile columns c-1 and c of row a), else r
@@ -774,19 +803,12 @@ __device__ __forceinline__ void face_flux(const StepParams& P, S& sm, const Gas<
             // faces however the tile was staged
             F[0] = F[1] = F[2] = F[3] = R(0);
             Sp = R(0);
-        } else if (hi && (same_sides || (L[0] == U[0] && L[1] == U[1] && L[2] == U[2] && L[3] == U[3]))) {
+        } else if (hi && (same_sides || same_state(L, U))) {
             // identical states: the exact solution is that state (the
             // reference reaches it through the two-rarefaction branch with
             // p* = p, u* = u_n, up to rounding), its flux the physical flux
             // and its largest wave speed |u_n| + c
-            const R r = L[0], p = L[1], un = L[NN], ut = L[TT];
-            const R cs = sqrt(g.ga * p / r);
-            const R m = r * un;
-            F[0] = m;
-            F[1] = m * un + p;
-            F[2] = m * ut;
-            F[3] = un * (p * g.inv_g1 + R(0.5) * r * (un * un + ut * ut) + p);
-            Sp = fmax(fabs(un) + cs, g.eps8);
+            Sp = exact_same_state(g, L[0], L[1], L[NN], L[TT], F);
             // stored here: fmax drops a NaN, so this wave speed needs no
             // test for one
             if (ZF) put4(sm.Fz[a][c], F[0], F[1], F[2], F[3]);
@@ -794,18 +816,21 @@ __device__ __forceinline__ void face_flux(const StepParams& P, S& sm, const Gas<
             if (active) smax = larger_speed(smax, Sp);
             return;
         } else if (hi) {
-            const RPre<R> q = godunov_pre(g, L[0], L[1], L[NN], L[TT], U[0], U[1], U[NN], U[TT]);
+            const RPre<R> q = face_pre(g, L[0], L[1], L[NN], L[TT], U[0], U[1], U[NN], U[TT]);
             if (q.pattern == 2 || q.pattern == 3) {
                 // the iterative faces go to the queue (room for every face
                 // of the tile); their flux is written by queue_pass
-                const bool strong = P.riemann_newton && wave_strength(q) > P.mlp_gate;
-                const unsigned old = atomicAdd(&sm.qn, strong ? 1u : 0x10000u);
-                const int slot = strong ? (int)(old & 0xffffu) : S::kQueueCap - 1 - (int)(old >> 16);
+                // front: the faces above the learned start's gate, or, with
+                // the reference's iterations, those of pattern 3 (another
+                // loop than pattern 2's: kept in other warps)
+                const bool front = P.riemann_newton ? wave_strength(q) > P.mlp_gate : q.pattern == 3;
+                const unsigned old = atomicAdd(&sm.qn, front ? 1u : 0x10000u);
+                const int slot = front ? (int)(old & 0xffffu) : S::kQueueCap - 1 - (int)(old >> 16);
                 const int f = a * W + c;
                 sm.qcode[slot] = (unsigned short)((ZF ? f : NFZ + f) | (active ? 1 << 12 : 0) | (q.pattern << 14));
                 return;
             }
-            Sp = godunov_sample<R, kSampleClosed>(g, q, R(0), F, rc);
+            Sp = face_sample<kSampleClosed>(g, q, R(0), F, rc);
         } else {
             Sp = flux_hll(g, L[0], L[1], L[NN], L[TT], U[0], U[1], U[NN], U[TT], F);
         }
@@ -1103,7 +1128,7 @@ __device__ __forceinline__ RPre<R> queued_face(const StepParams& P, const S& sm,
     // normal and tangential velocity: (v_z, v_r) on z faces, (v_r, v_z) on r faces
     const R unL = zf ? L[2] : L[3], utL = zf ? L[3] : L[2];
     const R unU = zf ? U[2] : U[3], utU = zf ? U[3] : U[2];
-    RPre<R> q = godunov_sides(g, L[0], L[1], unL, utL, U[0], U[1], unU, utU);
+    RPre<R> q = face_sides_of(g, L[0], L[1], unL, utL, U[0], U[1], unU, utU);
     q.pattern = pattern;
     return q;
 }
@@ -1181,7 +1206,7 @@ __device__ __forceinline__ void queue_pass(const StepParams& P, S& sm, int b, co
         const R p0 = (strong && P.guess == 1 && P.mlp) ? (zf ? sm.Fz[a][c][0] : sm.Fr[a][c][0]) : R(0);
         const R p = solve_queued(P, g, q, strong, p0, rc, fallback);
         R F[4];
-        R Sp = godunov_sample<R, kSampleIterative>(g, q, p, F, rc);
+        R Sp = face_sample<kSampleIterative>(g, q, p, F, rc);
         if (is_nan(Sp)) { rc.status |= 0x10u; Sp = R(0); }
         if (zf) {
             put4(sm.Fz[a][c], F[0], F[1], F[2], F[3]);
@@ -1354,13 +1379,7 @@ template <typename R, int FLUX>
 __device__ __forceinline__ R uniform_face(const Gas<R>& g, R r, R p, R un, R ut, R F[4])
 {
     if constexpr (FLUX == 2) {
-        const R cs = sqrt(g.ga * p / r);
-        const R m = r * un;
-        F[0] = m;
-        F[1] = m * un + p;
-        F[2] = m * ut;
-        F[3] = un * (p * g.inv_g1 + R(0.5) * r * (un * un + ut * ut) + p);
-        return fmax(fabs(un) + cs, g.eps8);
+        return exact_same_state(g, r, p, un, ut, F);
     } else if constexpr (FLUX == 1) {
         return flux_hllc(g, r, p, un, ut, r, p, un, ut, F);
     } else if constexpr (FLUX == 3) {
