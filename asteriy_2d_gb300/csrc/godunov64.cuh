@@ -47,26 +47,20 @@ __device__ __forceinline__ bool godunov_tame(const RPre<double>& q)
     return godunov_tame(q.rI, q.pI, q.enI, q.teI, q.rII, q.pII, q.enII, q.teII);
 }
 
-namespace d64 {
-// x^(-1/2) of a normal x: the approximate inverse root and one third-order step
-__device__ __forceinline__ double rsqrt(double x)
-{
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-mul(x, y), y, 1.0);
-    return fma(y, mul(e, fma(e, 0.375, 0.5)), y);
-}
 // y^n, n = 2 .. 16
-__device__ __forceinline__ double ipow(double y, int n)
+__device__ __forceinline__ double ipow(const d64::Pipe& o, double y, int n)
 {
     double r = (n & 1) ? y : 1.0, b = y;
+    bool one = !(n & 1);
     for (int k = n >> 1; k; k >>= 1) {
-        b = mul(b, b);
-        if (k & 1) r = (bits(r) == bits(1.0)) ? b : mul(r, b);
+        b = o.mul(b, b);
+        if (k & 1) {
+            r = one ? b : o.mul(r, b);
+            one = false;
+        }
     }
     return r;
 }
-}  // namespace d64
 
 // x^gm for 1/gm = n: with w = x^(-1/n) from FP32 and e = 1 - x w^n,
 // x^(-1/n) = w (1 - e)^(-1/n) = w (1 + e/n + (n+1) e^2/(2 n^2) + ...), |e| of
@@ -74,24 +68,26 @@ __device__ __forceinline__ double ipow(double y, int n)
 __device__ __forceinline__ double pow_gm(const Gas<double>& g, double x)
 {
     using namespace d64;
+    const Pipe o(g);
     if (g.n == 0) return pow(x, g.gm);
     const double w = (double)exp2f(-(float)g.gm * log2f(low_float(x)));
-    const double e = fma(-x, ipow(w, g.n), 1.0);
-    return rcp(fma(w, mul(e, fma(e, mul(mul(0.5, g.gm), add(g.gm, 1.0)), g.gm)), w));
+    const double e = fma(-x, ipow(o, w, g.n), 1.0);
+    return o.rcp(fma(w, o.mul(e, fma(e, o.mul(o.mul(o.half, g.gm), o.add(g.gm, 1.0)), g.gm)), w));
 }
 // x^(1/gm)
 __device__ __forceinline__ double pow_inv_gm(const Gas<double>& g, double x)
 {
-    return g.n ? d64::ipow(x, g.n) : pow(x, 1.0 / g.gm);
+    return g.n ? ipow(d64::Pipe(g), x, g.n) : pow(x, 1.0 / g.gm);
 }
 // rare_coef (physics.cuh) from y = (p/p_K)^gm: (1 - y^n)/(1 - y) = 1 + y + ...
 // + y^(n-1), and its limit rho c within the same absolute distance of p_K
 __device__ __forceinline__ double rare_coef_y(const Gas<double>& g, double rc, double y, double p, double pK)
 {
     using namespace d64;
-    double s = add(1.0, y);
+    const Pipe o(g);
+    double s = o.add(1.0, y);
     for (int k = 2; k < g.n; k++) s = fma(s, y, 1.0);
-    return sel(bits(abs(sub(p, pK))) < bits(g.eps), rc, mul(mul(g.gm, rc), s));
+    return sel(bits(abs(o.sub(p, pK))) < bits(g.eps), rc, o.mul(o.mul(g.gm, rc), s));
 }
 
 // godunov_sides and godunov_pre (physics.cuh) of a tame face
@@ -99,6 +95,7 @@ __device__ __forceinline__ RPre<double> godunov_sides64(const Gas<double>& g, do
                                                         double utL, double rR, double pR, double unR, double utR)
 {
     using namespace d64;
+    const Pipe o(g);
     RPre<double> q;
     q.swap = bits(pL) > bits(pR);
     q.enI = sel(q.swap, -unR, unL);
@@ -109,9 +106,9 @@ __device__ __forceinline__ RPre<double> godunov_sides64(const Gas<double>& g, do
     q.teII = sel(q.swap, utL, utR);
     q.pII = sel(q.swap, pL, pR);
     q.rII = sel(q.swap, rL, rR);
-    q.cI = sqrt_ratio(mul(g.ga, q.pI), q.rI);
-    q.cII = sqrt_ratio(mul(g.ga, q.pII), q.rII);
-    q.Udf = sub(q.enI, q.enII);
+    q.cI = o.sqrt_ratio(o.mul(g.ga, q.pI), q.rI);
+    q.cII = o.sqrt_ratio(o.mul(g.ga, q.pII), q.rII);
+    q.Udf = o.sub(q.enI, q.enII);
     q.Urz = q.Uvk = 0.0;
     q.pattern = 4;
     return q;
@@ -121,31 +118,32 @@ __device__ __forceinline__ RPre<double> godunov_pre64(const Gas<double>& g, doub
                                                       double utL, double rR, double pR, double unR, double utR)
 {
     using namespace d64;
+    const Pipe o(g);
     RPre<double> q = godunov_sides64(g, rL, pL, unL, utL, rR, pR, unR, utR);
-    const double dp = sub(q.pII, q.pI);
-    const double Uud = mul(dp, rsqrt(mul(q.rI, fma(g.hg2, q.pII, mul(g.hg1, q.pI)))));
+    const double dp = o.sub(q.pII, q.pI);
+    const double Uud = o.mul(dp, o.rsqrt(o.mul(q.rI, fma(g.hg2, q.pII, o.mul(g.hg1, q.pI)))));
     if (bits(q.Udf) > 0) {
         q.pattern = bits(q.Udf) <= bits(Uud) ? 2 : 3;
         return q;
     }
     // Udf <= 0 <= Uud: vacuum, two rarefactions or pattern 2
-    const double k2 = mul(2.0, g.inv_g1);
-    q.Uvk = mul(-k2, add(q.cII, q.cI));
+    const double k2 = o.mul(2.0, g.inv_g1);
+    q.Uvk = o.mul(-k2, o.add(q.cII, q.cI));
     if (key(q.Udf) < key(q.Uvk)) {
         q.pattern = 0;
         return q;
     }
     // Urz = -2 cII/(gamma-1) (1 - x^gm), x = pI/pII: FP32 decides unless Udf
     // lies within 1e-4 of it
-    const double x = mul(q.pI, rcp(q.pII));
-    const float y = -expm1f((float)g.gm * log1pf(-low_float(sub(1.0, x))));
+    const double x = o.mul(q.pI, o.rcp(q.pII));
+    const float y = -expm1f((float)g.gm * log1pf(-low_float(o.sub(1.0, x))));
     const float zf = -low_float(k2) * low_float(q.cII) * y, uf = low_float(q.Udf);
     const bool sure = fabsf(uf - zf) > 1e-4f * fabsf(zf) && y < 1.0f;
     if (sure && uf > zf) {
         q.pattern = 2;
         return q;
     }
-    q.Urz = mul(mul(-k2, q.cII), sub(1.0, pow_gm(g, x)));
+    q.Urz = o.mul(o.mul(-k2, q.cII), o.sub(1.0, pow_gm(g, x)));
     q.pattern = (sure || key(q.Udf) <= key(q.Urz)) ? 1 : 2;
     return q;
 }
@@ -224,6 +222,7 @@ static __device__ __noinline__ RPre<double> sides_wild(const Gas<double>& g, dou
 __device__ __forceinline__ double bisect_p64(const Gas<double>& g, const RPre<double>& q, RiemannCount& rc)
 {
     using namespace d64;
+    const Pipe o(g);
     const float pIf = low_float(q.pI), pIIf = low_float(q.pII), cIf = low_float(q.cI), cIIf = low_float(q.cII);
     const float dUf = low_float(q.Udf), tolf = (float)g.tol;
     const float band = 2.3e-13f * (cIf + cIIf + fabsf(low_float(q.enI)) + fabsf(low_float(q.enII)));
@@ -252,17 +251,17 @@ __device__ __forceinline__ double bisect_p64(const Gas<double>& g, const RPre<do
     // FP64 Newton steps until one is below 3e-7 p (usually the first)
     double p = (double)pf;
     if (ok) {
-        const double ipI = rcp(q.pI), ipII = rcp(q.pII), kI = rcp(mul(q.rI, q.cI));
-        const double gpI = mul(g.gp, ipI), c2 = mul(mul(2.0, g.inv_g1), q.cII);
+        const double ipI = o.rcp(q.pI), ipII = o.rcp(q.pII), kI = o.rcp(o.mul(q.rI, q.cI));
+        const double gpI = o.mul(g.gp, ipI), c2 = o.mul(o.mul(2.0, g.inv_g1), q.cII);
         ok = false;
         for (int k = 0; k < 4; k++) {
-            const double fI = mul(mul(sub(p, q.pI), kI), rsqrt(fma(gpI, p, g.gm)));
-            const double f = fma(c2, sub(pow_gm(g, mul(p, ipII)), 1.0), sub(fI, q.Udf));
+            const double fI = o.mul(o.mul(o.sub(p, q.pI), kI), o.rsqrt(fma(gpI, p, g.gm)));
+            const double f = fma(c2, o.sub(pow_gm(g, o.mul(p, ipII)), 1.0), o.sub(fI, q.Udf));
             float dummy;
             eval(low_float(p), dummy, df);
             if (bad(df)) break;
             const float step = (float)f / df;
-            p = sub(p, (double)step);
+            p = o.sub(p, (double)step);
             if (fabsf(step) <= 3e-7f * pf) {
                 ok = bits(p) >= bits(q.pI) && bits(p) <= bits(q.pII);
                 break;
@@ -273,7 +272,7 @@ __device__ __forceinline__ double bisect_p64(const Gas<double>& g, const RPre<do
     if (!ok) return solve_exact(g, q, rc);
     // iterates outside (lo, hi) are far from the stopping test
     const double far = (double)(8.0f * (tolf + band) / df);
-    const long long lo = key(sub(p, far)), hi = key(add(p, far));
+    const long long lo = key(o.sub(p, far)), hi = key(o.add(p, far));
     auto near = [&](double x) { return bits(x) > lo && bits(x) < hi; };
     auto residual = [&](double x) {
         return lev_exact(g, q.enI, q.pI, q.rI, q.cI, q.enII, q.pII, q.cII, x);
@@ -286,10 +285,10 @@ __device__ __forceinline__ double bisect_p64(const Gas<double>& g, const RPre<do
     for (;;) {
         it++;
         // (kl + kp)/2: the sum's exponent less one
-        kc = from(bits(add(kl, kp)) - (1ll << 52));
+        kc = from(bits(o.add(kl, kp)) - (1ll << 52));
         bool above = bits(kc) > bits(p);
         if (near(kc)) {
-            const float d = fabsf((float)sub(kc, p)), est = d * df, err = band + 2.0f * est * (d / pf) + 4e-6f * est;
+            const float d = fabsf((float)o.sub(kc, p)), est = d * df, err = band + 2.0f * est * (d / pf) + 4e-6f * est;
             if (est + err <= tolf) break;
             if (!(est - err > tolf)) {
                 const double f = residual(kc);
@@ -314,10 +313,11 @@ __device__ __forceinline__ double bisect_p64(const Gas<double>& g, const RPre<do
 __device__ __forceinline__ double newton_p64(const Gas<double>& g, const RPre<double>& q, RiemannCount& rc)
 {
     using namespace d64;
+    const Pipe o(g);
     if (g.max_iter < 16 || g.tol > 1e-7) return solve_exact(g, q, rc);
-    const double kI = rcp(mul(q.rI, q.cI)), kII = rcp(mul(q.rII, q.cII));
-    const double gI = mul(g.gp, rcp(q.pI)), gII = mul(g.gp, rcp(q.pII));
-    double pn = mul(fma(q.pI, kI, fma(q.pII, kII, q.Udf)), rcp(add(kI, kII)));
+    const double kI = o.rcp(o.mul(q.rI, q.cI)), kII = o.rcp(o.mul(q.rII, q.cII));
+    const double gI = o.mul(g.gp, o.rcp(q.pI)), gII = o.mul(g.gp, o.rcp(q.pII));
+    double pn = o.mul(fma(q.pI, kI, fma(q.pII, kII, q.Udf)), o.rcp(o.add(kI, kII)));
     // (p_I/(rho_I c_I) + p_II/(rho_II c_II) + Udf)/(1/(rho_I c_I) + 1/(rho_II c_II)), the reference's with both
     // terms divided by the impedances' product
     const float kIf = low_float(kI), kIIf = low_float(kII), tolp = fmaxf((float)g.tol * low_float(pn), 1.2e-38f);
@@ -328,8 +328,8 @@ __device__ __forceinline__ double newton_p64(const Gas<double>& g, const RPre<do
         const double p = pn;
         k++;
         const double qI = fma(gI, p, g.gm), qII = fma(gII, p, g.gm);
-        const double sI = rsqrt(qI), sII = rsqrt(qII);
-        const double f = fma(mul(sub(p, q.pI), kI), sI, fma(mul(sub(p, q.pII), kII), sII, -q.Udf));
+        const double sI = o.rsqrt(qI), sII = o.rsqrt(qII);
+        const double f = fma(o.mul(o.sub(p, q.pI), kI), sI, fma(o.mul(o.sub(p, q.pII), kII), sII, -q.Udf));
         const float uI = low_float(sI), uII = low_float(sII);
         // (gamma + 1) p/p_K + b from q_K = gp p/p_K + gm
         const float dI = (gg * (low_float(qI) - gmf) + b) * ga4 * uI * uI * uI * kIf;
@@ -337,7 +337,7 @@ __device__ __forceinline__ double newton_p64(const Gas<double>& g, const RPre<do
         const float df = dI + dII;
         if (!(df > 1e-30f && df < 1e30f)) return solve_exact(g, q, rc);   // FP32 does not hold it
         const float step = (float)f / df;
-        pn = sub(p, (double)step);
+        pn = o.sub(p, (double)step);
         if (!(fabsf(step) >= tolp)) break;
         if (k >= g.max_iter) { rc.status |= 0x04u; break; }
     }
@@ -353,56 +353,58 @@ __device__ __forceinline__ void godunov_flux64(const Gas<double>& g, bool swap, 
                                                double te, double F[4])
 {
     using namespace d64;
+    const Pipe o(g);
     en = sel(swap, -en, en);
-    const double m = mul(r, en);
+    const double m = o.mul(r, en);
     F[0] = m;
     F[1] = fma(m, en, p);
-    F[2] = mul(m, te);
+    F[2] = o.mul(m, te);
     // en (e + p), e + p = ga p/(ga - 1) + r (en^2 + te^2)/2
-    F[3] = fma(mul(0.5, m), fma(en, en, mul(te, te)), mul(mul(mul(g.ga, g.inv_g1), p), en));
+    F[3] = fma(o.mul(o.half, m), fma(en, en, o.mul(te, te)), o.mul(o.mul(o.mul(g.ga, g.inv_g1), p), en));
 }
 
 // godunov_sample (physics.cuh) of patterns 1, 2 and 3 at w = 0
 __device__ __forceinline__ double godunov_sample64(const Gas<double>& g, const RPre<double>& q, double p, double F[4])
 {
     using namespace d64;
+    const Pipe o(g);
     const bool two_raref = q.pattern == 1, shockII = q.pattern == 3;
     // mass-flux coefficients of the two waves
     double aI, aII;
     if (two_raref) {
         // p* in closed form: (p*/pI)^gm = B, (p*/pII)^gm = B (pI/pII)^gm
-        const double B = mul(sub(q.Udf, q.Uvk), rcp(sub(q.Urz, q.Uvk)));
-        p = mul(q.pI, ipow(B, g.n));
-        aI = rare_coef_y(g, mul(q.rI, q.cI), B, p, q.pI);
+        const double B = o.mul(o.sub(q.Udf, q.Uvk), o.rcp(o.sub(q.Urz, q.Uvk)));
+        p = o.mul(q.pI, ipow(o, B, g.n));
+        aI = rare_coef_y(g, o.mul(q.rI, q.cI), B, p, q.pI);
         // (pI/pII)^gm = 1 + Urz (gamma - 1)/(2 cII)
-        aII = rare_coef_y(g, mul(q.rII, q.cII), mul(B, fma(mul(q.Urz, g.hg1), rcp(q.cII), 1.0)), p, q.pII);
+        aII = rare_coef_y(g, o.mul(q.rII, q.cII), o.mul(B, fma(o.mul(q.Urz, g.hg1), o.rcp(q.cII), 1.0)), p, q.pII);
     } else {
-        const double x = mul(q.rI, fma(g.hg2, p, mul(g.hg1, q.pI)));
-        aI = mul(x, rsqrt(x));
+        const double x = o.mul(q.rI, fma(g.hg2, p, o.mul(g.hg1, q.pI)));
+        aI = o.mul(x, o.rsqrt(x));
         if (shockII) {
-            const double z = mul(q.rII, fma(g.hg2, p, mul(g.hg1, q.pII)));
-            aII = mul(z, rsqrt(z));
+            const double z = o.mul(q.rII, fma(g.hg2, p, o.mul(g.hg1, q.pII)));
+            aII = o.mul(z, o.rsqrt(z));
         } else {
-            const double z = mul(p, rcp(q.pII));
-            if (g.n) aII = rare_coef_y(g, mul(q.rII, q.cII), pow_gm(g, z), p, q.pII);
+            const double z = o.mul(p, o.rcp(q.pII));
+            if (g.n) aII = rare_coef_y(g, o.mul(q.rII, q.cII), pow_gm(g, z), p, q.pII);
             else aII = rare_coef(g, q.rII, q.cII, p, q.pII);
         }
     }
-    const double u = mul(fma(aI, q.enI, fma(aII, q.enII, sub(q.pI, q.pII))), rcp(add(aI, aII)));
+    const double u = o.mul(fma(aI, q.enI, fma(aII, q.enII, o.sub(q.pI, q.pII))), o.rcp(o.add(aI, aII)));
     // heads (d) and tails (dd) of the two waves; a shock is both
-    const double wI = sub(q.enI, u), wII = sub(q.enII, u);
+    const double wI = o.sub(q.enI, u), wII = o.sub(q.enII, u);
     double dI, ddI, dII, ddII;
     if (two_raref) {
-        dI = sub(q.enI, q.cI);
-        ddI = fma(-g.hg1, wI, sub(u, q.cI));
+        dI = o.sub(q.enI, q.cI);
+        ddI = fma(-g.hg1, wI, o.sub(u, q.cI));
     } else {
-        dI = ddI = fma(-aI, rcp(q.rI), q.enI);
+        dI = ddI = fma(-aI, o.rcp(q.rI), q.enI);
     }
     if (shockII) {
-        dII = ddII = fma(aII, rcp(q.rII), q.enII);
+        dII = ddII = fma(aII, o.rcp(q.rII), q.enII);
     } else {
-        dII = add(q.enII, q.cII);
-        ddII = fma(-g.hg1, wII, add(u, q.cII));
+        dII = o.add(q.enII, q.cII);
+        ddII = fma(-g.hg1, wII, o.add(u, q.cII));
     }
     const double UU = max_pos(max_abs(dI, dII), max_abs(ddI, ddII));
     // the interval that holds w = 0
@@ -417,10 +419,10 @@ __device__ __forceinline__ double godunov_sample64(const Gas<double>& g, const R
     } else if (key(dd) > key(0.0)) {
         // inside a rarefaction fan
         const double e = sel(left, en0, -en0);
-        const double ce = mul(fma(g.g1, e, mul(2.0, c0)), rcp(g.g2));
-        ps = mul(p0, pow_inv_gm(g, mul(ce, rcp(c0))));
-        const double ic = rcp(ce);
-        r = mul(mul(mul(g.ga, ps), ic), ic);
+        const double ce = o.mul(fma(g.g1, e, o.mul(2.0, c0)), o.rcp(g.g2));
+        ps = o.mul(p0, pow_inv_gm(g, o.mul(ce, o.rcp(c0))));
+        const double ic = o.rcp(ce);
+        r = o.mul(o.mul(o.mul(g.ga, ps), ic), ic);
         en = sel(left, ce, -ce);
     } else {
         // between the wave and the contact
@@ -428,10 +430,10 @@ __device__ __forceinline__ double godunov_sample64(const Gas<double>& g, const R
         ps = p;
         en = u;
         if (left ? !two_raref : shockII) {
-            r = mul(mul(r0, a), rcp(fma(-r0, w, a)));
+            r = o.mul(o.mul(r0, a), o.rcp(fma(-r0, w, a)));
         } else {
-            const double ic = rcp(fma(g.hg1, w, c0));
-            r = mul(mul(mul(g.ga, p), ic), ic);
+            const double ic = o.rcp(fma(g.hg1, w, c0));
+            r = o.mul(o.mul(o.mul(g.ga, p), ic), ic);
         }
     }
     godunov_flux64(g, q.swap, r, ps, en, te, F);

@@ -52,7 +52,10 @@ inline int sm_count()
 // must happen outside stream capture (ast_create, ast_step_raw).  The FP64
 // solver on a small grid (fewer 32x16 tiles than two per SM) steps with
 // 16x16 tiles: twice the CTAs with half the cells each, since there every
-// CTA runs alone on its SM at the FP64 rate.  P.band_hi > 0 launches the
+// CTA runs alone on its SM at the FP64 rate.  The exact solver does so up to
+// eight tiles per SM: its disturbed tiles cost many times the others, and
+// the step waits for the SM that holds the most of them (1021x509 blast, 8
+// steps: 2.27 ms with 32x16 tiles, 1.98 ms with 16x16).  P.band_hi > 0 launches the
 // tile rows [band_lo, band_hi) only (both tile shapes are 16 rows high), and
 // every tile of the grid counts towards the step's clock.
 template <typename R, int FLUX, bool RECON, int LAYOUT>
@@ -80,7 +83,7 @@ int launch_step_t(const StepParams& P, cudaStream_t st, bool launch)
     StepParams Q = P;
     const long long tiles = (long long)((P.N + kTZ - 1) / kTZ) * rows;
     if constexpr (kSmallTiles) {
-        if (tiles < 2LL * sm_count()) {
+        if (tiles < (FLUX == 2 ? 8LL : 2LL) * sm_count()) {
             dim3 grid((P.N + kSZ - 1) / kSZ, band);
             if (P.band_hi > 0) Q.units = (int)grid.x * rows;
             step_kernel<R, FLUX, RECON, LAYOUT, kSZ, kSR>
@@ -387,6 +390,19 @@ inline void fill_step_params(StepParams& P, const ast_config& c)
     P.body_hi = c.body_hi;
     P.body_rsplit = c.body_rsplit;
     P.body_amp = c.body_amp;
+    P.body_nlo = 0;
+    P.body_nhi = -1;
+    P.body_mlo = c.M;
+    if (c.body_force) {
+        // x and r grow with n and m, so each set is one interval
+        for (int n = 0; n < c.N; n++) {
+            const double x = std::fma((double)n, P.dx, P.x_min);
+            if (!(x > c.body_lo && x < c.body_hi)) continue;
+            if (P.body_nhi < 0) P.body_nlo = n;
+            P.body_nhi = n;
+        }
+        for (int m = c.M - 1; m >= 0 && std::fma((double)m, P.dy, P.y_min) >= c.body_rsplit; m--) P.body_mlo = m;
+    }
     P.nsrc = nullptr;   // set by ast_set_neutral / ast_add_mk_raw
     P.nsrc_coef = (c.neutral_kn != 0.0) ? c.neutral_nh / c.neutral_kn : 0.0;
 }

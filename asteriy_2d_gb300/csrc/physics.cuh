@@ -36,6 +36,7 @@ struct Gas {
     R hg1, hg2;               // (gamma-1)/2, (gamma+1)/2
     int max_iter;
     int n;                    // 1/gm when it is a whole number from 2 to 16, else 0
+    int zero;                 // 0, unknown to the compiler (d64::Pipe)
 };
 
 template <typename R>
@@ -58,6 +59,7 @@ __host__ __device__ inline Gas<R> make_gas(double gamma, double tol, int max_ite
     const double n = 2.0 * gamma / g1;
     const int ni = (n > 1.5 && n < 16.5) ? (int)(n + 0.5) : 0;
     g.n = (ni > 0 && n - ni < 1e-14 * n && ni - n < 1e-14 * n) ? ni : 0;
+    g.zero = 0;
     return g;
 }
 
@@ -97,23 +99,6 @@ __device__ __forceinline__ double minmod_d(double a, double b)
     return __longlong_as_double(((m < 0) ? 0ll : m) | sa);
 }
 
-// left / right face values of a cell from its three-point stencil; the
-// reference's linear2 with the coordinate differences folded in
-template <typename R>
-__device__ __forceinline__ void recon_pair(R tm, R t0, R tp, R& left, R& right)
-{
-    if constexpr (sizeof(R) == 8) {
-        // half the slope in the multiply-add: one FP64 operation per value
-        const R m = minmod_d(t0 - tm, tp - t0);
-        left = fma(m, R(-0.5), t0);
-        right = fma(m, R(0.5), t0);
-    } else {
-        R d = minmod_d(t0 - tm, tp - t0) * R(0.5);
-        left = t0 - d;
-        right = t0 + d;
-    }
-}
-
 // ------------------------------------------------------------------ FP64 arithmetic for a narrow pipe
 // GB300 issues one FP64 warp instruction per SM every 17-20 cycles (measured:
 // fma 17, add and mul 20, a compare-and-select 20, fmin 40; each waits 92
@@ -124,16 +109,13 @@ __device__ __forceinline__ void recon_pair(R tm, R t0, R tp, R& left, R& right)
 // (64-bit integer minimum: 0.4 cycles), and reciprocals and sound speeds
 // start from the approximation instructions (20 bits, 2 cycles) and take one
 // third-order step of the binomial series (Householder's iteration) instead
-// of a division (150 cycles) and a square root (150).  Written with explicit
-// roundings (fma, __dadd_rn, __dmul_rn) so that every kernel that inlines
-// them gives the same bits.
+// of a division (150 cycles) and a square root (150).  Every sum and product
+// is an explicit fma, so that every kernel that inlines them gives the same
+// bits.
 namespace d64 {
 constexpr long long kSign = (long long)0x8000000000000000ull;
 __device__ __forceinline__ long long bits(double a) { return __double_as_longlong(a); }
 __device__ __forceinline__ double from(long long a) { return __longlong_as_double(a); }
-__device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
-__device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
-__device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double abs(double a) { return from(bits(a) & ~kSign); }
 __device__ __forceinline__ bool neg(double a) { return __double2hiint(a) < 0; }   // the sign bit
 __device__ __forceinline__ double sel(bool c, double a, double b) { return from(c ? bits(a) : bits(b)); }
@@ -160,28 +142,72 @@ constexpr int kLo = (1023 - 150) << 20, kHi = (1023 + 150) << 20;
 __device__ __forceinline__ bool tame_pos(double a) { return (unsigned)(__double2hiint(a) - kLo) < (unsigned)(kHi - kLo); }
 __device__ __forceinline__ bool tame(double a) { return (__double2hiint(a) & 0x7fffffff) < kHi; }
 
-// 1/x of a normal number well inside the range: with y0 = (1 + d)/x and
-// e = 1 - x y0, 1/x = y0 (1 + e + e^2 + ...), cut after e^2 (|e| < 2^-19)
-__device__ __forceinline__ double rcp(double x)
-{
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x, y, 1.0);
-    return fma(y, fma(e, e, e), y);
-}
-// sqrt(a / r) of tame a and r as a (a r)^(-1/2): with y0 the approximate
-// inverse root of x = a r and e = 1 - x y0^2, x^(-1/2) = y0 (1 + e/2 +
-// 3 e^2/8 + ...), cut after e^2
-__device__ __forceinline__ double sqrt_ratio(double a, double r)
-{
-    const double x = mul(a, r);
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-mul(x, y), y, 1.0);
-    const double w = mul(a, y);
-    return fma(w, mul(e, fma(e, 0.375, 0.5)), w);
-}
+// Sums and products as fused multiply-adds of three different registers, the
+// same values: a + b = a 1 + b, a b = a b + (-0).  An FP64 instruction with
+// three register operands issues every 16 cycles, one with an immediate, a
+// constant or the same register twice every 19-20 (measured), so the factors
+// are kept in registers, where the compiler cannot see their values (g.zero).
+struct Pipe {
+    double one, half, nz;
+    __device__ __forceinline__ explicit Pipe(const Gas<double>& g)
+    {
+        one = from((long long)(0x3ff00000 + g.zero) << 32);
+        half = from((long long)(0x3fe00000 + g.zero) << 32);
+        nz = from((long long)((int)0x80000000 + g.zero) << 32);
+    }
+    __device__ __forceinline__ double add(double a, double b) const { return fma(a, one, b); }
+    __device__ __forceinline__ double sub(double a, double b) const { return fma(-b, one, a); }
+    __device__ __forceinline__ double mul(double a, double b) const { return fma(a, b, nz); }
+    // 1/x of a normal number well inside the range: with y0 = (1 + d)/x and
+    // e = 1 - x y0, 1/x = y0 (1 + e + e^2 + ...), cut after e^2 (|e| < 2^-19)
+    __device__ __forceinline__ double rcp(double x) const
+    {
+        double y;
+        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+        const double e = fma(-x, y, one);
+        return fma(y, fma(e, e, e), y);
+    }
+    // sqrt(a / r) of tame a and r as a (a r)^(-1/2): with y0 the approximate
+    // inverse root of x = a r and e = 1 - x y0^2, x^(-1/2) = y0 (1 + e/2 +
+    // 3 e^2/8 + ...), cut after e^2
+    __device__ __forceinline__ double sqrt_ratio(double a, double r) const
+    {
+        const double x = mul(a, r);
+        double y;
+        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+        const double e = fma(-mul(x, y), y, one);
+        const double w = mul(a, y);
+        return fma(w, mul(e, fma(e, 0.375, half)), w);
+    }
+    // x^(-1/2) of a normal x, the same step
+    __device__ __forceinline__ double rsqrt(double x) const
+    {
+        double y;
+        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+        const double e = fma(-mul(x, y), y, one);
+        return fma(y, mul(e, fma(e, 0.375, half)), y);
+    }
+};
+
 }  // namespace d64
+
+// left / right face values of a cell from its three-point stencil; the
+// reference's linear2 with the coordinate differences folded in
+__device__ __forceinline__ void recon_pair(const Gas<float>&, float tm, float t0, float tp, float& left, float& right)
+{
+    const float d = minmod_d(t0 - tm, tp - t0) * 0.5f;
+    left = t0 - d;
+    right = t0 + d;
+}
+// FP64: half the slope in the multiply-add, one operation per value
+__device__ __forceinline__ void recon_pair(const Gas<double>& g, double tm, double t0, double tp, double& left,
+                                           double& right)
+{
+    const d64::Pipe o(g);
+    const double m = minmod_d(o.sub(t0, tm), o.sub(tp, t0));
+    left = fma(-m, o.half, t0);
+    right = fma(m, o.half, t0);
+}
 
 // ------------------------------------------------------------------ HLL
 // the reference's formula (FP32, and FP64 states outside the short form's range)
@@ -249,8 +275,9 @@ __device__ __forceinline__ bool face_tame(double rL, double pL, double unL, doub
 __device__ __forceinline__ double sound_max(const Gas<double>& g, double rL, double pL, double rR, double pR)
 {
     using namespace d64;
-    const bool l = bits(mul(pL, rR)) >= bits(mul(pR, rL));
-    return sqrt_ratio(mul(g.ga, sel(l, pL, pR)), sel(l, rL, rR));
+    const Pipe o(g);
+    const bool l = bits(o.mul(pL, rR)) >= bits(o.mul(pR, rL));
+    return o.sqrt_ratio(o.mul(g.ga, sel(l, pL, pR)), sel(l, rL, rR));
 }
 static __device__ __noinline__ WildFlux flux_hll_wild(const Gas<double>& g, double rL, double pL, double unL, double utL,
                                                        double rR, double pR, double unR, double utR)
@@ -271,20 +298,21 @@ __device__ __forceinline__ double flux_hll_of(const Gas<double>& g, double c, do
                                               double utL, double rR, double pR, double unR, double utR, double F[4])
 {
     using namespace d64;
-    const double DL = sub(min(unL, unR), c), DR = add(max(unL, unR), c);
+    const Pipe o(g);
+    const double DL = o.sub(min(unL, unR), c), DR = o.add(max(unL, unR), c);
     const double SL = sel(neg(DL), DL, 0.0), SR = sel(neg(DR), 0.0, DR);
-    const double inv = rcp(sub(SR, SL));
-    const double a = sel(neg(DL), mul(SR, inv), 1.0), b = sel(neg(DR), 1.0, mul(-SL, inv));
-    const double A = mul(a, sub(unL, SL)), B = mul(b, sub(unR, SR));
-    const double mL = mul(A, rL), mR = mul(B, rR);
-    const double PL = mul(a, pL), PR = mul(b, pR);
-    F[0] = add(mL, mR);
-    F[1] = fma(mL, unL, fma(mR, unR, add(PL, PR)));
-    F[2] = fma(mL, utL, mul(mR, utR));
-    const double qL = fma(unL, unL, mul(utL, utL)), qR = fma(unR, unR, mul(utR, utR));
-    const double k = fma(mL, qL, mul(mR, qR));
-    const double h = fma(mul(A, pL), g.inv_g1, mul(PL, unL));
-    F[3] = fma(0.5, k, fma(mul(B, pR), g.inv_g1, fma(PR, unR, h)));
+    const double inv = o.rcp(o.sub(SR, SL));
+    const double a = sel(neg(DL), o.mul(SR, inv), 1.0), b = sel(neg(DR), 1.0, o.mul(-SL, inv));
+    const double A = o.mul(a, o.sub(unL, SL)), B = o.mul(b, o.sub(unR, SR));
+    const double mL = o.mul(A, rL), mR = o.mul(B, rR);
+    const double PL = o.mul(a, pL), PR = o.mul(b, pR);
+    F[0] = o.add(mL, mR);
+    F[1] = fma(mL, unL, fma(mR, unR, o.add(PL, PR)));
+    F[2] = fma(mL, utL, o.mul(mR, utR));
+    const double qL = fma(unL, unL, o.mul(utL, utL)), qR = fma(unR, unR, o.mul(utR, utR));
+    const double k = fma(mL, qL, o.mul(mR, qR));
+    const double h = fma(o.mul(A, pL), g.inv_g1, o.mul(PL, unL));
+    F[3] = fma(o.half, k, fma(o.mul(B, pR), g.inv_g1, fma(PR, unR, h)));
     return max_abs(DL, DR);
 }
 __device__ __forceinline__ double flux_hll(const Gas<double>& g, double rL, double pL, double unL, double utL,
@@ -331,17 +359,18 @@ __device__ __forceinline__ double flux_physical(const Gas<double>& g, double r, 
                                                 double F[4])
 {
     using namespace d64;
+    const Pipe o(g);
     if (!(tame_pos(r) && tame_pos(p) && tame(un) && tame(ut)))
         return flux_physical_wild(g, r, p, un, ut).get(F);
-    const double c = sqrt_ratio(mul(g.ga, p), r);
-    const double m = mul(r, un);
+    const double c = o.sqrt_ratio(o.mul(g.ga, p), r);
+    const double m = o.mul(r, un);
     F[0] = m;
     F[1] = fma(m, un, p);
-    F[2] = mul(m, ut);
+    F[2] = o.mul(m, ut);
     // (e + p) un, e + p = ga p/(ga - 1) + r q/2
-    const double q = fma(un, un, mul(ut, ut));
-    F[3] = fma(mul(0.5, m), q, mul(mul(mul(g.ga, p), g.inv_g1), un));
-    return max_abs(sub(un, c), add(un, c));
+    const double q = fma(un, un, o.mul(ut, ut));
+    F[3] = fma(o.mul(o.half, m), q, o.mul(o.mul(o.mul(g.ga, p), g.inv_g1), un));
+    return max_abs(o.sub(un, c), o.add(un, c));
 }
 
 // ------------------------------------------------------------------ HLL, two faces in packed FP32
@@ -399,7 +428,7 @@ __device__ __forceinline__ void flux_hll_x2(const Gas<float>& g, float2 rL, floa
 // evaluation serves z faces (tangent +v_r) and r faces (the reference's
 // tangent there is -v_z, its flux rotated back by the same sign).
 template <typename R>
-__device__ __forceinline__ R flux_hllc_a(const Gas<R>& g, R r1, R p1, R un1, R ut1, R r2, R p2, R un2, R ut2,
+__device__ __forceinline__ R flux_hllc_a_ref(const Gas<R>& g, R r1, R p1, R un1, R ut1, R r2, R p2, R un2, R ut2,
                                          R F[4])
 {
     const R cL = sqrt(g.ga * p1 / r1), cR = sqrt(g.ga * p2 / r2);
@@ -501,37 +530,52 @@ static __device__ __noinline__ WildFlux flux_hllc_wild(const Gas<double>& g, dou
     w.S = flux_hllc_ref(g, rL, pL, u1, v1, rR, pR, u2, v2, w.F);
     return w;
 }
-// The HLLC flux in 46 FP64 operations (the formula above compiles to about
-// 110).  The side K that the contact leaves behind is selected before its
-// star state is formed, and the flux is taken as the star state's own,
+// The HLLC flux of given wave bounds SL < SR in 39 FP64 operations (with
+// sound_max and the bounds below 51; the formula above compiles to about 110).
+// The side K that the contact leaves behind is selected before its star state
+// is formed, and the flux is taken as the star state's own,
 //   rho* SM (1, SM, v_K, .) + p* (0, 1, 0, .),  (E* + p*) SM,
 // rho* = rho_K (S_K - u_K)/(S_K - SM), which equals F_K + S_K (U* - U_K);
-// a supersonic face is its upwind side with SM = u_K and rho* = rho_K.
-__device__ __forceinline__ double flux_hllc_of(const Gas<double>& g, double c, double rL, double pL, double u1,
-                                               double v1, double rR, double pR, double u2, double v2, double F[4])
+// a supersonic face is its upwind side with SM = u_K and rho* = rho_K.  p* is
+// the mean of both sides' (MEAN) or the left side's.  FQ, when wanted: the
+// flux of a passive scalar Q* = Q (S_K - u_K)/(S_K - SM).
+template <bool MEAN>
+__device__ __forceinline__ double flux_star(const Gas<double>& g, double SL, double SR, double rL, double pL, double u1,
+                                            double v1, double rR, double pR, double u2, double v2, double F[4],
+                                            double QL = 0.0, double QR = 0.0, double* FQ = nullptr)
 {
     using namespace d64;
-    const double SL = sub(min(u1, u2), c), SR = add(max(u1, u2), c);
-    const double wL = sub(SL, u1), wR = sub(SR, u2);
-    const double aL = mul(rL, wL), aR = mul(rR, wR);     // aL < 0 < aR
-    const double num = fma(aR, u2, fma(-aL, u1, sub(pL, pR)));
-    const double SM = mul(num, rcp(sub(aR, aL)));
-    const double ptz = mul(0.5, add(fma(aR, sub(SM, u2), pR), fma(aL, sub(SM, u1), pL)));
+    const Pipe o(g);
+    const double wL = o.sub(SL, u1), wR = o.sub(SR, u2);
+    const double aL = o.mul(rL, wL), aR = o.mul(rR, wR);     // aL < 0 < aR
+    const double num = fma(aR, u2, fma(-aL, u1, o.sub(pL, pR)));
+    const double SM = o.mul(num, o.rcp(o.sub(aR, aL)));
+    const double psL = fma(aL, o.sub(SM, u1), pL);
+    const double ptz = MEAN ? o.mul(o.half, o.add(fma(aR, o.sub(SM, u2), pR), psL)) : psL;
     // SL >= 0, then SR <= 0, then the side of the contact
     const bool supL = bits(SL) >= 0, supR = bits(SR) <= 0;
     const bool left = supL || (!supR && bits(SM) >= 0), sup = supL || supR;
     const double r = sel(left, rL, rR), p = sel(left, pL, pR), u = sel(left, u1, u2), v = sel(left, v1, v2);
     const double S = sel(left, SL, SR), w = sel(left, wL, wR), a = sel(left, aL, aR);
-    const double inv = rcp(sub(S, SM));
-    const double q = fma(u, u, mul(v, v));
-    const double e = fma(p, g.inv_g1, mul(mul(0.5, r), q));
-    const double es = mul(fma(e, w, fma(ptz, SM, -mul(p, u))), inv);
+    const double inv = o.rcp(o.sub(S, SM));
+    const double q = fma(u, u, o.mul(v, v));
+    const double e = fma(p, g.inv_g1, o.mul(o.mul(o.half, r), q));
+    const double es = o.mul(fma(e, w, fma(ptz, SM, -o.mul(p, u))), inv);
     const double um = sel(sup, u, SM), pm = sel(sup, p, ptz);
-    F[0] = mul(sel(sup, r, mul(a, inv)), um);
+    F[0] = o.mul(sel(sup, r, o.mul(a, inv)), um);
     F[1] = fma(F[0], um, pm);
-    F[2] = mul(F[0], v);
-    F[3] = mul(add(sel(sup, e, es), pm), um);
+    F[2] = o.mul(F[0], v);
+    F[3] = o.mul(o.add(sel(sup, e, es), pm), um);
+    if (FQ) *FQ = o.mul(sel(left, QL, QR), sel(sup, u, o.mul(o.mul(w, inv), SM)));
     return max_abs(SL, SR);
+}
+// the bounds min u - c, max u + c with c the larger sound speed
+__device__ __forceinline__ double flux_hllc_of(const Gas<double>& g, double c, double rL, double pL, double u1,
+                                               double v1, double rR, double pR, double u2, double v2, double F[4])
+{
+    const d64::Pipe o(g);
+    return flux_star<true>(g, o.sub(d64::min(u1, u2), c), o.add(d64::max(u1, u2), c), rL, pL, u1, v1, rR, pR, u2, v2,
+                           F);
 }
 __device__ __forceinline__ double flux_hllc(const Gas<double>& g, double rL, double pL, double u1, double v1,
                                             double rR, double pR, double u2, double v2, double F[4])
@@ -582,7 +626,7 @@ __device__ __forceinline__ R flux_hllc_q(const Gas<R>& g, R rL, R pL, R u1, R QL
 // returns max(|S_L|, |S_R|), whose dt candidate the reference forms as
 // krit*rad/that.  Expression order as the reference's.
 template <typename R>
-__device__ __forceinline__ R flux_hllcq(const Gas<R>& g, R ro1, R p1, R u_L, R v_L, R Q_L, R ro2, R p2, R u_R, R v_R,
+__device__ __forceinline__ R flux_hllcq_ref(const Gas<R>& g, R ro1, R p1, R u_L, R v_L, R Q_L, R ro2, R p2, R u_R, R v_R,
                                         R Q_R, R F[4], R& FQ)
 {
     const R cL = sqrt(g.ga * p1 / ro1);
@@ -637,6 +681,63 @@ __device__ __forceinline__ R flux_hllcq(const Gas<R>& g, R ro1, R p1, R u_L, R v
         F[0] = F[1] = F[2] = F[3] = R(NAN);
     }
     return UU;
+}
+
+// FP32, and FP64 by the short form: both take the bounds min(u_L - c_L,
+// u_R - c_R) and max(u_L + c_L, u_R + c_R)
+__device__ __forceinline__ float flux_hllc_a(const Gas<float>& g, float r1, float p1, float un1, float ut1, float r2,
+                                             float p2, float un2, float ut2, float F[4])
+{
+    return flux_hllc_a_ref(g, r1, p1, un1, ut1, r2, p2, un2, ut2, F);
+}
+static __device__ __noinline__ WildFlux flux_hllc_a_wild(const Gas<double>& g, double r1, double p1, double un1,
+                                                         double ut1, double r2, double p2, double un2, double ut2)
+{
+    WildFlux w;
+    w.S = flux_hllc_a_ref(g, r1, p1, un1, ut1, r2, p2, un2, ut2, w.F);
+    return w;
+}
+__device__ __forceinline__ void own_bounds(const Gas<double>& g, double r1, double p1, double u1, double r2, double p2,
+                                           double u2, double& SL, double& SR)
+{
+    const d64::Pipe o(g);
+    const double cL = o.sqrt_ratio(o.mul(g.ga, p1), r1), cR = o.sqrt_ratio(o.mul(g.ga, p2), r2);
+    SL = d64::min(o.sub(u1, cL), o.sub(u2, cR));
+    SR = d64::max(o.add(u1, cL), o.add(u2, cR));
+}
+__device__ __forceinline__ double flux_hllc_a(const Gas<double>& g, double r1, double p1, double un1, double ut1,
+                                              double r2, double p2, double un2, double ut2, double F[4])
+{
+    if (!face_tame(r1, p1, un1, ut1, r2, p2, un2, ut2))
+        return flux_hllc_a_wild(g, r1, p1, un1, ut1, r2, p2, un2, ut2).get(F);
+    double SL, SR;
+    own_bounds(g, r1, p1, un1, r2, p2, un2, SL, SR);
+    return flux_star<true>(g, SL, SR, r1, p1, un1, ut1, r2, p2, un2, ut2, F);
+}
+struct WildFluxQ {
+    WildFlux f;
+    double FQ;
+};
+static __device__ __noinline__ WildFluxQ flux_hllcq_wild(const Gas<double>& g, double r1, double p1, double u1,
+                                                         double v1, double Q1, double r2, double p2, double u2,
+                                                         double v2, double Q2)
+{
+    WildFluxQ w;
+    w.f.S = flux_hllcq_ref(g, r1, p1, u1, v1, Q1, r2, p2, u2, v2, Q2, w.f.F, w.FQ);
+    return w;
+}
+__device__ __forceinline__ double flux_hllcq(const Gas<double>& g, double r1, double p1, double u1, double v1,
+                                             double Q1, double r2, double p2, double u2, double v2, double Q2,
+                                             double F[4], double& FQ)
+{
+    if (!face_tame(r1, p1, u1, v1, r2, p2, u2, v2)) {
+        const WildFluxQ w = flux_hllcq_wild(g, r1, p1, u1, v1, Q1, r2, p2, u2, v2, Q2);
+        FQ = w.FQ;
+        return w.f.get(F);
+    }
+    double SL, SR;
+    own_bounds(g, r1, p1, u1, r2, p2, u2, SL, SR);
+    return flux_star<false>(g, SL, SR, r1, p1, u1, v1, r2, p2, u2, v2, F, Q1, Q2, &FQ);
 }
 
 // ------------------------------------------------------------------ exact Riemann solver

@@ -75,9 +75,9 @@ __device__ __forceinline__ double face_q(const StepParams& P, const Gas<double>&
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             double x0, x1;
-            recon_pair(a0[k], a[k], b[k], x0, x1);
+            recon_pair(g, a0[k], a[k], b[k], x0, x1);
             L[k] = x1;
-            recon_pair(a[k], b[k], b1[k], x0, x1);
+            recon_pair(g, a[k], b[k], b1[k], x0, x1);
             U[k] = x0;
         }
         if (L[0] <= 0.0) L[0] = a[0];
@@ -85,9 +85,9 @@ __device__ __forceinline__ double face_q(const StepParams& P, const Gas<double>&
         if (L[1] <= 0.0 || !P.grad_p) L[1] = a[1];
         if (U[1] <= 0.0 || !P.grad_p) U[1] = b[1];
         double x0, x1;
-        recon_pair(qa0, qa, qb, x0, x1);
+        recon_pair(g, qa0, qa, qb, x0, x1);
         QL = (x1 <= 0.0) ? qa : x1;
-        recon_pair(qa, qb, qb1, x0, x1);
+        recon_pair(g, qa, qb, qb1, x0, x1);
         QU = (x0 <= 0.0) ? qb : x0;
     }
     if constexpr (FLUX == 4) {

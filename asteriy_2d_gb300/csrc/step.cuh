@@ -127,6 +127,10 @@ struct __align__(16) StepParams {
     int region_zlo, region_zhi, region_rlo, region_rhi;
     int body_force;
     double body_lo, body_hi, body_rsplit, body_amp;
+    // the cells of the body force (found on the host with the kernels' FP64
+    // positions): columns body_nlo .. body_nhi; rows from body_mlo on take
+    // the force of r >= body_rsplit
+    int body_nlo, body_nhi, body_mlo;
     // the neutral-coupling momentum source of add_MK: null, or per cell
     // (nn2.x, nn2.y) as two SoA planes of the state's precision and pitch
     // (solver) or the reference's double3 array (raw entry points); the
@@ -459,35 +463,36 @@ __device__ __forceinline__ void update_cell64(const Gas<double>& g, double p_flo
                                               int& np, unsigned& status, R out[4])
 {
     using namespace d64;
+    const Pipe o(g);
     const double r1 = (double)in[0], p1 = (double)in[1], vz1 = (double)in[2], vr1 = (double)in[3];
-    const double mz1 = mul(r1, vz1), mr1 = mul(r1, vr1);
-    const double E1 = fma(0.5, fma(mz1, vz1, mul(mr1, vr1)), mul(p1, g.inv_g1));
+    const double mz1 = o.mul(r1, vz1), mr1 = o.mul(r1, vr1);
+    const double E1 = fma(o.half, fma(mz1, vz1, o.mul(mr1, vr1)), o.mul(p1, g.inv_g1));
     double U[4] = {r1, mz1, mr1, E1};
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        const double fz = sub((double)f[k][0], (double)f[k][1]), fr = sub((double)f[k][3], (double)f[k][2]);
+        const double fz = o.sub((double)f[k][0], (double)f[k][1]), fr = o.sub((double)f[k][3], (double)f[k][2]);
         U[k] = fma(-tr, fr, fma(-tz, fz, U[k]));
     }
     if (axisym) {
-        const double w = mul(ty, mr1);
-        U[0] = sub(U[0], w);
+        const double w = o.mul(ty, mr1);
+        U[0] = o.sub(U[0], w);
         U[1] = fma(-w, vz1, U[1]);
         U[2] = fma(-w, vr1, U[2]);
-        U[3] = fma(-mul(ty, vr1), add(E1, p1), U[3]);
+        U[3] = fma(-o.mul(ty, vr1), o.add(E1, p1), U[3]);
     }
     if (body) {
         U[2] = fma(T_do, Q2, U[2]);
-        U[3] = fma(T_do, mul(Q2, vr1), U[3]);
+        U[3] = fma(T_do, o.mul(Q2, vr1), U[3]);
     }
     if (source) {
-        U[1] = add(U[1], Sz);
-        U[2] = add(U[2], Sr);
+        U[1] = o.add(U[1], Sz);
+        U[2] = o.add(U[2], Sr);
     }
     double rho2 = U[0];
     if (le_zero(rho2)) { nrho++; rho2 = r1; }
-    const double irho = tame_pos(rho2) ? rcp(rho2) : 1.0 / rho2;
-    const double vz2 = mul(U[1], irho), vr2 = mul(U[2], irho);
-    double p2 = mul(fma(-0.5, fma(U[1], vz2, mul(U[2], vr2)), U[3]), g.g1);
+    const double irho = tame_pos(rho2) ? o.rcp(rho2) : 1.0 / rho2;
+    const double vz2 = o.mul(U[1], irho), vr2 = o.mul(U[2], irho);
+    double p2 = o.mul(fma(-o.half, fma(U[1], vz2, o.mul(U[2], vr2)), U[3]), g.g1);
     if (le_zero(p2)) { np++; p2 = p_floor; }
     if (is_nan(p2)) status |= 0x10u;
     out[0] = (R)rho2; out[1] = (R)p2; out[2] = (R)vz2; out[3] = (R)vr2;
@@ -690,9 +695,9 @@ __device__ __forceinline__ bool face_states(const StepParams& P, const S& sm, in
 #pragma unroll
             for (int k = 0; k < 4; k++) {
                 R x0, x1;
-                recon_pair(tll[k], tl[k], tu[k], x0, x1);
+                recon_pair(gas_of<R>(P), tll[k], tl[k], tu[k], x0, x1);
                 L[k] = x1;                  // right/top value of the lower cell
-                recon_pair(tl[k], tu[k], tuu[k], x0, x1);
+                recon_pair(gas_of<R>(P), tl[k], tu[k], tuu[k], x0, x1);
                 U[k] = x0;                  // left/bottom value of the upper cell
             }
         }
@@ -949,7 +954,9 @@ __device__ __forceinline__ void face_two(const StepParams& P, S& sm, int b, cons
         R v[5];
         load5(k, v);
         L0[k] = v[1]; U0[k] = v[2]; L1[k] = v[2]; U1[k] = v[3];
-        if (RECON) {
+        // (FP64: first-order faces leave the slopes out; every face is in the
+        // high-order region unless region_select is on)
+        if (RECON && (sizeof(R) == 4 || hi0 || hi1)) {
             R x0, x1, y0, y1, z0, z1;
             // FP64: five cells of one bit pattern in every active lane of
             // the warp (undisturbed gas): every limited slope is +0, so the
@@ -967,9 +974,9 @@ __device__ __forceinline__ void face_two(const StepParams& P, S& sm, int b, cons
                 y1 = v[2] + R(0);
                 z0 = v[3];
             } else {
-                recon_pair(v[0], v[1], v[2], x0, x1);   // lower cell of the first face
-                recon_pair(v[1], v[2], v[3], y0, y1);   // the cell between the faces
-                recon_pair(v[2], v[3], v[4], z0, z1);   // upper cell of the second face
+                recon_pair(g, v[0], v[1], v[2], x0, x1);   // lower cell of the first face
+                recon_pair(g, v[1], v[2], v[3], y0, y1);   // the cell between the faces
+                recon_pair(g, v[2], v[3], v[4], z0, z1);   // upper cell of the second face
             }
             if (hi0) { L0[k] = x1; U0[k] = y0; }
             if (hi1) { L1[k] = y1; U1[k] = z0; }
@@ -1514,13 +1521,9 @@ __device__ __forceinline__ void tile_body(const StepParams& P, S& sm, int b, con
     // through the FP32 form's loop)
     auto update_fp64 = [&](int row, int n, const R in[4], const R f[4][4], R o[4]) {
         const double T_do = K.T_do;
-        const double y = sm.ydrow[row];
         double Q2 = 0.0, Sz = 0.0, Sr = 0.0;
-        if (P.body_force) {
-            const double x = P.x_min + n * P.dx;
-            if (x > P.body_lo && x < P.body_hi)
-                Q2 = (y >= P.body_rsplit) ? -P.body_amp * (double)in[0] : P.body_amp * (double)in[0];
-        }
+        const bool body = P.body_force && n >= P.body_nlo && n <= P.body_nhi;
+        if (body) Q2 = (m0 + row >= P.body_mlo) ? -P.body_amp * (double)in[0] : P.body_amp * (double)in[0];
         // the neutral-coupling source in the update (FP64 kernels; the FP32
         // form adds it in neutral_kernel after the step)
         if (sizeof(R) == 8 && P.nsrc) {
@@ -1530,8 +1533,8 @@ __device__ __forceinline__ void tile_body(const StepParams& P, S& sm, int b, con
             Sz = w * az;
             Sr = w * ar;
         }
-        const double ty = (sizeof(R) == 8) ? sm.tydrow[row] : ((P.geom == 1) ? T_do / y : 0.0);
-        update_cell64(P.gd, P.p_floor, P.geom == 1, in, f, T_do, K.tz, K.tr, ty, P.body_force != 0, Q2,
+        const double ty = (sizeof(R) == 8) ? sm.tydrow[row] : ((P.geom == 1) ? T_do / sm.ydrow[row] : 0.0);
+        update_cell64(P.gd, P.p_floor, P.geom == 1, in, f, T_do, K.tz, K.tr, ty, body, Q2,
                       sizeof(R) == 8 && P.nsrc != nullptr, Sz, Sr, acc.nrho, acc.np, acc.rc.status, o);
     };
     // the FP32 form's source terms of a cell: ty = T_do/r and the body force

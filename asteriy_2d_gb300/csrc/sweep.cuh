@@ -78,7 +78,7 @@ __device__ __forceinline__ void sw_recon(const StepParams& P, const float a[4], 
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         if (RECON) {
-            recon_pair(a[k], t[k], b[k], lo[k], hi[k]);
+            recon_pair(P.gf, a[k], t[k], b[k], lo[k], hi[k]);
         } else {
             lo[k] = t[k];
             hi[k] = t[k];
