@@ -71,7 +71,7 @@ __device__ __forceinline__ double pow_gm(const Gas<double>& g, double x)
     const Pipe o(g);
     if (g.n == 0) return pow(x, g.gm);
     const double w = (double)exp2f(-(float)g.gm * log2f(low_float(x)));
-    const double e = fma(-x, ipow(o, w, g.n), 1.0);
+    const double e = fma(flip(x), ipow(o, w, g.n), o.one);
     return o.rcp(fma(w, o.mul(e, fma(e, o.mul(o.mul(o.half, g.gm), o.add(g.gm, 1.0)), g.gm)), w));
 }
 // x^(1/gm)
@@ -98,11 +98,11 @@ __device__ __forceinline__ RPre<double> godunov_sides64(const Gas<double>& g, do
     const Pipe o(g);
     RPre<double> q;
     q.swap = bits(pL) > bits(pR);
-    q.enI = sel(q.swap, -unR, unL);
+    q.enI = sel(q.swap, flip(unR), unL);
     q.teI = sel(q.swap, utR, utL);
     q.pI = sel(q.swap, pR, pL);
     q.rI = sel(q.swap, rR, rL);
-    q.enII = sel(q.swap, -unL, unR);
+    q.enII = sel(q.swap, flip(unL), unR);
     q.teII = sel(q.swap, utL, utR);
     q.pII = sel(q.swap, pL, pR);
     q.rII = sel(q.swap, rL, rR);
@@ -329,7 +329,7 @@ __device__ __forceinline__ double newton_p64(const Gas<double>& g, const RPre<do
         k++;
         const double qI = fma(gI, p, g.gm), qII = fma(gII, p, g.gm);
         const double sI = o.rsqrt(qI), sII = o.rsqrt(qII);
-        const double f = fma(o.mul(o.sub(p, q.pI), kI), sI, fma(o.mul(o.sub(p, q.pII), kII), sII, -q.Udf));
+        const double f = fma(o.mul(o.sub(p, q.pI), kI), sI, fma(o.mul(o.sub(p, q.pII), kII), sII, flip(q.Udf)));
         const float uI = low_float(sI), uII = low_float(sII);
         // (gamma + 1) p/p_K + b from q_K = gp p/p_K + gm
         const float dI = (gg * (low_float(qI) - gmf) + b) * ga4 * uI * uI * uI * kIf;
@@ -354,7 +354,7 @@ __device__ __forceinline__ void godunov_flux64(const Gas<double>& g, bool swap, 
 {
     using namespace d64;
     const Pipe o(g);
-    en = sel(swap, -en, en);
+    en = sel(swap, flip(en), en);
     const double m = o.mul(r, en);
     F[0] = m;
     F[1] = fma(m, en, p);
@@ -396,41 +396,41 @@ __device__ __forceinline__ double godunov_sample64(const Gas<double>& g, const R
     double dI, ddI, dII, ddII;
     if (two_raref) {
         dI = o.sub(q.enI, q.cI);
-        ddI = fma(-g.hg1, wI, o.sub(u, q.cI));
+        ddI = fma(flip(wI), g.hg1, o.sub(u, q.cI));
     } else {
-        dI = ddI = fma(-aI, o.rcp(q.rI), q.enI);
+        dI = ddI = fma(flip(aI), o.rcp(q.rI), q.enI);
     }
     if (shockII) {
         dII = ddII = fma(aII, o.rcp(q.rII), q.enII);
     } else {
         dII = o.add(q.enII, q.cII);
-        ddII = fma(-g.hg1, wII, o.add(u, q.cII));
+        ddII = fma(flip(wII), g.hg1, o.add(u, q.cII));
     }
     const double UU = max_pos(max_abs(dI, dII), max_abs(ddI, ddII));
     // the interval that holds w = 0
     const bool left = key(u) >= key(-0.0);   // 0 <= u: the contact's side I
     const double en0 = sel(left, q.enI, q.enII), p0 = sel(left, q.pI, q.pII), r0 = sel(left, q.rI, q.rII);
     const double te = sel(left, q.teI, q.teII), c0 = sel(left, q.cI, q.cII);
-    const double d = sel(left, dI, -dII), dd = sel(left, ddI, -ddII);   // side II mirrored
+    const double d = sel(left, dI, flip(dII)), dd = sel(left, ddI, flip(ddII));   // side II mirrored
     double r, en, ps;
     if (key(d) >= key(-0.0)) {
         // outside the wave: the side's own state
         r = r0; en = en0; ps = p0;
     } else if (key(dd) > key(0.0)) {
         // inside a rarefaction fan
-        const double e = sel(left, en0, -en0);
+        const double e = sel(left, en0, flip(en0));
         const double ce = o.mul(fma(g.g1, e, o.mul(2.0, c0)), o.rcp(g.g2));
         ps = o.mul(p0, pow_inv_gm(g, o.mul(ce, o.rcp(c0))));
         const double ic = o.rcp(ce);
         r = o.mul(o.mul(o.mul(g.ga, ps), ic), ic);
-        en = sel(left, ce, -ce);
+        en = sel(left, ce, flip(ce));
     } else {
         // between the wave and the contact
-        const double a = sel(left, aI, aII), w = sel(left, wI, -wII);
+        const double a = sel(left, aI, aII), w = sel(left, wI, flip(wII));
         ps = p;
         en = u;
         if (left ? !two_raref : shockII) {
-            r = o.mul(o.mul(r0, a), o.rcp(fma(-r0, w, a)));
+            r = o.mul(o.mul(r0, a), o.rcp(fma(flip(r0), w, a)));
         } else {
             const double ic = o.rcp(fma(g.hg1, w, c0));
             r = o.mul(o.mul(o.mul(g.ga, p), ic), ic);

@@ -88,17 +88,6 @@ __device__ __forceinline__ float minmod_d(float a, float b)
     const float m = fmaxf(0.0f, fminf(fabsf(a), __uint_as_float(__float_as_uint(b) ^ sa)));
     return __uint_as_float(__float_as_uint(m) | sa);
 }
-// FP64: minimum, maximum and signs on the bit patterns (section "FP64
-// arithmetic for a narrow pipe" below)
-__device__ __forceinline__ double minmod_d(double a, double b)
-{
-    const long long ia = __double_as_longlong(a);
-    const long long sa = ia & (long long)0x8000000000000000ull;
-    const long long ma = ia & 0x7fffffffffffffffll, bs = __double_as_longlong(b) ^ sa;
-    const long long m = (ma < bs) ? ma : bs;   // negative: opposite signs
-    return __longlong_as_double(((m < 0) ? 0ll : m) | sa);
-}
-
 // ------------------------------------------------------------------ FP64 arithmetic for a narrow pipe
 // GB300 issues one FP64 warp instruction per SM every 17-20 cycles (measured:
 // fma 17, add and mul 20, a compare-and-select 20, fmin 40; each waits 92
@@ -114,11 +103,28 @@ __device__ __forceinline__ double minmod_d(double a, double b)
 // bits.
 namespace d64 {
 constexpr long long kSign = (long long)0x8000000000000000ull;
-__device__ __forceinline__ long long bits(double a) { return __double_as_longlong(a); }
-__device__ __forceinline__ double from(long long a) { return __longlong_as_double(a); }
+// the bit pattern, as a move that the compiler does not look through (it would
+// turn the integer tests below back into FP64 instructions)
+__device__ __forceinline__ long long bits(double a)
+{
+    long long i;
+    asm("mov.b64 %0, %1;" : "=l"(i) : "d"(a));
+    return i;
+}
+__device__ __forceinline__ double from(long long i)
+{
+    double a;
+    asm("mov.b64 %0, %1;" : "=d"(a) : "l"(i));
+    return a;
+}
 __device__ __forceinline__ double abs(double a) { return from(bits(a) & ~kSign); }
-__device__ __forceinline__ bool neg(double a) { return __double2hiint(a) < 0; }   // the sign bit
+__device__ __forceinline__ bool neg(double a) { return bits(a) < 0; }   // the sign bit
 __device__ __forceinline__ double sel(bool c, double a, double b) { return from(c ? bits(a) : bits(b)); }
+// -a (the compiler writes a negation in front of an fma as an FP64 sum)
+__device__ __forceinline__ double flip(double a) { return from(bits(a) ^ kSign); }
+// keeps a branch a branch (a short one's operations would be computed on both
+// sides and selected)
+__device__ __forceinline__ void branch() { asm volatile(""); }
 // an integer that orders as the numbers do (no NaN)
 __device__ __forceinline__ long long key(double a)
 {
@@ -148,15 +154,16 @@ __device__ __forceinline__ bool tame(double a) { return (__double2hiint(a) & 0x7
 // constant or the same register twice every 19-20 (measured), so the factors
 // are kept in registers, where the compiler cannot see their values (g.zero).
 struct Pipe {
-    double one, half, nz;
+    double one, mone, half, nz;
     __device__ __forceinline__ explicit Pipe(const Gas<double>& g)
     {
         one = from((long long)(0x3ff00000 + g.zero) << 32);
+        mone = from((long long)((int)0xbff00000 + g.zero) << 32);
         half = from((long long)(0x3fe00000 + g.zero) << 32);
         nz = from((long long)((int)0x80000000 + g.zero) << 32);
     }
     __device__ __forceinline__ double add(double a, double b) const { return fma(a, one, b); }
-    __device__ __forceinline__ double sub(double a, double b) const { return fma(-b, one, a); }
+    __device__ __forceinline__ double sub(double a, double b) const { return fma(b, mone, a); }
     __device__ __forceinline__ double mul(double a, double b) const { return fma(a, b, nz); }
     // 1/x of a normal number well inside the range: with y0 = (1 + d)/x and
     // e = 1 - x y0, 1/x = y0 (1 + e + e^2 + ...), cut after e^2 (|e| < 2^-19)
@@ -164,7 +171,7 @@ struct Pipe {
     {
         double y;
         asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-        const double e = fma(-x, y, one);
+        const double e = fma(x, flip(y), one);
         return fma(y, fma(e, e, e), y);
     }
     // sqrt(a / r) of tame a and r as a (a r)^(-1/2): with y0 the approximate
@@ -175,7 +182,7 @@ struct Pipe {
         const double x = mul(a, r);
         double y;
         asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-        const double e = fma(-mul(x, y), y, one);
+        const double e = fma(mul(x, y), flip(y), one);
         const double w = mul(a, y);
         return fma(w, mul(e, fma(e, 0.375, half)), w);
     }
@@ -184,12 +191,21 @@ struct Pipe {
     {
         double y;
         asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-        const double e = fma(-mul(x, y), y, one);
+        const double e = fma(mul(x, y), flip(y), one);
         return fma(y, mul(e, fma(e, 0.375, half)), y);
     }
 };
 
 }  // namespace d64
+
+// minmod (above) on the bit patterns
+__device__ __forceinline__ double minmod_d(double a, double b)
+{
+    const long long ia = d64::bits(a), sa = ia & d64::kSign;
+    const long long ma = ia & ~d64::kSign, bs = d64::bits(b) ^ sa;
+    const long long m = (ma < bs) ? ma : bs;   // negative: opposite signs
+    return d64::from(((m < 0) ? 0ll : m) | sa);
+}
 
 // left / right face values of a cell from its three-point stencil; the
 // reference's linear2 with the coordinate differences folded in
@@ -205,7 +221,7 @@ __device__ __forceinline__ void recon_pair(const Gas<double>& g, double tm, doub
 {
     const d64::Pipe o(g);
     const double m = minmod_d(o.sub(t0, tm), o.sub(tp, t0));
-    left = fma(-m, o.half, t0);
+    left = fma(d64::flip(m), o.half, t0);
     right = fma(m, o.half, t0);
 }
 
@@ -250,6 +266,9 @@ __device__ __forceinline__ R flux_hll(const Gas<R>& g, R rL, R pL, R unL, R utL,
 {
     return flux_hll_ref(g, rL, pL, unL, utL, rR, pR, unR, utR, F);
 }
+
+// out of line: inlined, a division's FP64 operations run whether wanted or not
+static __device__ __noinline__ double rcp_wild(double a) { return 1.0 / a; }
 
 // a face's flux and wave speed from an out-of-line call (by value, so that
 // the caller's flux stays in registers on its own path)
@@ -302,7 +321,7 @@ __device__ __forceinline__ double flux_hll_of(const Gas<double>& g, double c, do
     const double DL = o.sub(min(unL, unR), c), DR = o.add(max(unL, unR), c);
     const double SL = sel(neg(DL), DL, 0.0), SR = sel(neg(DR), 0.0, DR);
     const double inv = o.rcp(o.sub(SR, SL));
-    const double a = sel(neg(DL), o.mul(SR, inv), 1.0), b = sel(neg(DR), 1.0, o.mul(-SL, inv));
+    const double a = sel(neg(DL), o.mul(SR, inv), 1.0), b = sel(neg(DR), 1.0, o.mul(flip(SL), inv));
     const double A = o.mul(a, o.sub(unL, SL)), B = o.mul(b, o.sub(unR, SR));
     const double mL = o.mul(A, rL), mR = o.mul(B, rR);
     const double PL = o.mul(a, pL), PR = o.mul(b, pR);
@@ -548,7 +567,7 @@ __device__ __forceinline__ double flux_star(const Gas<double>& g, double SL, dou
     const Pipe o(g);
     const double wL = o.sub(SL, u1), wR = o.sub(SR, u2);
     const double aL = o.mul(rL, wL), aR = o.mul(rR, wR);     // aL < 0 < aR
-    const double num = fma(aR, u2, fma(-aL, u1, o.sub(pL, pR)));
+    const double num = fma(aR, u2, fma(flip(aL), u1, o.sub(pL, pR)));
     const double SM = o.mul(num, o.rcp(o.sub(aR, aL)));
     const double psL = fma(aL, o.sub(SM, u1), pL);
     const double ptz = MEAN ? o.mul(o.half, o.add(fma(aR, o.sub(SM, u2), pR), psL)) : psL;
@@ -560,7 +579,7 @@ __device__ __forceinline__ double flux_star(const Gas<double>& g, double SL, dou
     const double inv = o.rcp(o.sub(S, SM));
     const double q = fma(u, u, o.mul(v, v));
     const double e = fma(p, g.inv_g1, o.mul(o.mul(o.half, r), q));
-    const double es = o.mul(fma(e, w, fma(ptz, SM, -o.mul(p, u))), inv);
+    const double es = o.mul(fma(e, w, fma(ptz, SM, flip(o.mul(p, u)))), inv);
     const double um = sel(sup, u, SM), pm = sel(sup, p, ptz);
     F[0] = o.mul(sel(sup, r, o.mul(a, inv)), um);
     F[1] = fma(F[0], um, pm);

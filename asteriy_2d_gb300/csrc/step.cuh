@@ -397,12 +397,20 @@ __device__ __forceinline__ S& tile_smem()
 }
 
 // ------------------------------------------------------------------ sign and NaN tests
-// a <= 0, and whether a is a NaN, for values that seldom are: FP64 on the bit
-// pattern (an FP64 comparison only where the pattern says it may be so)
+// a <= 0, and whether a is a NaN (FP64: on the bit pattern; an FP64
+// comparison holds the FP64 pipe as long as a sum)
 __device__ __forceinline__ bool le_zero(float a) { return a <= 0.0f; }
-__device__ __forceinline__ bool le_zero(double a) { return __double_as_longlong(a) <= 0 && a <= 0.0; }
+__device__ __forceinline__ bool le_zero(double a)
+{
+    const long long i = d64::bits(a);   // +0, or the sign bit and not a NaN
+    return i <= 0 && (unsigned long long)i <= 0xfff0000000000000ull;
+}
 __device__ __forceinline__ bool is_nan(float a) { return !(a == a); }
-__device__ __forceinline__ bool is_nan(double a) { return !d64::finite(a) && !(a == a); }
+__device__ __forceinline__ bool is_nan(double a)
+{
+    return (d64::bits(a) & ~d64::kSign) > 0x7ff0000000000000ll;
+}
+
 // ------------------------------------------------------------------ cell update
 // Conservative update of one cell in FP32 from its state `in`
 // (rho, p, vz, vr) and its four face fluxes f[k][face] (k = mass, mom_z,
@@ -452,13 +460,13 @@ __device__ __forceinline__ void update_cell(const StepParams& P, float ga, float
 }
 
 // The same update in FP64, in 38 operations (the expressions above compile
-// to about 65): tz = T_do/dx and tr = T_do/dy multiply the flux differences
+// to about 65): ntz = -T_do/dx and ntr = -T_do/dy multiply the flux differences
 // themselves, the momenta serve the energies (rho v^2 = (rho v) v), and the
 // signs are read off the bit patterns.  `body`, `source`: whether Q2, and
 // Sz and Sr, are to be added.
 template <typename R>
 __device__ __forceinline__ void update_cell64(const Gas<double>& g, double p_floor, bool axisym, const R in[4],
-                                              const R f[4][4], double T_do, double tz, double tr, double ty,
+                                              const R f[4][4], double T_do, double ntz, double ntr, double ty,
                                               bool body, double Q2, bool source, double Sz, double Sr, int& nrho,
                                               int& np, unsigned& status, R out[4])
 {
@@ -471,28 +479,31 @@ __device__ __forceinline__ void update_cell64(const Gas<double>& g, double p_flo
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         const double fz = o.sub((double)f[k][0], (double)f[k][1]), fr = o.sub((double)f[k][3], (double)f[k][2]);
-        U[k] = fma(-tr, fr, fma(-tz, fz, U[k]));
+        U[k] = fma(ntr, fr, fma(ntz, fz, U[k]));
     }
     if (axisym) {
-        const double w = o.mul(ty, mr1);
-        U[0] = o.sub(U[0], w);
-        U[1] = fma(-w, vz1, U[1]);
-        U[2] = fma(-w, vr1, U[2]);
-        U[3] = fma(-o.mul(ty, vr1), o.add(E1, p1), U[3]);
+        branch();
+        const double w = flip(o.mul(ty, mr1));
+        U[0] = o.add(w, U[0]);
+        U[1] = fma(w, vz1, U[1]);
+        U[2] = fma(w, vr1, U[2]);
+        U[3] = fma(flip(o.mul(ty, vr1)), o.add(E1, p1), U[3]);
     }
     if (body) {
+        branch();
         U[2] = fma(T_do, Q2, U[2]);
         U[3] = fma(T_do, o.mul(Q2, vr1), U[3]);
     }
     if (source) {
+        branch();
         U[1] = o.add(U[1], Sz);
         U[2] = o.add(U[2], Sr);
     }
     double rho2 = U[0];
     if (le_zero(rho2)) { nrho++; rho2 = r1; }
-    const double irho = tame_pos(rho2) ? o.rcp(rho2) : 1.0 / rho2;
+    const double irho = tame_pos(rho2) ? o.rcp(rho2) : rcp_wild(rho2);
     const double vz2 = o.mul(U[1], irho), vr2 = o.mul(U[2], irho);
-    double p2 = o.mul(fma(-o.half, fma(U[1], vz2, o.mul(U[2], vr2)), U[3]), g.g1);
+    double p2 = o.mul(fma(flip(fma(U[1], vz2, o.mul(U[2], vr2))), o.half, U[3]), g.g1);
     if (le_zero(p2)) { np++; p2 = p_floor; }
     if (is_nan(p2)) status |= 0x10u;
     out[0] = (R)rho2; out[1] = (R)p2; out[2] = (R)vz2; out[3] = (R)vr2;
@@ -1249,24 +1260,28 @@ struct TileAcc {
 // constants of the step every tile shares (set by thread 0, read after a barrier)
 struct StepConsts {
     double T_do;           // the step's dt
-    double tz, tr;         // T_do / dx, T_do / dy
+    double ntz, ntr;       // -T_do / dx, -T_do / dy
     float tdv_f, T_f;      // T_do / (dx dy), T_do
     int step;
 };
 
+template <typename R>
 __device__ __forceinline__ void step_consts_of(const StepParams& P, double T_do, int step, StepConsts& K)
 {
     K.T_do = T_do;
     K.step = step;
-    K.tz = K.T_do / P.dx;
-    K.tr = K.T_do / P.dy;
-    K.tdv_f = (float)(K.T_do / (P.dx * P.dy));
-    K.T_f = (float)K.T_do;
+    K.ntz = -K.T_do / P.dx;
+    K.ntr = -K.T_do / P.dy;
+    if constexpr (sizeof(R) == 4) {
+        K.tdv_f = (float)(K.T_do / (P.dx * P.dy));
+        K.T_f = (float)K.T_do;
+    }
 }
 
+template <typename R>
 __device__ __forceinline__ void step_consts(const StepParams& P, StepConsts& K)
 {
-    step_consts_of(P, (P.clock != nullptr) ? *(volatile double*)&P.clock->T_do : *P.T_do_ptr,
+    step_consts_of<R>(P, (P.clock != nullptr) ? *(volatile double*)&P.clock->T_do : *P.T_do_ptr,
                    (P.clock != nullptr) ? (int)P.clock->step : 0, K);
 }
 
@@ -1534,7 +1549,7 @@ __device__ __forceinline__ void tile_body(const StepParams& P, S& sm, int b, con
             Sr = w * ar;
         }
         const double ty = (sizeof(R) == 8) ? sm.tydrow[row] : ((P.geom == 1) ? T_do / sm.ydrow[row] : 0.0);
-        update_cell64(P.gd, P.p_floor, P.geom == 1, in, f, T_do, K.tz, K.tr, ty, body, Q2,
+        update_cell64(P.gd, P.p_floor, P.geom == 1, in, f, T_do, K.ntz, K.ntr, ty, body, Q2,
                       sizeof(R) == 8 && P.nsrc != nullptr, Sz, Sr, acc.nrho, acc.np, acc.rc.status, o);
     };
     // the FP32 form's source terms of a cell: ty = T_do/r and the body force
@@ -1738,7 +1753,7 @@ __device__ __forceinline__ void step_tile(const StepParams& P, int bx, int by, u
     const Gas<R>& g = *reinterpret_cast<const Gas<R>*>(sizeof(R) == 8 ? (const void*)&P.gd : (const void*)&P.gf);
     if (threadIdx.x == 0) {
         sm.qn = 0u;
-        step_consts(P, sK);
+        step_consts<R>(P, sK);
     }
     stage_tile<R, LAYOUT, TZ, TR>(P, sm, 0, n0, m0);
     __syncthreads();
@@ -1871,7 +1886,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == 4 ? 4 : 2)
         tma::mbar_init(&bar[0], 1);
         tma::mbar_init(&bar[1], 1);
         tma::fence_async_shared();
-        step_consts(P, sK);
+        step_consts<R>(P, sK);
         s_pend = make_int2(-1, -1);
         sm.qn = 0u;   // later tiles: reset after the previous tile's queue
         // the first two tiles: the first is copied now, the second at the
@@ -2173,7 +2188,7 @@ __global__ void __launch_bounds__(kThreads, 4)
                 claim = (int)atomicAdd(counter, 1u);
             }
             // this tile's step constants (read after the face pass's barrier)
-            step_consts_of(P, s_tdo[b], (int)s_step[b], sK[b]);
+            step_consts_of<R>(P, s_tdo[b], (int)s_step[b], sK[b]);
         }
         if constexpr (MIXED) {
             switch (w.x >> 24) {

@@ -415,7 +415,7 @@ __device__ __forceinline__ void sweep_strip(const StepParams& P, const StepConst
                         if (x > P.body_lo && x < P.body_hi)
                             Q2 = (y >= P.body_rsplit) ? -P.body_amp * (double)w0[0] : P.body_amp * (double)w0[0];
                     }
-                    update_cell64(P.gd, P.p_floor, true, w0, f, T_do, K.tz, K.tr, T_do / y, P.body_force != 0, Q2,
+                    update_cell64(P.gd, P.p_floor, true, w0, f, T_do, K.ntz, K.ntr, T_do / y, P.body_force != 0, Q2,
                                   false, 0.0, 0.0, acc.nrho, acc.np, acc.rc.status, o);
                 } else {
                     const float y = P.y_minf + (float)m * P.dyf;
@@ -471,7 +471,7 @@ __global__ void __launch_bounds__(kThreads, 2) sweep_kernel(StepParams P)
         if (P.guess == 1 && P.mlp != nullptr) sweep_stage_net(P.mlp, snet);
         net = &snet;
     }
-    if (threadIdx.x == 0) step_consts(P, sK);
+    if (threadIdx.x == 0) step_consts<float>(P, sK);
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const int r_lo = P.band_lo * 16;
