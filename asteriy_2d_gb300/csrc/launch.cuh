@@ -106,15 +106,12 @@ template <typename R, int FLUX, bool RECON>
 int launch_tma_t(const StepParams& P, const CUtensorMap& tin, const CUtensorMap& tout, int grid, cudaStream_t st,
                  bool launch, int* per_sm)
 {
-    // two variants: with the uniform-tile test (skip_uniform) and without it
-    auto k = P.skip_uniform ? step_kernel_tma<R, FLUX, RECON, true> : step_kernel_tma<R, FLUX, RECON, false>;
+    auto k = step_kernel_tma<R, FLUX, RECON>;
     constexpr size_t smem = tile_smem_bytes<R, FLUX, kTmaTZ, kTmaTR, 2>();
     cudaError_t e;
     if (!launch) {
-        for (auto kv : {step_kernel_tma<R, FLUX, RECON, true>, step_kernel_tma<R, FLUX, RECON, false>}) {
-            e = cudaFuncSetAttribute(kv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute");
-        }
+        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute");
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k, kThreads, smem);
         return e == cudaSuccess ? AST_OK : cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
     }
@@ -356,7 +353,6 @@ inline void fill_step_params(StepParams& P, const ast_config& c)
         P.fixed_mhi = clampi(std::ceil((c.fixed_ar - P.y_min) / P.dy) + 1.0);
     }
     P.region_select = c.region_select;
-    P.skip_uniform = c.skip_uniform;
     {
         // columns whose face positions pass the reference's region test
         // lo < x < hi (x = x_min + n dx, plus dx/2 for the z face above the

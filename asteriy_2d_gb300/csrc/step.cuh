@@ -112,7 +112,6 @@ struct __align__(16) StepParams {
     double fixed_zc, fixed_az2, fixed_ar2;
     int fixed_nlo, fixed_nhi, fixed_mhi;   // cells that can lie in the region (one cell of margin)
     int region_select;
-    int skip_uniform;              // uniform tiles skip the face pass
     // one step launched in bands of tile rows: this launch steps tile rows
     // [band_lo, band_hi) (band_hi 0: all rows of the grid), and `units` CTAs
     // of all the step's launches report to the clock (0: this launch's grid)
@@ -319,7 +318,7 @@ struct TileCore {
     // in the same order
     alignas(16) R Fz[TR][TZ + 1][4];
     alignas(16) R Fr[TR + 1][TZ][4];
-    unsigned char fx[HR][HZ];    // 1 = cell held fixed (fixed_region only)
+    unsigned char fx[HR][HZ];    // 1 = cell held fixed (tiles near the fixed region only)
     unsigned qn;                 // queued faces: above the gate (low 16 bits), others (high 16 bits)
     double ydrow[TR];            // r of the tile's cell rows, y_min + m dy, in FP64
     float yfrow[TR];             // and in FP32
@@ -397,6 +396,16 @@ __device__ __forceinline__ S& tile_smem()
 }
 
 // ------------------------------------------------------------------ sign and NaN tests
+// bitwise equality of two staged values
+__device__ __forceinline__ bool same_bits(float a, float b) { return __float_as_uint(a) == __float_as_uint(b); }
+// a > 0 or a positive NaN, on the bit pattern
+__device__ __forceinline__ bool positive_bits(float a) { return __float_as_int(a) > 0; }
+__device__ __forceinline__ bool positive_bits(double a) { return __double_as_longlong(a) > 0; }
+__device__ __forceinline__ bool same_bits(double a, double b)
+{
+    return __double_as_longlong(a) == __double_as_longlong(b);
+}
+
 // a <= 0, and whether a is a NaN (FP64: on the bit pattern; an FP64
 // comparison holds the FP64 pipe as long as a sum)
 __device__ __forceinline__ bool le_zero(float a) { return a <= 0.0f; }
@@ -404,6 +413,14 @@ __device__ __forceinline__ bool le_zero(double a)
 {
     const long long i = d64::bits(a);   // +0, or the sign bit and not a NaN
     return i <= 0 && (unsigned long long)i <= 0xfff0000000000000ull;
+}
+__device__ __forceinline__ bool any_le_zero(float a, float b, float c, float d)
+{
+    return fminf(fminf(a, b), fminf(c, d)) <= 0.0f;   // (fminf leaves a NaN out)
+}
+__device__ __forceinline__ bool any_le_zero(double a, double b, double c, double d)
+{
+    return le_zero(a) || le_zero(b) || le_zero(c) || le_zero(d);
 }
 __device__ __forceinline__ bool is_nan(float a) { return !(a == a); }
 __device__ __forceinline__ bool is_nan(double a)
@@ -647,16 +664,6 @@ __device__ __forceinline__ void record_face(const StepParams& P, const Gas<R>& g
 }
 
 // ------------------------------------------------------------------ face passes
-// bitwise equality of two staged values
-__device__ __forceinline__ bool same_bits(float a, float b) { return __float_as_uint(a) == __float_as_uint(b); }
-// a > 0 or a positive NaN, on the bit pattern
-__device__ __forceinline__ bool positive_bits(float a) { return __float_as_int(a) > 0; }
-__device__ __forceinline__ bool positive_bits(double a) { return __double_as_longlong(a) > 0; }
-__device__ __forceinline__ bool same_bits(double a, double b)
-{
-    return __double_as_longlong(a) == __double_as_longlong(b);
-}
-
 // The reconstructed states on both sides of face (a, c) of orientation ZF
 // (minmod on the staged cells when RECON and the face is in the
 // high-order region `hi`; the cell values otherwise).  When the four
@@ -695,7 +702,7 @@ __device__ __forceinline__ bool face_states(const StepParams& P, const S& sm, in
             tuu[k] = q[k][ju + DJ][iu + DI];
             flat = flat && same_bits(tll[k], tl[k]) && same_bits(tl[k], tu[k]) && same_bits(tu[k], tuu[k]);
         }
-        if (VOTE && __all_sync(__activemask(), flat)) {
+        if (VOTE && sizeof(R) == 8 && __all_sync(__activemask(), flat)) {
 #pragma unroll
             for (int k = 0; k < 4; k++) L[k] = tl[k] + R(0);
             // (the positivity rule below leaves equal sides equal)
@@ -713,10 +720,12 @@ __device__ __forceinline__ bool face_states(const StepParams& P, const S& sm, in
             }
         }
         // positivity of the reconstructed rho and p (kernel.cu:2706-2743)
-        if (le_zero(L[0])) L[0] = tl[0];
-        if (le_zero(U[0])) U[0] = tu[0];
-        if (le_zero(L[1]) || !P.grad_p) L[1] = tl[1];
-        if (le_zero(U[1]) || !P.grad_p) U[1] = tu[1];
+        if (!P.grad_p || any_le_zero(L[0], U[0], L[1], U[1])) {
+            if (le_zero(L[0])) L[0] = q[0][jl][il];
+            if (le_zero(U[0])) U[0] = q[0][ju][iu];
+            if (le_zero(L[1]) || !P.grad_p) L[1] = q[1][jl][il];
+            if (le_zero(U[1]) || !P.grad_p) U[1] = q[1][ju][iu];
+        }
     }
     return false;
 }
@@ -754,8 +763,8 @@ __device__ __forceinline__ bool same_state(const double L[4], const double U[4])
 // (hi).  ZF: z faces (between tile columns c-1 and c of row a), else r
 // faces (between tile rows a-1 and a of column c).
 template <int TZ, int TR, bool ZF, typename S>
-__device__ __forceinline__ void face_meta(const StepParams& P, const S& sm, int n0, int m0, bool interior, int a,
-                                          int c, bool& active, bool& hi)
+__device__ __forceinline__ void face_meta(const StepParams& P, const S& sm, int n0, int m0, bool interior, bool near,
+                                          int a, int c, bool& active, bool& hi)
 {
     // smem indices of the lower (l) and upper (u) cell of the face
     const int jl = ZF ? a + 2 : a + 1, il = ZF ? c + 1 : c + 2;
@@ -768,7 +777,7 @@ __device__ __forceinline__ void face_meta(const StepParams& P, const S& sm, int 
         uval = nu >= 0 && nu < P.N && mu >= 0 && mu < P.M;
     }
     active = lval || uval;
-    if (active && P.fixed_region) active = (lval && !sm.fx[jl][il]) || (uval && !sm.fx[ju][iu]);
+    if (active && near) active = (lval && !sm.fx[jl][il]) || (uval && !sm.fx[ju][iu]);
     hi = true;
     if (P.region_select) {
         // the face's z position as the reference's lower cell sees it, as an
@@ -882,16 +891,17 @@ __device__ __forceinline__ void face_flux(const StepParams& P, S& sm, const Gas<
 // once, so the cell between the two faces is reconstructed once for both
 // (minmod, linear2 and the positivity rule as face_states applies them, the
 // same values).  Z faces take c even and load the cells as aligned pairs.
-template <typename R, int FLUX, bool RECON, int TZ, int TR, bool ZF, bool FF = false, typename S>
+template <typename R, int FLUX, bool RECON, int TZ, int TR, bool ZF, typename S>
 __device__ __forceinline__ void face_two(const StepParams& P, S& sm, int b, const Gas<R>& g, int n0, int m0,
-                                         bool interior, RiemannCount& rc, R& smax, int a, int c, bool two)
+                                         bool interior, bool near, RiemannCount& rc, R& smax, int a, int c,
+                                         bool two)
 {
     constexpr int QX = S::QX, HR = S::HR;
     using R2 = std::conditional_t<sizeof(R) == 4, float2, double2>;
     const int a1 = ZF ? a : a + 1, c1 = ZF ? c + 1 : c;
     bool act0, hi0, act1 = false, hi1 = true;
-    face_meta<TZ, TR, ZF>(P, sm, n0, m0, interior, a, c, act0, hi0);
-    if (two) face_meta<TZ, TR, ZF>(P, sm, n0, m0, interior, a1, c1, act1, hi1);
+    face_meta<TZ, TR, ZF>(P, sm, n0, m0, interior, near, a, c, act0, hi0);
+    if (two) face_meta<TZ, TR, ZF>(P, sm, n0, m0, interior, near, a1, c1, act1, hi1);
     R L0[4], U0[4], L1[4], U1[4];
     const auto& q = sm.qb[b];
     // the five staged cells of variable k along the normal
@@ -918,55 +928,13 @@ __device__ __forceinline__ void face_two(const StepParams& P, S& sm, int b, cons
         else put4(sm.Fr[fa][fc], f0, f2, f1, f3);
         if (act) smax = larger_speed(smax, sp);
     };
-    // FF (kernels with the skip_uniform code, when it is set): HLL in FP32,
-    // a face pair in the high-order region.  When the five staged cells of
-    // every variable hold one bit pattern (rho, p > 0, velocities not -0) in
-    // every active lane of the warp (undisturbed gas), every limited slope is
-    // +0 and all four face values are the middle cell's value plus +0, so
-    // both faces take that state's physical flux (as below, where the four
-    // sides are found equal after the reconstruction: the same bits), with no
-    // reconstruction.  The density is voted on first, the other variables
-    // only when it is flat in the whole warp.  Measured at 4096x2048: the
-    // blast at step 1000 0.1414 -> 0.1229 ms per step, but the wind problem
-    // with HLL (its seeded noise disturbs every face) 0.0555 -> 0.0599 ms, so
-    // it goes with the opt-in skip_uniform and not into the default kernel.
-    constexpr bool kFlatFirst = FF && FLUX == 0 && sizeof(R) == 4 && RECON;
-    R rho5[5];
-    const bool ff = kFlatFirst && P.skip_uniform;
-    if (kFlatFirst && ff) {
-        constexpr int NN = ZF ? 2 : 3, TT = ZF ? 3 : 2;
-        load5(0, rho5);
-        bool flat = two && hi0 && hi1 && same_bits(rho5[0], rho5[1]) && same_bits(rho5[1], rho5[2]) &&
-                    same_bits(rho5[2], rho5[3]) && same_bits(rho5[3], rho5[4]) && positive_bits(rho5[2]);
-        if (__all_sync(__activemask(), flat)) {
-            R st[4];
-            st[0] = rho5[2];
-#pragma unroll
-            for (int k = 1; k < 4; k++) {
-                R v[5];
-                load5(k, v);
-                flat = flat && same_bits(v[0], v[1]) && same_bits(v[1], v[2]) && same_bits(v[2], v[3]) &&
-                       same_bits(v[3], v[4]);
-                st[k] = v[2];
-            }
-            flat = flat && positive_bits(st[1]) && __float_as_uint(st[2]) != 0x80000000u &&
-                   __float_as_uint(st[3]) != 0x80000000u;
-            if (__all_sync(__activemask(), flat)) {
-                R f[4];
-                const R sp = flux_physical(g, st[0], st[1], st[NN], st[TT], f);
-                store(a, c, act0, f[0], f[1], f[2], f[3], sp);
-                store(a1, c1, act1, f[0], f[1], f[2], f[3], sp);
-                return;
-            }
-        }
-    }
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         R v[5];
         load5(k, v);
         L0[k] = v[1]; U0[k] = v[2]; L1[k] = v[2]; U1[k] = v[3];
         // (FP64: first-order faces leave the slopes out; every face is in the
-        // high-order region unless region_select is on)
+        // high-order region unless region_select is on.  FP32: put right below)
         if (RECON && (sizeof(R) == 4 || hi0 || hi1)) {
             R x0, x1, y0, y1, z0, z1;
             // FP64: five cells of one bit pattern in every active lane of
@@ -989,44 +957,46 @@ __device__ __forceinline__ void face_two(const StepParams& P, S& sm, int b, cons
                 recon_pair(g, v[1], v[2], v[3], y0, y1);   // the cell between the faces
                 recon_pair(g, v[2], v[3], v[4], z0, z1);   // upper cell of the second face
             }
-            if (hi0) { L0[k] = x1; U0[k] = y0; }
-            if (hi1) { L1[k] = y1; U1[k] = z0; }
-            // positivity of the reconstructed rho and p (kernel.cu:2706-2743)
-            if (k == 0) {
-                if (le_zero(L0[0])) L0[0] = v[1];
-                if (le_zero(U0[0])) U0[0] = v[2];
-                if (le_zero(L1[0])) L1[0] = v[2];
-                if (le_zero(U1[0])) U1[0] = v[3];
-            } else if (k == 1) {
-                if (le_zero(L0[1]) || !P.grad_p) L0[1] = v[1];
-                if (le_zero(U0[1]) || !P.grad_p) U0[1] = v[2];
-                if (le_zero(L1[1]) || !P.grad_p) L1[1] = v[2];
-                if (le_zero(U1[1]) || !P.grad_p) U1[1] = v[3];
+            if (sizeof(R) == 4) {
+                L0[k] = x1; U0[k] = y0;
+                L1[k] = y1; U1[k] = z0;
+            } else {
+                if (hi0) { L0[k] = x1; U0[k] = y0; }
+                if (hi1) { L1[k] = y1; U1[k] = z0; }
+                // positivity of the reconstructed rho and p (kernel.cu:2706-2743)
+                const bool off = k == 1 && !P.grad_p;
+                if (off || (k < 2 && le_zero(L0[k]))) L0[k] = v[1];
+                if (off || (k < 2 && le_zero(U0[k]))) U0[k] = v[2];
+                if (off || (k < 2 && le_zero(L1[k]))) L1[k] = v[2];
+                if (off || (k < 2 && le_zero(U1[k]))) U1[k] = v[3];
+            }
+        }
+    }
+    // FP32, seldom: the same positivity rule, and the faces outside the
+    // high-order region, from the staged cells (tests and selects of every
+    // value took 16 of the pair's ALU instructions)
+    if (RECON && sizeof(R) == 4) {
+        const bool low = !P.grad_p || (P.region_select && !(hi0 && hi1)) ||
+                         any_le_zero(L0[0], U0[0], L1[0], U1[0]) || any_le_zero(L0[1], U0[1], L1[1], U1[1]);
+        if (low) {
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                R v[5];
+                load5(k, v);
+                const bool off = k == 1 && !P.grad_p;
+                if (!hi0 || off || (k < 2 && le_zero(L0[k]))) L0[k] = v[1];
+                if (!hi0 || off || (k < 2 && le_zero(U0[k]))) U0[k] = v[2];
+                if (!hi1 || off || (k < 2 && le_zero(L1[k]))) L1[k] = v[2];
+                if (!hi1 || off || (k < 2 && le_zero(U1[k]))) U1[k] = v[3];
             }
         }
     }
     if constexpr (FLUX == 0 && sizeof(R) == 4) {
-        // HLL in FP32: both faces in packed arithmetic; or, when both faces
-        // of every active lane of the warp hold one state on all four sides
-        // (one bit pattern, rho > 0, p > 0: undisturbed gas), that state's
-        // physical flux once for both (flux_physical: what the HLL formula
-        // gives up to rounding, its wave speed formed as the formula forms it)
+        // HLL in FP32: both faces in packed arithmetic
         constexpr int NN = ZF ? 2 : 3, TT = ZF ? 3 : 2;
         float2 F[4], Sp;
-        bool one = two && positive_bits(L0[0]) && positive_bits(L0[1]);
-#pragma unroll
-        for (int k = 0; k < 4; k++)
-            one = one && same_bits(L0[k], U0[k]) && same_bits(L0[k], L1[k]) && same_bits(L0[k], U1[k]);
-        if (__all_sync(__activemask(), one)) {
-            float f[4];
-            const float s = flux_physical(g, L0[0], L0[1], L0[NN], L0[TT], f);
-#pragma unroll
-            for (int k = 0; k < 4; k++) F[k] = pk(f[k], f[k]);
-            Sp = pk(s, s);
-        } else {
-            flux_hll_x2(g, pk(L0[0], L1[0]), pk(L0[1], L1[1]), pk(L0[NN], L1[NN]), pk(L0[TT], L1[TT]),
-                        pk(U0[0], U1[0]), pk(U0[1], U1[1]), pk(U0[NN], U1[NN]), pk(U0[TT], U1[TT]), F, Sp);
-        }
+        flux_hll_x2(g, pk(L0[0], L1[0]), pk(L0[1], L1[1]), pk(L0[NN], L1[NN]), pk(L0[TT], L1[TT]), pk(U0[0], U1[0]),
+                    pk(U0[1], U1[1]), pk(U0[NN], U1[NN]), pk(U0[TT], U1[TT]), F, Sp);
         store(a, c, act0, F[0].x, F[1].x, F[2].x, F[3].x, Sp.x);
         if (two) store(a1, c1, act1, F[0].y, F[1].y, F[2].y, F[3].y, Sp.y);
     } else {
@@ -1049,10 +1019,10 @@ __device__ __forceinline__ void face_two(const StepParams& P, S& sm, int b, cons
 // form's extra code costs more in instruction fetch than it saves).
 template <typename R, int FLUX, bool RECON, int TZ, int TR, bool ZF, typename S>
 __device__ __forceinline__ void face_one(const StepParams& P, S& sm, int b, const Gas<R>& g, int n0, int m0,
-                                         bool interior, RiemannCount& rc, R& smax, int a, int c)
+                                         bool interior, bool near, RiemannCount& rc, R& smax, int a, int c)
 {
     bool active, hi;
-    face_meta<TZ, TR, ZF>(P, sm, n0, m0, interior, a, c, active, hi);
+    face_meta<TZ, TR, ZF>(P, sm, n0, m0, interior, near, a, c, active, hi);
     R L[4], U[4];
     const bool same = face_states<R, RECON, ZF>(P, sm, b, a, c, hi, L, U);
     face_flux<R, FLUX, TZ, TR, ZF>(P, sm, g, a, c, active, hi, L, U, rc, smax, same);
@@ -1068,9 +1038,9 @@ __device__ __forceinline__ void face_one(const StepParams& P, S& sm, int b, cons
 // per row when TZ = 32, so the warp's staged-cell loads hit distinct
 // banks), then the last z face (c = TZ) of every row, then the r faces; each
 // group padded to whole warps so that no warp mixes groups.
-template <typename R, int FLUX, bool RECON, int TZ, int TR, bool FF = false, typename S>
+template <typename R, int FLUX, bool RECON, int TZ, int TR, typename S>
 __device__ __forceinline__ void face_pass(const StepParams& P, S& sm, int b, const Gas<R>& g, int n0, int m0,
-                                          int step, RiemannCount& rc, int& fallback, R& smz, R& smr)
+                                          bool near, int step, RiemannCount& rc, int& fallback, R& smz, R& smr)
 {
     // every cell the tile's faces touch lies inside the grid
     const bool interior = n0 >= 1 && n0 + TZ < P.N && m0 >= 1 && m0 + TR < P.M;
@@ -1083,16 +1053,16 @@ __device__ __forceinline__ void face_pass(const StepParams& P, S& sm, int b, con
         for (int t = threadIdx.x; t < NP + TZP + TR; t += kThreads) {
             if (t < NZP) {
                 const int a = t / (TZ / 2);
-                face_two<R, FLUX, RECON, TZ, TR, true, FF>(P, sm, b, g, n0, m0, interior, rc, smz, a,
+                face_two<R, FLUX, RECON, TZ, TR, true>(P, sm, b, g, n0, m0, interior, near, rc, smz, a,
                                                        2 * (t - a * (TZ / 2)), true);
             } else if (t < NP) {
                 const int u = t - NZP, a = u / TZ;
-                face_two<R, FLUX, RECON, TZ, TR, false, FF>(P, sm, b, g, n0, m0, interior, rc, smr, 2 * a, u - a * TZ,
+                face_two<R, FLUX, RECON, TZ, TR, false>(P, sm, b, g, n0, m0, interior, near, rc, smr, 2 * a, u - a * TZ,
                                                         true);
             } else if (t < NP + TZ) {
-                face_two<R, FLUX, RECON, TZ, TR, false, FF>(P, sm, b, g, n0, m0, interior, rc, smr, TR, t - NP, false);
+                face_two<R, FLUX, RECON, TZ, TR, false>(P, sm, b, g, n0, m0, interior, near, rc, smr, TR, t - NP, false);
             } else if (t >= NP + TZP) {
-                face_two<R, FLUX, RECON, TZ, TR, true, FF>(P, sm, b, g, n0, m0, interior, rc, smz, t - NP - TZP, TZ,
+                face_two<R, FLUX, RECON, TZ, TR, true>(P, sm, b, g, n0, m0, interior, near, rc, smz, t - NP - TZP, TZ,
                                                        false);
             }
         }
@@ -1114,10 +1084,10 @@ __device__ __forceinline__ void face_pass(const StepParams& P, S& sm, int b, con
                 } else {
                     continue;
                 }
-                face_one<R, FLUX, RECON, TZ, TR, true>(P, sm, b, g, n0, m0, interior, rc, smz, a, c);
+                face_one<R, FLUX, RECON, TZ, TR, true>(P, sm, b, g, n0, m0, interior, near, rc, smz, a, c);
             } else {
                 const int a = (t - NZLP) / TZ;
-                face_one<R, FLUX, RECON, TZ, TR, false>(P, sm, b, g, n0, m0, interior, rc, smr, a,
+                face_one<R, FLUX, RECON, TZ, TR, false>(P, sm, b, g, n0, m0, interior, near, rc, smr, a,
                                                         t - NZLP - a * TZ);
             }
         }
@@ -1295,12 +1265,16 @@ __device__ __forceinline__ bool tile_near_fixed(const StepParams& P, int n0, int
 }
 
 // stage tile + halo from global memory into buffer b, ghost rules applied;
-// the corners are never read by the cross stencil
+// the corners are never read by the cross stencil.  Returns whether a density
+// that this thread staged differs from the tile's first cell's.
 template <typename R, int LAYOUT, int TZ, int TR, typename S>
-__device__ __forceinline__ void stage_tile(const StepParams& P, S& sm, int b, int n0, int m0)
+__device__ __forceinline__ bool stage_tile(const StepParams& P, S& sm, int b, int n0, int m0)
 {
     constexpr int HZ = S::HZ, HR = S::HR, QX = S::QX;
     const bool near_fixed = tile_near_fixed<TZ, TR>(P, n0, m0);
+    R first[4];
+    read_cell<R, LAYOUT>(P, n0, m0, first);
+    bool differs = false;
     for (int idx = threadIdx.x; idx < HR * HZ; idx += kThreads) {
         const int j = idx / HZ, i = idx - j * HZ;
         const bool rin = (j >= 2 && j < TR + 2), cin = (i >= 2 && i < TZ + 2);
@@ -1308,14 +1282,16 @@ __device__ __forceinline__ void stage_tile(const StepParams& P, S& sm, int b, in
         const int n = n0 - 2 + i, m = m0 - 2 + j;
         R v[4];
         fetch_cell<R, LAYOUT>(P, n, m, v);
+        differs = differs || !same_bits(v[0], first[0]);
         sm.qb[b][0][j][i + QX] = v[0]; sm.qb[b][1][j][i + QX] = v[1];
         sm.qb[b][2][j][i + QX] = v[2]; sm.qb[b][3][j][i + QX] = v[3];
-        if (P.fixed_region) {
+        if (near_fixed) {
             const bool inside = (n >= 0 && n < P.N && m >= 0 && m < P.M);
-            sm.fx[j][i] = (inside && near_fixed) ? (unsigned char)cell_fixed(P, P.x_min + n * P.dx, P.y_min + m * P.dy)
+            sm.fx[j][i] = inside ? (unsigned char)cell_fixed(P, P.x_min + n * P.dx, P.y_min + m * P.dy)
                                                  : 0;
         }
     }
+    return differs;
 }
 
 // After a bulk copy of the tile box into buffer b (zeros outside the
@@ -1332,7 +1308,7 @@ __device__ __forceinline__ void patch_tile_body(const StepParams& P, S& sm, int 
     const int N = P.N, M = P.M;
     const bool edge = n0 - 2 < 0 || n0 + TZ + 2 > N || m0 - 2 < 0 || m0 + TR + 2 > M;
     const bool near_fixed = tile_near_fixed<TZ, TR>(P, n0, m0);
-    if (!edge && !P.fixed_region) return;
+    if (!edge && !near_fixed) return;
     auto& q = sm.qb[b];
     for (int idx = threadIdx.x; idx < HR * HZ; idx += kThreads) {
         const int j = idx / HZ, i = idx - j * HZ;
@@ -1340,8 +1316,8 @@ __device__ __forceinline__ void patch_tile_body(const StepParams& P, S& sm, int 
         if (!rin && !cin) continue;
         const int n = n0 - 2 + i, m = m0 - 2 + j;
         const bool inside = (n >= 0 && n < N && m >= 0 && m < M);
-        if (P.fixed_region)
-            sm.fx[j][i] = (inside && near_fixed) ? (unsigned char)cell_fixed(P, P.x_min + n * P.dx, P.y_min + m * P.dy)
+        if (near_fixed)
+            sm.fx[j][i] = inside ? (unsigned char)cell_fixed(P, P.x_min + n * P.dx, P.y_min + m * P.dy)
                                                  : 0;
         if (inside) continue;
         int side, g, bn, bm, mn, mm;
@@ -1414,7 +1390,20 @@ __device__ __forceinline__ R uniform_face(const Gas<R>& g, R r, R p, R un, R ut,
     }
 }
 
-// A uniform tile (skip_uniform): every staged cell a face of the tile reads
+// Whether this thread's sample of the staged tile (every second cell of each
+// row) differs in density from the tile's first cell: the persistent kernels
+// ask it before the barrier that follows a tile's arrival, so a disturbed tile
+// is told from one that may be uniform without a barrier of its own.
+template <typename R, int TZ, int TR, typename S>
+__device__ __forceinline__ bool sample_differs(const S& sm, int b)
+{
+    static_assert(kThreads == TR * (TZ / 2), "a thread per second cell");
+    constexpr int QX = S::QX;
+    const int j = 2 + threadIdx.x / (TZ / 2), i = 2 + 2 * (threadIdx.x % (TZ / 2));
+    return !same_bits(sm.qb[b][0][j][i + QX], sm.qb[b][0][2][2 + QX]);
+}
+
+// A uniform tile: every staged cell a face of the tile reads
 // (the tile's rows over the full halo width, its columns over the full halo
 // height, ghost cells included) holds the bits of tile cell (0, 0), and the
 // flux of that state is finite.  Then every face of one orientation has the
@@ -1450,11 +1439,12 @@ __device__ __forceinline__ bool tile_uniform(const S& sm, int b, const Gas<R>& g
 
 // faces, exact-solver queue and conservative update of the tile staged in
 // buffer b.  TO_SMEM: the updated cells go to sm.out (for a bulk store)
-// instead of global memory.  Ends without a barrier.
-template <typename R, int FLUX, bool RECON, int LAYOUT, int TZ, int TR, bool TO_SMEM, bool SKIP = true,
+// instead of global memory.  may_skip (the same in all threads): the tile may
+// be uniform.  Ends without a barrier.
+template <typename R, int FLUX, bool RECON, int LAYOUT, int TZ, int TR, bool TO_SMEM,
           bool LATE_K = false, typename S>
 __device__ __forceinline__ void tile_body(const StepParams& P, S& sm, int b, const Gas<R>& g, int n0, int m0,
-                                          const StepConsts& K, TileAcc<R>& acc)
+                                          const StepConsts& K, TileAcc<R>& acc, bool may_skip)
 {
     constexpr int QX = S::QX;
     // ---- every face of the tile once, then the queue
@@ -1474,16 +1464,21 @@ __device__ __forceinline__ void tile_body(const StepParams& P, S& sm, int b, con
         if constexpr (sizeof(R) == 8) sm.tydrow[threadIdx.x] = (P.geom == 1) ? K.T_do / yd : 0.0;
         if constexpr (sizeof(R) == 4 && !LATE_K) sm.tyfrow[threadIdx.x] = (P.geom == 1) ? K.T_f / yf : 0.0f;
     }
-    // SKIP: the kernel carries the uniform-tile test (skip_uniform); the
-    // persistent kernel has a variant without it, so that the default path
-    // holds none of its code
-    bool skipped = false;
+    // A uniform tile skips the faces: those of one orientation have one flux,
+    // so the update's flux differences are exactly zero (it runs on zero
+    // fluxes: the same results), and thread 0 finds the two wave speeds.
+    // Undisturbed gas is most of a blast's grid: at 4096x2048, a third of the
+    // radius grown, FP32 HLL UNI_HLL ms per step; where every face is
+    // disturbed the sample taken before (may_skip) leaves nothing to test here.
+    // (Not in the FP64 kernels' small tiles, but for the exact solver: a grid
+    // that takes them waits for its disturbed tiles and for the code's fetch,
+    // 256x128 HLL 22.7 us per step without the test, 26.2 with it.)
+    constexpr bool kSkip = !(sizeof(R) == 8 && TZ == 16 && FLUX != 2);
     R sz, sr;
-    if (SKIP && P.skip_uniform && !P.region_select && !tile_near_fixed<TZ, TR>(P, n0, m0) &&
-        tile_uniform<R, FLUX, TZ, TR>(sm, b, g, sz, sr)) {
-        skipped = true;
-        // zero fluxes (the same flux on every face of an orientation: its
-        // differences are exactly zero) and the two wave speeds
+    const bool near = tile_near_fixed<TZ, TR>(P, n0, m0);
+    const bool skipped = kSkip && may_skip && !P.region_select && !near &&
+                         tile_uniform<R, FLUX, TZ, TR>(sm, b, g, sz, sr);
+    if (skipped) {
         constexpr int NF4 = (TR * (TZ + 1) + (TR + 1) * TZ) * 4;
         R* fz = &sm.Fz[0][0][0];
         R* fr = &sm.Fr[0][0][0];
@@ -1492,12 +1487,12 @@ __device__ __forceinline__ void tile_body(const StepParams& P, S& sm, int b, con
             put4(d, R(0), R(0), R(0), R(0));
         }
         if (threadIdx.x == 0) {
-            acc.smz = fmax(acc.smz, sz);
-            acc.smr = fmax(acc.smr, sr);
+            acc.smz = larger_speed(acc.smz, sz);
+            acc.smr = larger_speed(acc.smr, sr);
         }
+    } else {
+        face_pass<R, FLUX, RECON, TZ, TR>(P, sm, b, g, n0, m0, near, K.step, acc.rc, acc.fallback, acc.smz, acc.smr);
     }
-    if (!skipped)
-        face_pass<R, FLUX, RECON, TZ, TR, SKIP>(P, sm, b, g, n0, m0, K.step, acc.rc, acc.fallback, acc.smz, acc.smr);
     // persistent kernel: the previous tile's bulk store, issued by the copy
     // thread at the start of this face pass, has read sm.out before anything
     // overwrites it (the network's space in the queue phase, then the update)
@@ -1507,13 +1502,15 @@ __device__ __forceinline__ void tile_body(const StepParams& P, S& sm, int b, con
     __syncthreads();
     phase_mark(2);
     if constexpr (FLUX == 2) {
-        queue_pass<R, RECON, TZ, TR>(P, sm, b, g, n0, m0, K.step, acc.rc, acc.fallback, acc.smz, acc.smr);
-        __syncthreads();
-        phase_mark(3);
-        // persistent kernels: the next tile's queue starts empty (ordered
-        // before its face pass by the barrier between the tiles)
-        if constexpr (TO_SMEM) {
-            if (threadIdx.x == kCopyThread) sm.qn = 0u;
+        if (!skipped) {
+            queue_pass<R, RECON, TZ, TR>(P, sm, b, g, n0, m0, K.step, acc.rc, acc.fallback, acc.smz, acc.smr);
+            __syncthreads();
+            phase_mark(3);
+            // persistent kernels: the next tile's queue starts empty (ordered
+            // before its face pass by the barrier between the tiles)
+            if constexpr (TO_SMEM) {
+                if (threadIdx.x == kCopyThread) sm.qn = 0u;
+            }
         }
     }
 
@@ -1595,7 +1592,7 @@ __device__ __forceinline__ void tile_body(const StepParams& P, S& sm, int b, con
         if (n >= P.N || m >= P.M) continue;
         const int j = row + 2, i = col + 2;
         R o[4] = {qv[0][j][i + QX], qv[1][j][i + QX], qv[2][j][i + QX], qv[3][j][i + QX]};
-        if (!(P.fixed_region && sm.fx[j][i])) {
+        if (!(near && sm.fx[j][i])) {
             R in[4], f[4][4];
             load_cell(row, col, in, f);
             if constexpr (sizeof(R) == 8) {
@@ -1755,11 +1752,10 @@ __device__ __forceinline__ void step_tile(const StepParams& P, int bx, int by, u
         sm.qn = 0u;
         step_consts<R>(P, sK);
     }
-    stage_tile<R, LAYOUT, TZ, TR>(P, sm, 0, n0, m0);
-    __syncthreads();
+    const bool mixed = __syncthreads_or(stage_tile<R, LAYOUT, TZ, TR>(P, sm, 0, n0, m0));
     TileAcc<R> acc;
     acc.clear();
-    tile_body<R, FLUX, RECON, LAYOUT, TZ, TR, false>(P, sm, 0, g, n0, m0, sK, acc);
+    tile_body<R, FLUX, RECON, LAYOUT, TZ, TR, false>(P, sm, 0, g, n0, m0, sK, acc, !mixed);
     cta_epilogue<R>(P, acc, tiles, false);
 }
 
@@ -1861,7 +1857,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas<R, 2>())
 // once (one ticket per CTA).  A bulk copy that does not arrive within the
 // wait limit (P.wait_polls) sets AST_ST_TIMEOUT and is waited for with the
 // long limit; one that does not arrive even then ends the CTA's loop.
-template <typename R, int FLUX, bool RECON, bool SKIP>
+template <typename R, int FLUX, bool RECON>
 __global__ void __launch_bounds__(kThreads, sizeof(R) == 4 ? 4 : 2)
     step_kernel_tma(StepParams P, const __grid_constant__ CUtensorMap tin, const __grid_constant__ CUtensorMap tout)
 {
@@ -1875,6 +1871,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == 4 ? 4 : 2)
     __shared__ int2 s_org[2];      // their origins (n0, m0), set with s_tile by the copy thread
     __shared__ StepConsts sK;
     __shared__ int2 s_pend;        // copy thread: origin of the tile whose cells wait in sm.out
+    __shared__ volatile int s_late;   // a thread's wait for the tile ran out
     const int tid = threadIdx.x;
     const bool copier = tid == kCopyThread;
     const int tiles_z = (P.N + TZ - 1) / TZ;
@@ -1887,6 +1884,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == 4 ? 4 : 2)
         tma::mbar_init(&bar[1], 1);
         tma::fence_async_shared();
         step_consts<R>(P, sK);
+        s_late = 0;
         s_pend = make_int2(-1, -1);
         sm.qn = 0u;   // later tiles: reset after the previous tile's queue
         // the first two tiles: the first is copied now, the second at the
@@ -1919,8 +1917,11 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == 4 ? 4 : 2)
         // two tiles: every thread has finished the previous tile (its
         // update and its reads of the other buffer and of the output tile)
         // and fenced its shared-memory writes for the bulk copies.
+        // The barrier also asks whether the tile's sampled densities differ.
         bool arrived = tma::mbar_wait(&bar[b], (uint32_t)((k >> 1) & 1), P.wait_polls);
-        if (__syncthreads_or(!arrived)) {
+        if (!arrived) s_late = 1;
+        const bool mixed = __syncthreads_or(!arrived || sample_differs<R, TZ, TR>(sm, b));
+        if (s_late) {
             // the copy did not arrive within the wait limit: reported, then
             // waited for with the long limit (every CTA leaves with no copy
             // in flight; the next tile's copy is not issued yet), and the
@@ -1929,11 +1930,14 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == 4 ? 4 : 2)
             if (copier) acc.rc.status |= AST_ST_TIMEOUT;
             arrived = tma::mbar_wait(&bar[b], (uint32_t)((k >> 1) & 1));
             if (__syncthreads_or(!arrived)) break;
+            if (copier) s_late = 0;
+            __syncthreads();
         }
         phase_mark(0);
         // ghost cells (tiles at the grid's edge or near the fixed region
         // only: the others need no second barrier)
-        if (n0 - 2 < 0 || n0 + TZ + 2 > P.N || m0 - 2 < 0 || m0 + TR + 2 > P.M || P.fixed_region) {
+        if (n0 - 2 < 0 || n0 + TZ + 2 > P.N || m0 - 2 < 0 || m0 + TR + 2 > P.M ||
+            tile_near_fixed<TZ, TR>(P, n0, m0)) {
             patch_tile<R, TZ, TR>(P, sm, b, n0, m0);
             __syncthreads();
         }
@@ -1961,7 +1965,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == 4 ? 4 : 2)
             s_tile[b] = tnn;
             s_org[b] = make_int2((tnn % tiles_z) * TZ, (tnn / tiles_z) * TR);
         }
-        tile_body<R, FLUX, RECON, kSoA, TZ, TR, true, SKIP>(P, sm, b, g, n0, m0, sK, acc);
+        tile_body<R, FLUX, RECON, kSoA, TZ, TR, true>(P, sm, b, g, n0, m0, sK, acc, !mixed);
         // this thread's shared-memory writes (sm.out, ghost cells) before
         // the bulk copies that read or overwrite them (ordered by the next
         // tile's barrier, or the one below)
@@ -2097,6 +2101,7 @@ __global__ void __launch_bounds__(kThreads, 4)
     __shared__ int4 s_pend;
     __shared__ StepConsts sK[2];
     __shared__ int s_last;
+    __shared__ volatile int s_late;   // a thread's wait for the tile ran out
     // copy thread only: the entry of the next tile to be issued, and per
     // buffer the dt and step of its tile's problem (asynchronous copies)
     __shared__ __align__(16) BatchTile s_next;
@@ -2124,6 +2129,7 @@ __global__ void __launch_bounds__(kThreads, 4)
         tma::mbar_init(&bar[1], 1);
         tma::fence_async_shared();
         sm.qn = 0u;
+        s_late = 0;
         s_pend = make_int4(-1, 0, 0, 0);
         const int t0 = (int)atomicAdd(counter, 1u);
         s_tile[0] = t0;
@@ -2151,7 +2157,9 @@ __global__ void __launch_bounds__(kThreads, 4)
         // previous tile (its update, its reads of this buffer's slots) and
         // fenced its shared-memory writes for the bulk copies
         bool arrived = tma::mbar_wait(&bar[b], (uint32_t)((k >> 1) & 1), wait_polls);
-        if (__syncthreads_or(!arrived)) {
+        if (!arrived) s_late = 1;
+        const bool mixed = __syncthreads_or(!arrived || sample_differs<R, TZ, TR>(sm, b));
+        if (s_late) {
             // reported (from global memory: the parameters come with the
             // copy), then waited for with the long limit and computed; the
             // next tile's copy is not issued yet, so a copy that does not
@@ -2159,10 +2167,13 @@ __global__ void __launch_bounds__(kThreads, 4)
             if (copier) atomicOr(&Ps[j].clock->status, AST_ST_TIMEOUT);
             arrived = tma::mbar_wait(&bar[b], (uint32_t)((k >> 1) & 1));
             if (__syncthreads_or(!arrived)) break;
+            if (copier) s_late = 0;
+            __syncthreads();
         }
         phase_mark(0);
         const StepParams& P = sP[b];
-        if (n0 - 2 < 0 || n0 + TZ + 2 > P.N || m0 - 2 < 0 || m0 + TR + 2 > P.M || P.fixed_region) {
+        if (n0 - 2 < 0 || n0 + TZ + 2 > P.N || m0 - 2 < 0 || m0 + TR + 2 > P.M ||
+            tile_near_fixed<TZ, TR>(P, n0, m0)) {
             patch_tile<R, TZ, TR>(P, sm, b, n0, m0);
             __syncthreads();
         }
@@ -2192,13 +2203,13 @@ __global__ void __launch_bounds__(kThreads, 4)
         }
         if constexpr (MIXED) {
             switch (w.x >> 24) {
-            case 0: tile_body<R, 0, RECON, kSoA, TZ, TR, true, true, true>(P, sm, b, P.gf, n0, m0, sK[b], acc); break;
-            case 1: tile_body<R, 1, RECON, kSoA, TZ, TR, true, true, true>(P, sm, b, P.gf, n0, m0, sK[b], acc); break;
-            case 3: tile_body<R, 3, RECON, kSoA, TZ, TR, true, true, true>(P, sm, b, P.gf, n0, m0, sK[b], acc); break;
-            default: tile_body<R, 2, RECON, kSoA, TZ, TR, true, true, true>(P, sm, b, P.gf, n0, m0, sK[b], acc); break;
+            case 0: tile_body<R, 0, RECON, kSoA, TZ, TR, true, true>(P, sm, b, P.gf, n0, m0, sK[b], acc, !mixed); break;
+            case 1: tile_body<R, 1, RECON, kSoA, TZ, TR, true, true>(P, sm, b, P.gf, n0, m0, sK[b], acc, !mixed); break;
+            case 3: tile_body<R, 3, RECON, kSoA, TZ, TR, true, true>(P, sm, b, P.gf, n0, m0, sK[b], acc, !mixed); break;
+            default: tile_body<R, 2, RECON, kSoA, TZ, TR, true, true>(P, sm, b, P.gf, n0, m0, sK[b], acc, !mixed); break;
             }
         } else {
-            tile_body<R, FLUX, RECON, kSoA, TZ, TR, true, true, true>(P, sm, b, P.gf, n0, m0, sK[b], acc);
+            tile_body<R, FLUX, RECON, kSoA, TZ, TR, true, true>(P, sm, b, P.gf, n0, m0, sK[b], acc, !mixed);
         }
         // this thread's shared-memory writes before the bulk copies that
         // read or overwrite them (ordered by the next barrier)
