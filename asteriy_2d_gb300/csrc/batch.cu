@@ -456,6 +456,7 @@ int ast_batch_create(const ast_config* cfgs, int nprob, ast_batch** out)
                     e.sf = s | (fk << 24);
                     e.n0 = (t % tz) * kTmaTZ;
                     e.m0 = (t / tz) * kTmaTR;
+                    e.inside = e.n0 >= 4 && e.n0 + kTmaTZ + 4 <= c.N && e.m0 >= 2 && e.m0 + kTmaTR + 2 <= c.M;
                     e.clock = B->clocks + order[s];
                     work.push_back(e);
                 }

@@ -324,6 +324,13 @@ struct TileCore {
     float yfrow[TR];             // and in FP32
     double tydrow[TR];           // T_do / r of the rows (axisymmetric grid; FP64 kernels)
     float tyfrow[TR];            // and in FP32 (FP32 kernels with the step's constants set before the tile)
+    // a CTA's last uniform state (persistent kernels of one problem): its wave
+    // speeds are counted (uni_known), its update gives all cells one state
+    // (uni_one); and per buffer the last iteration that left this state's
+    // updated cells in the whole output tile
+    R uni[4];
+    R uni_max[2];                // the uniform tiles' largest wave speeds (thread 0)
+    int uni_known, uni_one, uni_out[2];
 };
 
 // the exact solver's queue: faces as 16-bit codes (face index | active <<
@@ -803,25 +810,7 @@ __device__ __forceinline__ void face_flux(const StepParams& P, S& sm, const Gas<
     constexpr int TT = ZF ? 3 : 2;           // tangential velocity component
     R F[4];
     R Sp;
-    // FP64, the HLL or HLLC flux, the faces of every active lane of the warp
-    // with one state (one bit pattern, rho > 0, p > 0) on both sides
-    // (undisturbed gas): that state's physical flux (flux_physical; the
-    // solvers' formulas give it up to rounding) for two divisions, two square
-    // roots and the star-state arithmetic.  A warp vote, so that warps with
-    // other faces run as before; bit tests, not FP64 compares (this GPU's
-    // FP64 pipe is slow).
-    bool same = false;
-    if constexpr (sizeof(R) == 8 && FLUX != 2) {
-        const bool eq = (FLUX == 0 || FLUX == 1 || !hi) && same_bits(L[0], U[0]) && same_bits(L[1], U[1]) &&
-                        same_bits(L[2], U[2]) && same_bits(L[3], U[3]) && positive_bits(L[0]) &&
-                        positive_bits(L[1]);
-        if (__all_sync(__activemask(), eq)) {
-            Sp = flux_physical(g, L[0], L[1], L[NN], L[TT], F);
-            same = true;
-        }
-    }
-    if (same) {
-    } else if constexpr (FLUX == 2) {
+    if constexpr (FLUX == 2) {
         if (!active) {
             // no updated cell uses this face (both cells outside the grid or
             // held fixed): not solved, so the solver's counters see the same
@@ -1403,50 +1392,132 @@ __device__ __forceinline__ bool sample_differs(const S& sm, int b)
     return !same_bits(sm.qb[b][0][j][i + QX], sm.qb[b][0][2][2 + QX]);
 }
 
-// A uniform tile: every staged cell a face of the tile reads
-// (the tile's rows over the full halo width, its columns over the full halo
-// height, ghost cells included) holds the bits of tile cell (0, 0), and the
-// flux of that state is finite.  Then every face of one orientation has the
-// same flux, the update's flux differences are exactly zero, and only the
-// wave speeds of the two orientations are needed: returned in sz / sr
-// (valid in thread 0).  A barrier: called by all threads.
-template <typename R, int FLUX, int TZ, int TR, typename S>
-__device__ __forceinline__ bool tile_uniform(const S& sm, int b, const Gas<R>& g, R& sz, R& sr)
+// Whether every staged cell a face of the tile reads (the tile's rows over the
+// full halo width, its columns over the full halo height, ghost cells
+// included) holds the bits of tile cell (0, 0).  box: the staged box lies
+// inside the grid and is compared whole, in 16-byte words.  A barrier.
+template <typename R, int TZ, int TR, typename S>
+__device__ __forceinline__ bool tile_same(const S& sm, int b, bool box)
 {
     constexpr int HZ = S::HZ, HR = S::HR, QX = S::QX;
-    using U = std::conditional_t<sizeof(R) == 4, unsigned int, unsigned long long>;
+    constexpr int W = 16 / sizeof(R), NV = HR * S::HZP / W;   // words per plane
+    static_assert(HR * S::HZP % W == 0, "whole words");
     const auto& q = sm.qb[b];
-    auto bits = [](R v) { return *reinterpret_cast<const U*>(&v); };
-    const R s0 = q[0][2][2 + QX], s1 = q[1][2][2 + QX], s2 = q[2][2][2 + QX], s3 = q[3][2][2 + QX];
-    const U r0 = bits(s0), r1 = bits(s1), r2 = bits(s2), r3 = bits(s3);
-    bool same = true;
-    for (int idx = threadIdx.x; idx < HR * HZ; idx += kThreads) {
-        const int j = idx / HZ, i = idx - j * HZ;
-        const bool rin = (j >= 2 && j < TR + 2), cin = (i >= 2 && i < TZ + 2);
-        if (!rin && !cin) continue;   // the corners: read by no face
-        same = same && bits(q[0][j][i + QX]) == r0 && bits(q[1][j][i + QX]) == r1 && bits(q[2][j][i + QX]) == r2 &&
-               bits(q[3][j][i + QX]) == r3;
+    int d = 0;
+    if (box) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const R c = q[k][2][2 + QX];
+            for (int v = threadIdx.x; v < NV; v += kThreads) {
+                const int4 w = reinterpret_cast<const int4*>(&q[k][0][0])[v];
+                if constexpr (sizeof(R) == 4) {
+                    const int i = __float_as_int(c);
+                    d |= (w.x ^ i) | (w.y ^ i) | (w.z ^ i) | (w.w ^ i);
+                } else {
+                    const int lo = (int)__double_as_longlong(c), hi = (int)(__double_as_longlong(c) >> 32);
+                    d |= (w.x ^ lo) | (w.y ^ hi) | (w.z ^ lo) | (w.w ^ hi);
+                }
+            }
+        }
+    } else {
+        for (int idx = threadIdx.x; idx < HR * HZ; idx += kThreads) {
+            const int j = idx / HZ, i = idx - j * HZ;
+            const bool rin = (j >= 2 && j < TR + 2), cin = (i >= 2 && i < TZ + 2);
+            if (!rin && !cin) continue;   // the corners: read by no face
+#pragma unroll
+            for (int k = 0; k < 4; k++) d |= same_bits(q[k][j][i + QX], q[k][2][2 + QX]) ? 0 : 1;
+        }
     }
+    return __syncthreads_and(d == 0);
+}
+
+// The wave speeds of a uniform tile's faces (valid in thread 0), and whether
+// its flux is finite: then every face of one orientation has the same flux
+// and the update's flux differences are exactly zero.  A barrier.
+template <typename R, int FLUX, typename S>
+__device__ __forceinline__ bool uniform_speeds(const S& sm, int b, const Gas<R>& g, R& sz, R& sr)
+{
+    constexpr int QX = S::QX;
+    const auto& q = sm.qb[b];
+    bool ok = true;
     if (threadIdx.x == 0) {
+        const R s0 = q[0][2][2 + QX], s1 = q[1][2][2 + QX], s2 = q[2][2][2 + QX], s3 = q[3][2][2 + QX];
         R F[4], G[4];
         sz = uniform_face<R, FLUX>(g, s0, s1, s2, s3, F);   // z faces: normal v_z
         sr = uniform_face<R, FLUX>(g, s0, s1, s3, s2, G);   // r faces: normal v_r
-        for (int k = 0; k < 4; k++) same = same && isfinite(F[k]) && isfinite(G[k]);
-        same = same && isfinite(sz) && isfinite(sr);
+        for (int k = 0; k < 4; k++) ok = ok && isfinite(F[k]) && isfinite(G[k]);
+        ok = ok && isfinite(sz) && isfinite(sr);
     }
-    return __syncthreads_and(same);
+    return __syncthreads_and(ok);
+}
+
+// What the faces and the update of a tile that may be uniform (its sampled
+// densities are equal) have to do: kMixed everything; kUniform only the update:
+// every face of one orientation has one flux, so the update's flux differences
+// are exactly zero, and it runs on zero fluxes (the same results); kStored
+// nothing: with CACHE (a CTA's tiles of one problem), the CTA's last tile had
+// this state, its cells update to one state (no v_r, no source or force:
+// uni_one) and the output tile still holds them.  The wave speeds of a new
+// state go to sm.uni_max.  box: the staged box lies inside the grid; plain: a
+// whole tile whose cells all take the same update (no row of the FP32 form's
+// FP64 update, no force or source).  A barrier; out of line, so that the disturbed tiles'
+// code stays as it is without it (inlined it cost them up to 25%).
+// Undisturbed gas is most of a blast's grid: UNI_MEASURED
+// Not used by the FP64 kernels' small tiles but for the exact solver (kSkip): a
+// grid that takes them waits for its disturbed tiles and for the code's fetch,
+// 256x128 HLL 22.7 us per step without the test, 26.2 with it.
+enum { kMixed = 0, kUniform = 1, kStored = 2 };
+template <typename R, int FLUX, int TZ>
+constexpr bool skips_uniform() { return !(sizeof(R) == 8 && TZ == 16 && FLUX != 2); }
+
+template <typename R, int FLUX, int TZ, int TR, bool CACHE, typename S>
+__device__ __noinline__ int uniform_tile(const StepParams& P, int b, bool box, bool plain, int iter)
+{
+    S& sm = tile_smem<S>();
+    if (!tile_same<R, TZ, TR>(sm, b, box)) return kMixed;
+    const auto& q = sm.qb[b];
+    constexpr int QX = S::QX;
+    bool known = false;
+    if constexpr (CACHE) {
+        known = sm.uni_known != 0;
+#pragma unroll
+        for (int k = 0; k < 4; k++) known = known && same_bits(sm.uni[k], q[k][2][2 + QX]);
+        // (slots by parity: this iteration's is written while the last one's is read)
+        const bool stored = known && plain && sm.uni_out[b ^ 1] == iter - 1;
+        if (threadIdx.x == 0) sm.uni_out[b] = (stored || (known && plain && sm.uni_one)) ? iter : -1;
+        if (stored) return kStored;
+    }
+    if (known) return kUniform;
+    const Gas<R>& g = gas_of<R>(P);
+    R sz = R(0), sr = R(0);
+    if (!uniform_speeds<R, FLUX>(sm, b, g, sz, sr)) return kMixed;
+    if (threadIdx.x == 0) {
+        // (every thread has read the record before the barrier in uniform_speeds)
+        sm.uni_max[0] = larger_speed(sm.uni_max[0], sz);
+        sm.uni_max[1] = larger_speed(sm.uni_max[1], sr);
+        if constexpr (CACHE) {
+            const R r = q[0][2][2 + QX], p = q[1][2][2 + QX], vz = q[2][2][2 + QX], vr = q[3][2][2 + QX];
+            sm.uni[0] = r; sm.uni[1] = p; sm.uni[2] = vz; sm.uni[3] = vr;
+            // one updated state, no floor, no FP64 pressure recovery
+            const R ke = R(0.5) * r * (vz * vz + vr * vr);
+            sm.uni_one = (P.geom != 1 || vr == R(0)) && r > R(0) && p > R(0) && ke < R(0.98) * (p * g.inv_g1 + ke);
+            sm.uni_known = 1;
+        }
+    }
+    return kUniform;
 }
 
 // faces, exact-solver queue and conservative update of the tile staged in
 // buffer b.  TO_SMEM: the updated cells go to sm.out (for a bulk store)
-// instead of global memory.  may_skip (the same in all threads): the tile may
-// be uniform.  Ends without a barrier.
-template <typename R, int FLUX, bool RECON, int LAYOUT, int TZ, int TR, bool TO_SMEM,
-          bool LATE_K = false, typename S>
+// instead of global memory.  uniform (the same in all threads): the tile is
+// uniform (uniform_tile).  Ends without a barrier.
+template <typename R, int FLUX, bool RECON, int LAYOUT, int TZ, int TR, bool TO_SMEM, bool LATE_K = false,
+          typename S>
 __device__ __forceinline__ void tile_body(const StepParams& P, S& sm, int b, const Gas<R>& g, int n0, int m0,
-                                          const StepConsts& K, TileAcc<R>& acc, bool may_skip)
+                                          const StepConsts& K, TileAcc<R>& acc, bool uniform)
 {
     constexpr int QX = S::QX;
+    const bool near = tile_near_fixed<TZ, TR>(P, n0, m0);
     // ---- every face of the tile once, then the queue
     // r of the tile's rows for the update (the barrier after the faces
     // orders these writes before their use)
@@ -1464,31 +1535,14 @@ __device__ __forceinline__ void tile_body(const StepParams& P, S& sm, int b, con
         if constexpr (sizeof(R) == 8) sm.tydrow[threadIdx.x] = (P.geom == 1) ? K.T_do / yd : 0.0;
         if constexpr (sizeof(R) == 4 && !LATE_K) sm.tyfrow[threadIdx.x] = (P.geom == 1) ? K.T_f / yf : 0.0f;
     }
-    // A uniform tile skips the faces: those of one orientation have one flux,
-    // so the update's flux differences are exactly zero (it runs on zero
-    // fluxes: the same results), and thread 0 finds the two wave speeds.
-    // Undisturbed gas is most of a blast's grid: at 4096x2048, a third of the
-    // radius grown, FP32 HLL UNI_HLL ms per step; where every face is
-    // disturbed the sample taken before (may_skip) leaves nothing to test here.
-    // (Not in the FP64 kernels' small tiles, but for the exact solver: a grid
-    // that takes them waits for its disturbed tiles and for the code's fetch,
-    // 256x128 HLL 22.7 us per step without the test, 26.2 with it.)
-    constexpr bool kSkip = !(sizeof(R) == 8 && TZ == 16 && FLUX != 2);
-    R sz, sr;
-    const bool near = tile_near_fixed<TZ, TR>(P, n0, m0);
-    const bool skipped = kSkip && may_skip && !P.region_select && !near &&
-                         tile_uniform<R, FLUX, TZ, TR>(sm, b, g, sz, sr);
-    if (skipped) {
+    if (uniform) {
+        // zero fluxes: the differences of a uniform tile's fluxes
         constexpr int NF4 = (TR * (TZ + 1) + (TR + 1) * TZ) * 4;
         R* fz = &sm.Fz[0][0][0];
         R* fr = &sm.Fr[0][0][0];
         for (int w = threadIdx.x; w < NF4 / 4; w += kThreads) {
             R* d = (w < TR * (TZ + 1)) ? fz + 4 * w : fr + 4 * (w - TR * (TZ + 1));
             put4(d, R(0), R(0), R(0), R(0));
-        }
-        if (threadIdx.x == 0) {
-            acc.smz = larger_speed(acc.smz, sz);
-            acc.smr = larger_speed(acc.smr, sr);
         }
     } else {
         face_pass<R, FLUX, RECON, TZ, TR>(P, sm, b, g, n0, m0, near, K.step, acc.rc, acc.fallback, acc.smz, acc.smr);
@@ -1502,15 +1556,13 @@ __device__ __forceinline__ void tile_body(const StepParams& P, S& sm, int b, con
     __syncthreads();
     phase_mark(2);
     if constexpr (FLUX == 2) {
-        if (!skipped) {
-            queue_pass<R, RECON, TZ, TR>(P, sm, b, g, n0, m0, K.step, acc.rc, acc.fallback, acc.smz, acc.smr);
-            __syncthreads();
-            phase_mark(3);
-            // persistent kernels: the next tile's queue starts empty (ordered
-            // before its face pass by the barrier between the tiles)
-            if constexpr (TO_SMEM) {
-                if (threadIdx.x == kCopyThread) sm.qn = 0u;
-            }
+        queue_pass<R, RECON, TZ, TR>(P, sm, b, g, n0, m0, K.step, acc.rc, acc.fallback, acc.smz, acc.smr);
+        __syncthreads();
+        phase_mark(3);
+        // persistent kernels: the next tile's queue starts empty (ordered
+        // before its face pass by the barrier between the tiles)
+        if constexpr (TO_SMEM) {
+            if (threadIdx.x == kCopyThread) sm.qn = 0u;
         }
     }
 
@@ -1750,12 +1802,22 @@ __device__ __forceinline__ void step_tile(const StepParams& P, int bx, int by, u
     const Gas<R>& g = *reinterpret_cast<const Gas<R>*>(sizeof(R) == 8 ? (const void*)&P.gd : (const void*)&P.gf);
     if (threadIdx.x == 0) {
         sm.qn = 0u;
+        sm.uni_max[0] = sm.uni_max[1] = R(0);
         step_consts<R>(P, sK);
     }
     const bool mixed = __syncthreads_or(stage_tile<R, LAYOUT, TZ, TR>(P, sm, 0, n0, m0));
     TileAcc<R> acc;
     acc.clear();
-    tile_body<R, FLUX, RECON, LAYOUT, TZ, TR, false>(P, sm, 0, g, n0, m0, sK, acc, !mixed);
+    int uni = kMixed;
+    if constexpr (skips_uniform<R, FLUX, TZ>()) {
+        if (!mixed && !P.region_select && !tile_near_fixed<TZ, TR>(P, n0, m0))
+            uni = uniform_tile<R, FLUX, TZ, TR, false, S>(P, 0, false, false, 0);
+    }
+    tile_body<R, FLUX, RECON, LAYOUT, TZ, TR, false>(P, sm, 0, g, n0, m0, sK, acc, uni == kUniform);
+    if (threadIdx.x == 0) {
+        acc.smz = larger_speed(acc.smz, sm.uni_max[0]);
+        acc.smr = larger_speed(acc.smr, sm.uni_max[1]);
+    }
     cta_epilogue<R>(P, acc, tiles, false);
 }
 
@@ -1769,7 +1831,7 @@ constexpr int min_ctas() { return sizeof(R) == 8 ? 2 : 4; }
 
 // one problem: a CTA per tile, grid (tiles along z, tiles along r)
 template <typename R, int FLUX, bool RECON, int LAYOUT, int TZ, int TR>
-__global__ void __launch_bounds__(kThreads, min_ctas<R, FLUX>()) step_kernel(StepParams P)
+__global__ void __launch_bounds__(kThreads, min_ctas<R, FLUX>()) step_kernel(const __grid_constant__ StepParams P)
 {
     step_tile<R, FLUX, RECON, LAYOUT, TZ, TR>(P, blockIdx.x, blockIdx.y + P.band_lo,
                                               P.units > 0 ? (unsigned)P.units : gridDim.x * gridDim.y);
@@ -1859,7 +1921,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas<R, 2>())
 // long limit; one that does not arrive even then ends the CTA's loop.
 template <typename R, int FLUX, bool RECON>
 __global__ void __launch_bounds__(kThreads, sizeof(R) == 4 ? 4 : 2)
-    step_kernel_tma(StepParams P, const __grid_constant__ CUtensorMap tin, const __grid_constant__ CUtensorMap tout)
+    step_kernel_tma(const __grid_constant__ StepParams P, const __grid_constant__ CUtensorMap tin, const __grid_constant__ CUtensorMap tout)
 {
     constexpr int TZ = kTmaTZ, TR = kTmaTR;
     using S = TileSmem<R, FLUX, TZ, TR, 2>;
@@ -1885,6 +1947,9 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == 4 ? 4 : 2)
         tma::fence_async_shared();
         step_consts<R>(P, sK);
         s_late = 0;
+        sm.uni_known = 0;
+        sm.uni_max[0] = sm.uni_max[1] = R(0);
+        sm.uni_out[0] = sm.uni_out[1] = -2;
         s_pend = make_int2(-1, -1);
         sm.qn = 0u;   // later tiles: reset after the previous tile's queue
         // the first two tiles: the first is copied now, the second at the
@@ -1920,7 +1985,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == 4 ? 4 : 2)
         // The barrier also asks whether the tile's sampled densities differ.
         bool arrived = tma::mbar_wait(&bar[b], (uint32_t)((k >> 1) & 1), P.wait_polls);
         if (!arrived) s_late = 1;
-        const bool mixed = __syncthreads_or(!arrived || sample_differs<R, TZ, TR>(sm, b));
+        const bool mixed = __syncthreads_or((int)!arrived | (int)sample_differs<R, TZ, TR>(sm, b));
         if (s_late) {
             // the copy did not arrive within the wait limit: reported, then
             // waited for with the long limit (every CTA leaves with no copy
@@ -1965,7 +2030,14 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == 4 ? 4 : 2)
             s_tile[b] = tnn;
             s_org[b] = make_int2((tnn % tiles_z) * TZ, (tnn / tiles_z) * TR);
         }
-        tile_body<R, FLUX, RECON, kSoA, TZ, TR, true>(P, sm, b, g, n0, m0, sK, acc, !mixed);
+        int uni = kMixed;
+        if (!mixed && !P.region_select && !tile_near_fixed<TZ, TR>(P, n0, m0)) {
+            const bool box = n0 >= 4 && n0 + TZ + 4 <= P.N && m0 >= 2 && m0 + TR + 2 <= P.M;
+            const bool plain =
+                !(P.geom == 1 && m0 < 4) && n0 + TZ <= P.N && m0 + TR <= P.M && !P.body_force && !P.nsrc;
+            uni = uniform_tile<R, FLUX, TZ, TR, true, S>(P, b, box, plain, k);
+        }
+        if (uni != kStored) tile_body<R, FLUX, RECON, kSoA, TZ, TR, true>(P, sm, b, g, n0, m0, sK, acc, uni == kUniform);
         // this thread's shared-memory writes (sm.out, ghost cells) before
         // the bulk copies that read or overwrite them (ordered by the next
         // tile's barrier, or the one below)
@@ -1980,6 +2052,10 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == 4 ? 4 : 2)
         }
         tma::store_wait_all();
     }
+    if (tid == 0) {
+        acc.smz = larger_speed(acc.smz, sm.uni_max[0]);
+        acc.smr = larger_speed(acc.smr, sm.uni_max[1]);
+    }
     cta_epilogue<R>(P, acc, P.units > 0 ? (unsigned)P.units : gridDim.x, true);
     phase_mark(5);
     phase_mark(kPhaseFlush, P.clock);
@@ -1990,7 +2066,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == 4 ? 4 : 2)
 struct __align__(16) BatchTile {
     int sf;
     int n0, m0;
-    int rsv_;
+    int inside;                    // the staged box lies inside the grid
     DevClock* clock;
     long long rsv2_;
 };
@@ -2097,7 +2173,7 @@ __global__ void __launch_bounds__(kThreads, 4)
     __shared__ __align__(16) StepParams sP[2];
     __shared__ __align__(8) uint64_t bar[2];
     __shared__ int s_tile[2];
-    __shared__ int4 s_work[2];     // {slot | FLUX << 24, n0, m0, 0} of the buffer's tile
+    __shared__ int4 s_work[2];     // {slot | FLUX << 24, n0, m0, inside} of the buffer's tile
     __shared__ int4 s_pend;
     __shared__ StepConsts sK[2];
     __shared__ int s_last;
@@ -2112,7 +2188,7 @@ __global__ void __launch_bounds__(kThreads, 4)
     // the box and the parameters of entry w into buffer bb; its dt and step
     auto issue = [&](int bb, const BatchTile& w) {
         const int jn = w.sf & 0xffffff;
-        s_work[bb] = make_int4(w.sf, w.n0, w.m0, 0);
+        s_work[bb] = make_int4(w.sf, w.n0, w.m0, w.inside);
         tma::mbar_expect(&bar[bb], kBoxBytes + kParBytes);
         tma::load_3d(&tin[jn], &sm.qb[bb][0][0][0], &bar[bb], w.n0 - 4, w.m0 - 2, 0);
         tma::load_bulk(&sP[bb], Ps + jn, kParBytes, &bar[bb]);
@@ -2158,7 +2234,7 @@ __global__ void __launch_bounds__(kThreads, 4)
         // fenced its shared-memory writes for the bulk copies
         bool arrived = tma::mbar_wait(&bar[b], (uint32_t)((k >> 1) & 1), wait_polls);
         if (!arrived) s_late = 1;
-        const bool mixed = __syncthreads_or(!arrived || sample_differs<R, TZ, TR>(sm, b));
+        const bool mixed = __syncthreads_or((int)!arrived | (int)sample_differs<R, TZ, TR>(sm, b));
         if (s_late) {
             // reported (from global memory: the parameters come with the
             // copy), then waited for with the long limit and computed; the
@@ -2201,15 +2277,34 @@ __global__ void __launch_bounds__(kThreads, 4)
             // this tile's step constants (read after the face pass's barrier)
             step_consts_of<R>(P, s_tdo[b], (int)s_step[b], sK[b]);
         }
+        int uni = kMixed;
+        if (!mixed && !P.region_select && !tile_near_fixed<TZ, TR>(P, n0, m0)) {
+            if (tid == 0) sm.uni_max[0] = sm.uni_max[1] = 0.0f;
+            if constexpr (MIXED) {
+                switch (w.x >> 24) {
+                case 0: uni = uniform_tile<R, 0, TZ, TR, false, S>(P, b, w.w != 0, false, 0); break;
+                case 1: uni = uniform_tile<R, 1, TZ, TR, false, S>(P, b, w.w != 0, false, 0); break;
+                case 3: uni = uniform_tile<R, 3, TZ, TR, false, S>(P, b, w.w != 0, false, 0); break;
+                default: uni = uniform_tile<R, 2, TZ, TR, false, S>(P, b, w.w != 0, false, 0); break;
+                }
+            } else {
+                uni = uniform_tile<R, FLUX, TZ, TR, false, S>(P, b, w.w != 0, false, 0);
+            }
+            if (tid == 0) {
+                acc.smz = larger_speed(acc.smz, sm.uni_max[0]);
+                acc.smr = larger_speed(acc.smr, sm.uni_max[1]);
+            }
+        }
+        const bool one = uni == kUniform;
         if constexpr (MIXED) {
             switch (w.x >> 24) {
-            case 0: tile_body<R, 0, RECON, kSoA, TZ, TR, true, true>(P, sm, b, P.gf, n0, m0, sK[b], acc, !mixed); break;
-            case 1: tile_body<R, 1, RECON, kSoA, TZ, TR, true, true>(P, sm, b, P.gf, n0, m0, sK[b], acc, !mixed); break;
-            case 3: tile_body<R, 3, RECON, kSoA, TZ, TR, true, true>(P, sm, b, P.gf, n0, m0, sK[b], acc, !mixed); break;
-            default: tile_body<R, 2, RECON, kSoA, TZ, TR, true, true>(P, sm, b, P.gf, n0, m0, sK[b], acc, !mixed); break;
+            case 0: tile_body<R, 0, RECON, kSoA, TZ, TR, true, true>(P, sm, b, P.gf, n0, m0, sK[b], acc, one); break;
+            case 1: tile_body<R, 1, RECON, kSoA, TZ, TR, true, true>(P, sm, b, P.gf, n0, m0, sK[b], acc, one); break;
+            case 3: tile_body<R, 3, RECON, kSoA, TZ, TR, true, true>(P, sm, b, P.gf, n0, m0, sK[b], acc, one); break;
+            default: tile_body<R, 2, RECON, kSoA, TZ, TR, true, true>(P, sm, b, P.gf, n0, m0, sK[b], acc, one); break;
             }
         } else {
-            tile_body<R, FLUX, RECON, kSoA, TZ, TR, true, true>(P, sm, b, P.gf, n0, m0, sK[b], acc, !mixed);
+            tile_body<R, FLUX, RECON, kSoA, TZ, TR, true, true>(P, sm, b, P.gf, n0, m0, sK[b], acc, one);
         }
         // this thread's shared-memory writes before the bulk copies that
         // read or overwrite them (ordered by the next barrier)
