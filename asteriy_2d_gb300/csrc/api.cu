@@ -209,14 +209,10 @@ int ast_create(const ast_config* cfg, ast_solver** out)
             S->sweep = true;
         }
     }
-    // FP64: the persistent kernel for the HLL family on grids of at least
-    // two 32x16 tiles per SM (smaller grids step with one CTA per tile of
-    // 16x16).  The exact solver keeps one CTA per tile: for it the
-    // persistent kernel measured 8% slower (11.32 against 10.44 ms per step
-    // at step 1000 of the 4096x2048 blast; HLL 4.79 against 5.20 ms), and
-    // 10% slower again with today's face pass (11.02 against 10.03 ms).
+    // FP64: the persistent kernel on grids of at least two 32x16 tiles per SM
+    // (the exact solver: eight), smaller grids with one CTA per tile of 16x16
     const long long tiles32 = (long long)((cfg->N + kTZ - 1) / kTZ) * ((cfg->M + kTR - 1) / kTR);
-    const bool tma64 = S->elem == 8 && cfg->flux != AST_FLUX_GODUNOV && tiles32 >= 2LL * sm_count();
+    const bool tma64 = S->elem == 8 && tiles32 >= (cfg->flux == AST_FLUX_GODUNOV ? 8LL : 2LL) * sm_count();
     if (rc == AST_OK && (S->elem == 4 || tma64) && cfg->persistent && !want_sweep) {
         // box loads of tile + halo (TZ+8 x TR+4), stores of the tile (TZ x TR)
         for (int b = 0; b < 2 && rc == AST_OK; b++) {

@@ -1,5 +1,5 @@
 // step_f64.cu - step kernel instantiations for FP64 state planes (solver path):
-// one CTA per tile, and the persistent kernel (not for the exact solver).
+// one CTA per tile, and the persistent kernel.
 #include "launch.cuh"
 
 namespace ast {
@@ -14,13 +14,13 @@ int launch_step_tma64(const StepParams& P, const CUtensorMap& tin, const CUtenso
         if (flux == AST_FLUX_HLLC) AST_TMA64(1, true);
         if (flux == AST_FLUX_HLLC_A) AST_TMA64(3, true);
         if (flux == AST_FLUX_HLLCQ) AST_TMA64(4, true);
-        return set_error(AST_ERR_UNSUPPORTED, "the FP64 exact solver steps with one CTA per tile");
+        AST_TMA64(2, true);
     }
     if (flux == AST_FLUX_HLL) AST_TMA64(0, false);
     if (flux == AST_FLUX_HLLC) AST_TMA64(1, false);
     if (flux == AST_FLUX_HLLC_A) AST_TMA64(3, false);
     if (flux == AST_FLUX_HLLCQ) AST_TMA64(4, false);
-    return set_error(AST_ERR_UNSUPPORTED, "the FP64 exact solver steps with one CTA per tile");
+    AST_TMA64(2, false);
 #undef AST_TMA64
 }
 }  // namespace ast
