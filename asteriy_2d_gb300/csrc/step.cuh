@@ -2039,6 +2039,18 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == 4 ? 4 : 2)
         }
         phase_mark(1);
         if (copier) {
+            // the next tile's box into the other buffer (last read by the
+            // previous tile, which every thread finished before the barriers
+            // above): first, since uniform tiles wait for nothing else; then
+            // the counter's atomic for the tile after it, into this buffer's
+            // slots (every thread has read them)
+            int tnn = tiles;
+            if (s_tile[b ^ 1] < tiles) {
+                tma::mbar_expect(&bar[b ^ 1], kBoxBytes);
+                tma::load_3d(&tin, &sm.qb[b ^ 1][0][0][0], &bar[b ^ 1], s_org[b ^ 1].x - 4, s_org[b ^ 1].y - 2,
+                             0);
+                tnn = t_lo + (int)atomicAdd(&P.clock->next_tile, 1u);
+            }
             // the previous tile's cells (sm.out is not written again before
             // the store has read it: see tile_body)
             const int2 pend = s_pend;
@@ -2047,17 +2059,6 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == 4 ? 4 : 2)
                 tma::store_commit();
             }
             s_pend = make_int2(n0, m0);
-            // the next tile's box into the other buffer (last read by the
-            // previous tile, which every thread finished before the barriers
-            // above), then the counter's atomic for the tile after it, into
-            // this buffer's slots (every thread has read them)
-            int tnn = tiles;
-            if (s_tile[b ^ 1] < tiles) {
-                tma::mbar_expect(&bar[b ^ 1], kBoxBytes);
-                tma::load_3d(&tin, &sm.qb[b ^ 1][0][0][0], &bar[b ^ 1], s_org[b ^ 1].x - 4, s_org[b ^ 1].y - 2,
-                             0);
-                tnn = t_lo + (int)atomicAdd(&P.clock->next_tile, 1u);
-            }
             s_tile[b] = tnn;
             s_org[b] = make_int2((tnn % tiles_z) * TZ, (tnn / tiles_z) * TR);
         }
