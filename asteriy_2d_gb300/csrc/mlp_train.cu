@@ -1,13 +1,17 @@
 // mlp_train.cu - forward, backward and Adam kernels of the learned start
 // value (the network of mlp.cuh), and the C entry points that train it.
 //
-// Loss: mean squared error of y = log(p*/p_L) over a batch.  One thread
-// carries one sample through the forward and backward pass; the CTA then
-// reduces the per-sample weight gradients from shared memory (each weight
-// gradient is a sum over the CTA's samples of an outer-product term) and
-// adds its partial gradient to the global one with atomics.  The network is
-// too small (1313 weights) for tensor-core tiles to pay; everything is FP32
-// SIMT.
+// Loss: mean squared error of y = log(p*/p_L) over a batch.  A CTA takes 64
+// samples at a time, four threads a sample (eight units of each layer each),
+// and then reduces the per-sample weight gradients from shared memory (each
+// weight gradient is a sum over the samples of an outer-product term, four
+// W2 entries a thread); the sums of its samples go to the global gradient by
+// one atomic each.  The last CTA of a training batch takes the Adam step, so a
+// batch is one launch.  The network is too small (1313 weights) for
+// tensor-core tiles to pay; everything is FP32 SIMT.  A batch of 16384 is
+// bound by the latency of a CTA's phases: with one thread a sample, 256 samples
+// a CTA and the Adam step as a second launch it took 34 us on 64 SMs, as here
+// 21 us on all SMs.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -28,143 +32,195 @@ using namespace ast;
 
 namespace {
 
-constexpr int kB = 256;          // samples per CTA
+constexpr int kB = 64;           // samples of a CTA at a time
+constexpr int kG = 4;            // threads per sample
+constexpr int kT = kB * kG;
+constexpr int kBatchUnit = 256;  // ast_mlp_train's batches are multiples of this
 constexpr int kH = kMlpH, kI = kMlpIn;
-constexpr int kPad = kH + 1;     // row pitch of the per-sample activations (no bank conflicts)
+constexpr int kU = kH / kG;      // units of a thread in each layer
+constexpr int kPad = kH + 2;     // row pitch of the per-sample activations (pairs aligned)
+static_assert(kH * kH == 4 * kT, "four W2 entries a thread");
 
 struct GradSmem {
-    float W[kMlpParams];
-    float X[kB][kI];
-    float H1[kB][kPad];
-    float H2[kB][kPad];
-    float DZ1[kB][kPad];
-    float DZ2[kB][kPad];
+    alignas(16) float W[kMlpParams + 3];
+    float X[kB][kI + 1];
+    alignas(8) float H1[kB][kPad];
+    alignas(8) float H2[kB][kPad];
+    alignas(8) float DZ1[kB][kPad];
+    alignas(8) float DZ2[kB][kPad];
+    float Y[kG][kB];
     float DY[kB];
+    int last;
+};
+
+// the Adam step that ends a training batch (shift/scale are fixed): the
+// moments and the CTAs' ticket (null: no step)
+struct Adam {
+    float *m1, *m2;
+    unsigned* ticket;
+    float lr, b1, b2, eps, c1, c2;
 };
 
 // samples: n records of AST_RECORD_FLOATS (x[6], target, ...); idx: optional
 // permutation (sample i of this pass is samples[idx[i]]).  grad (1325 floats,
-// the shift/scale slots stay zero) and loss_sum are accumulated.
-__global__ void __launch_bounds__(kB) mlp_grad_kernel(const float* __restrict__ W_g, const float* __restrict__ samples,
+// the shift/scale slots stay zero) and loss_sum are accumulated; with Adam,
+// W_g is updated and grad zeroed.
+__global__ void __launch_bounds__(kT) mlp_grad_kernel(float* __restrict__ W_g, const float* __restrict__ samples,
                                                       const int* __restrict__ idx, long long first, long long count,
-                                                      float inv_count, float* __restrict__ grad, float* loss_sum)
+                                                      float inv_count, float* grad, float* loss_sum, Adam adam)
 {
-    extern __shared__ __align__(16) unsigned char raw[];
-    GradSmem& s = *reinterpret_cast<GradSmem*>(raw);
-    const int t = threadIdx.x;
-    for (int i = t; i < kMlpParams; i += kB) s.W[i] = W_g[i];
-    __syncthreads();
-
-    const long long gi = (long long)blockIdx.x * kB + t;
-    const bool valid = gi < count;
-    float x[kI], target = 0.0f;
-    if (valid) {
-        const long long k = idx ? (long long)idx[first + gi] : first + gi;
-        const float* r = samples + k * AST_RECORD_FLOATS;
+    __shared__ GradSmem s;
+    const int t = threadIdx.x, q = t % kB, j0 = t / kB * kU;   // a warp's threads: one group of units
+    for (int i = t; i < kMlpParams; i += kT) s.W[i] = W_g[i];
+    // this thread's gradient entries: W2[k0..k0+1][l0..l0+1], then the others in turn
+    const int k0 = t / (kH / 2) * 2, l0 = t % (kH / 2) * 2;
+    constexpr int kRest = kH * kI + 3 * kH + 1, kR = (kRest + kT - 1) / kT;
+    float g2[4] = {0.0f, 0.0f, 0.0f, 0.0f}, gr[kR];
 #pragma unroll
-        for (int i = 0; i < kI; i++) x[i] = (mlp_map(i, r[i]) - s.W[kOffShift + i]) * s.W[kOffScale + i];
-        target = r[6];
-    } else {
+    for (int r = 0; r < kR; r++) gr[r] = 0.0f;
+    float loss = 0.0f;
+    for (long long base = (long long)blockIdx.x * kB; base < count; base += (long long)gridDim.x * kB) {
+        __syncthreads();   // the weights; the last block's activations are read
+        const long long gi = base + q;
+        const bool valid = gi < count;
+        const float* rec = samples;
+        if (valid) rec += (idx ? (long long)idx[first + gi] : first + gi) * AST_RECORD_FLOATS;
+        for (int i = t / kB; i < kI; i += kG)
+            s.X[q][i] = valid ? (mlp_map(i, rec[i]) - s.W[kOffShift + i]) * s.W[kOffScale + i] : 0.0f;
+        __syncthreads();
+        // forward
+        float z1[kU], z2[kU];
 #pragma unroll
-        for (int i = 0; i < kI; i++) x[i] = 0.0f;
-    }
-    // forward
-    float z1[kH], h1[kH];
+        for (int u = 0; u < kU; u++) {
+            float z = s.W[kOffB1 + j0 + u];
 #pragma unroll
-    for (int j = 0; j < kH; j++) {
-        float z = s.W[kOffB1 + j];
-#pragma unroll
-        for (int i = 0; i < kI; i++) z = fmaf(s.W[kOffW1 + j * kI + i], x[i], z);
-        z1[j] = z;
-        h1[j] = silu(z);
-    }
-    float y = s.W[kOffB3];
-    float z2[kH];
-#pragma unroll 4
-    for (int k = 0; k < kH; k++) {
-        float z = s.W[kOffB2 + k];
-#pragma unroll
-        for (int j = 0; j < kH; j++) z = fmaf(s.W[kOffW2 + k * kH + j], h1[j], z);
-        z2[k] = z;
-        y = fmaf(s.W[kOffW3 + k], silu(z), y);
-    }
-    const float err = valid ? (y - target) : 0.0f;
-    const float dy = 2.0f * err * inv_count;
-    // backward through the output and the second layer
-    float dh1[kH];
-#pragma unroll
-    for (int j = 0; j < kH; j++) dh1[j] = 0.0f;
-#pragma unroll 4
-    for (int k = 0; k < kH; k++) {
-        const float h2 = silu(z2[k]);
-        const float dz2 = dy * s.W[kOffW3 + k] * silu_grad(z2[k]);
-        s.H2[t][k] = h2;
-        s.DZ2[t][k] = dz2;
-#pragma unroll
-        for (int j = 0; j < kH; j++) dh1[j] = fmaf(s.W[kOffW2 + k * kH + j], dz2, dh1[j]);
-    }
-#pragma unroll
-    for (int j = 0; j < kH; j++) {
-        s.H1[t][j] = h1[j];
-        s.DZ1[t][j] = dh1[j] * silu_grad(z1[j]);
-    }
-#pragma unroll
-    for (int i = 0; i < kI; i++) s.X[t][i] = x[i];
-    s.DY[t] = dy;
-    // loss
-    float l = err * err;
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if ((t & 31) == 0 && l != 0.0f) atomicAdd(loss_sum, l);
-    __syncthreads();
-
-    // CTA reduction over samples of the outer-product gradient terms
-    for (int o = t; o < kH * kH; o += kB) {           // W2[k][j]: sum_s dz2[s][k] h1[s][j]
-        const int k = o / kH, j = o - k * kH;
-        float acc = 0.0f;
-        for (int q = 0; q < kB; q++) acc = fmaf(s.DZ2[q][k], s.H1[q][j], acc);
-        if (acc != 0.0f) atomicAdd(&grad[kOffW2 + o], acc);
-    }
-    for (int o = t; o < kH * kI + 3 * kH + 1; o += kB) {
-        float acc = 0.0f;
-        int dst;
-        if (o < kH * kI) {                             // W1[j][i]: sum_s dz1[s][j] x[s][i]
-            const int j = o / kI, i = o - j * kI;
-            for (int q = 0; q < kB; q++) acc = fmaf(s.DZ1[q][j], s.X[q][i], acc);
-            dst = kOffW1 + o;
-        } else if (o < kH * kI + kH) {                 // b1[j]
-            const int j = o - kH * kI;
-            for (int q = 0; q < kB; q++) acc += s.DZ1[q][j];
-            dst = kOffB1 + j;
-        } else if (o < kH * kI + 2 * kH) {             // b2[k]
-            const int k = o - kH * kI - kH;
-            for (int q = 0; q < kB; q++) acc += s.DZ2[q][k];
-            dst = kOffB2 + k;
-        } else if (o < kH * kI + 3 * kH) {             // w3[k]: sum_s dy[s] h2[s][k]
-            const int k = o - kH * kI - 2 * kH;
-            for (int q = 0; q < kB; q++) acc = fmaf(s.DY[q], s.H2[q][k], acc);
-            dst = kOffW3 + k;
-        } else {                                       // b3
-            for (int q = 0; q < kB; q++) acc += s.DY[q];
-            dst = kOffB3;
+            for (int i = 0; i < kI; i++) z = fmaf(s.W[kOffW1 + (j0 + u) * kI + i], s.X[q][i], z);
+            z1[u] = z;
+            s.H1[q][j0 + u] = silu(z);
         }
-        if (acc != 0.0f) atomicAdd(&grad[dst], acc);
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < kU; u++) z2[u] = s.W[kOffB2 + j0 + u];
+#pragma unroll
+        for (int j = 0; j < kH; j += 4) {
+            const float2 ha = *reinterpret_cast<const float2*>(&s.H1[q][j]);
+            const float2 hb = *reinterpret_cast<const float2*>(&s.H1[q][j + 2]);
+#pragma unroll
+            for (int u = 0; u < kU; u++) {
+                const float4 w = *reinterpret_cast<const float4*>(&s.W[kOffW2 + (j0 + u) * kH + j]);
+                z2[u] = fmaf(w.w, hb.y, fmaf(w.z, hb.x, fmaf(w.y, ha.y, fmaf(w.x, ha.x, z2[u]))));
+            }
+        }
+        float y = 0.0f;
+#pragma unroll
+        for (int u = 0; u < kU; u++) {
+            const float h2 = silu(z2[u]);
+            s.H2[q][j0 + u] = h2;
+            y = fmaf(s.W[kOffW3 + j0 + u], h2, y);
+        }
+        s.Y[t / kB][q] = y;
+        __syncthreads();
+        // backward through the output and the second layer
+        y = s.W[kOffB3] + ((s.Y[0][q] + s.Y[1][q]) + (s.Y[2][q] + s.Y[3][q]));
+        const float err = valid ? y - rec[6] : 0.0f;
+        const float dy = 2.0f * err * inv_count;
+        if (t < kB) {
+            s.DY[q] = dy;
+            loss = fmaf(err, err, loss);
+        }
+#pragma unroll
+        for (int u = 0; u < kU; u++) s.DZ2[q][j0 + u] = dy * s.W[kOffW3 + j0 + u] * silu_grad(z2[u]);
+        __syncthreads();
+        float dh1[kU];
+#pragma unroll
+        for (int u = 0; u < kU; u++) dh1[u] = 0.0f;
+#pragma unroll 8
+        for (int k = 0; k < kH; k++) {
+            const float dz2 = s.DZ2[q][k];
+#pragma unroll
+            for (int u = 0; u < kU; u += 4) {
+                const float4 w = *reinterpret_cast<const float4*>(&s.W[kOffW2 + k * kH + j0 + u]);
+                dh1[u] = fmaf(w.x, dz2, dh1[u]);
+                dh1[u + 1] = fmaf(w.y, dz2, dh1[u + 1]);
+                dh1[u + 2] = fmaf(w.z, dz2, dh1[u + 2]);
+                dh1[u + 3] = fmaf(w.w, dz2, dh1[u + 3]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kU; u++) s.DZ1[q][j0 + u] = dh1[u] * silu_grad(z1[u]);
+        __syncthreads();
+        // the outer-product sums over the CTA's samples
+#pragma unroll 8
+        for (int n = 0; n < kB; n++) {             // W2[k][l]: sum_n dz2[n][k] h1[n][l]
+            const float2 d = *reinterpret_cast<const float2*>(&s.DZ2[n][k0]);
+            const float2 h = *reinterpret_cast<const float2*>(&s.H1[n][l0]);
+            g2[0] = fmaf(d.x, h.x, g2[0]);
+            g2[1] = fmaf(d.x, h.y, g2[1]);
+            g2[2] = fmaf(d.y, h.x, g2[2]);
+            g2[3] = fmaf(d.y, h.y, g2[3]);
+        }
+#pragma unroll
+        for (int r = 0; r < kR; r++) {
+            int o = t + r * kT;
+            float acc = 0.0f;
+            if (o < kH * kI) {                     // W1[j][i]: sum_n dz1[n][j] x[n][i]
+                const int j = o / kI, i = o - j * kI;
+#pragma unroll 8
+                for (int n = 0; n < kB; n++) acc = fmaf(s.DZ1[n][j], s.X[n][i], acc);
+            } else if ((o -= kH * kI) < kH) {      // b1[j]
+#pragma unroll 8
+                for (int n = 0; n < kB; n++) acc += s.DZ1[n][o];
+            } else if ((o -= kH) < kH) {           // b2[k]
+#pragma unroll 8
+                for (int n = 0; n < kB; n++) acc += s.DZ2[n][o];
+            } else if ((o -= kH) < kH) {           // w3[k]: sum_n dy[n] h2[n][k]
+#pragma unroll 8
+                for (int n = 0; n < kB; n++) acc = fmaf(s.DY[n], s.H2[n][o], acc);
+            } else if (o == kH) {                  // b3
+                for (int n = 0; n < kB; n++) acc += s.DY[n];
+            }
+            gr[r] += acc;
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+    if ((t & 31) == 0 && loss != 0.0f) atomicAdd(loss_sum, loss);
+    auto give = [&](int o, float v) {
+        if (v != 0.0f) atomicAdd(&grad[o], v);
+    };
+    give(kOffW2 + k0 * kH + l0, g2[0]);
+    give(kOffW2 + k0 * kH + l0 + 1, g2[1]);
+    give(kOffW2 + (k0 + 1) * kH + l0, g2[2]);
+    give(kOffW2 + (k0 + 1) * kH + l0 + 1, g2[3]);
+#pragma unroll
+    for (int r = 0; r < kR; r++) {
+        // W1 and b1 lie before W2, then b2, w3 and b3 after it
+        const int o = t + r * kT, lo = kH * kI + kH;
+        if (o < kRest) give(o < lo ? kOffW1 + o : kOffB2 + o - lo, gr[r]);
+    }
+    if (!adam.ticket) return;
+    // the CTA that gives last takes the step
+    __threadfence();
+    __syncthreads();
+    if (t == 0) s.last = atomicAdd(adam.ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s.last) return;
+    __threadfence();
+    if (t == 0) *adam.ticket = 0u;
+    for (int i = kOffW1 + t; i < kMlpParams; i += kT) {
+        const float g = __ldcg(&grad[i]);
+        grad[i] = 0.0f;
+        const float a = adam.b1 * adam.m1[i] + (1.0f - adam.b1) * g;
+        const float v = adam.b2 * adam.m2[i] + (1.0f - adam.b2) * g * g;
+        adam.m1[i] = a;
+        adam.m2[i] = v;
+        W_g[i] = s.W[i] - adam.lr * (a * adam.c1) / (sqrtf(v * adam.c2) + adam.eps);
     }
 }
+static_assert(kOffW1 + kH * kI == kOffB1 && kOffB1 + kH == kOffW2 && kOffB2 + kH == kOffW3 && kOffW3 + kH == kOffB3,
+              "the parameter block's order");
 
-// Adam step on the trainable slots (shift/scale are fixed); zeroes grad
-__global__ void adam_kernel(float* __restrict__ W, float* __restrict__ grad, float* __restrict__ m1,
-                            float* __restrict__ m2, float lr, float b1, float b2, float eps, float c1, float c2)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < kOffW1 || i >= kMlpParams) return;
-    const float gr = grad[i];
-    grad[i] = 0.0f;
-    const float a = b1 * m1[i] + (1.0f - b1) * gr;
-    const float v = b2 * m2[i] + (1.0f - b2) * gr * gr;
-    m1[i] = a;
-    m2[i] = v;
-    W[i] -= lr * (a * c1) / (sqrtf(v * c2) + eps);
-}
+// CTAs of a pass over count samples: at most two per SM of a GB300
+int grad_blocks(long long count) { return (int)std::min<long long>((count + kB - 1) / kB, 304); }
 
 __global__ void mlp_forward_kernel(const float* __restrict__ W_g, const float* __restrict__ x, long long n,
                                    int stride, float* __restrict__ y)
@@ -194,16 +250,6 @@ struct DevBuf {
         cudaError_t e_ = (call);                                    \
         if (e_ != cudaSuccess) return ast::cuda_fail(e_, #call);    \
     } while (0)
-
-int set_grad_smem()
-{
-    static bool done = false;
-    if (!done) {
-        TRY(cudaFuncSetAttribute(mlp_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GradSmem)));
-        done = true;
-    }
-    return AST_OK;
-}
 
 }  // namespace
 
@@ -250,8 +296,6 @@ int ast_mlp_init(const float* samples, int64_t n, uint64_t seed, float* params)
 int ast_mlp_grad(const float* params, const float* samples, int64_t n, float* grad, float* loss)
 {
     if (!params || !samples || !grad || n < 1) return AST_ERR_INVALID;
-    int rc = set_grad_smem();
-    if (rc != AST_OK) return rc;
     DevBuf dW, dS, dG, dL;
     TRY(dW.alloc(sizeof(float) * kMlpParams));
     TRY(dS.alloc(sizeof(float) * AST_RECORD_FLOATS * n));
@@ -261,9 +305,8 @@ int ast_mlp_grad(const float* params, const float* samples, int64_t n, float* gr
     TRY(cudaMemcpy(dS.p, samples, sizeof(float) * AST_RECORD_FLOATS * n, cudaMemcpyHostToDevice));
     TRY(cudaMemset(dG.p, 0, sizeof(float) * kMlpParams));
     TRY(cudaMemset(dL.p, 0, sizeof(float)));
-    const int blocks = (int)((n + kB - 1) / kB);
-    mlp_grad_kernel<<<blocks, kB, sizeof(GradSmem)>>>(dW.as<float>(), dS.as<float>(), nullptr, 0, n, 1.0f / (float)n,
-                                                       dG.as<float>(), dL.as<float>());
+    mlp_grad_kernel<<<grad_blocks(n), kT>>>(dW.as<float>(), dS.as<float>(), nullptr, 0, n, 1.0f / (float)n,
+                                            dG.as<float>(), dL.as<float>(), Adam{});
     TRY(cudaGetLastError());
     TRY(cudaMemcpy(grad, dG.p, sizeof(float) * kMlpParams, cudaMemcpyDeviceToHost));
     float l = 0.0f;
@@ -295,29 +338,34 @@ int ast_mlp_forward(const float* params, const float* x, int64_t n, int stride, 
 int ast_mlp_train(const float* samples, int64_t n, int epochs, int batch, float lr, uint64_t seed, float* params,
                   float* loss_per_epoch)
 {
-    if (!samples || !params || n < batch || epochs < 1 || batch < kB || batch % kB) return AST_ERR_INVALID;
-    int rc = set_grad_smem();
-    if (rc != AST_OK) return rc;
+    if (!samples || !params || n < batch || epochs < 1 || batch < kBatchUnit || batch % kBatchUnit)
+        return AST_ERR_INVALID;
     const int64_t nb = n / batch;
     std::vector<int> perm(n);
     for (int64_t i = 0; i < n; i++) perm[i] = (int)i;
     std::mt19937_64 gen(seed);
     std::shuffle(perm.begin(), perm.end(), gen);
-    DevBuf dW, dS, dG, dM1, dM2, dL, dI;
-    TRY(dW.alloc(sizeof(float) * kMlpParams));
-    TRY(dS.alloc(sizeof(float) * AST_RECORD_FLOATS * n));
-    TRY(dI.alloc(sizeof(int) * n));
-    TRY(dG.alloc(sizeof(float) * kMlpParams));
-    TRY(dM1.alloc(sizeof(float) * kMlpParams));
-    TRY(dM2.alloc(sizeof(float) * kMlpParams));
-    TRY(dL.alloc(sizeof(float) * epochs));
-    TRY(cudaMemcpy(dW.p, params, sizeof(float) * kMlpParams, cudaMemcpyHostToDevice));
-    TRY(cudaMemcpy(dS.p, samples, sizeof(float) * AST_RECORD_FLOATS * n, cudaMemcpyHostToDevice));
-    TRY(cudaMemcpy(dI.p, perm.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
-    TRY(cudaMemset(dG.p, 0, sizeof(float) * kMlpParams));
-    TRY(cudaMemset(dM1.p, 0, sizeof(float) * kMlpParams));
-    TRY(cudaMemset(dM2.p, 0, sizeof(float) * kMlpParams));
-    TRY(cudaMemset(dL.p, 0, sizeof(float) * epochs));
+    // one allocation (seven took some 200 us more): the samples and their
+    // order, the parameters, then what starts at zero (gradient, moments,
+    // losses, ticket)
+    auto pad = [](size_t b) { return (b + 255) / 256 * 256; };
+    const size_t bS = pad(sizeof(float) * AST_RECORD_FLOATS * n), bI = pad(sizeof(int) * n);
+    const size_t bW = pad(sizeof(float) * kMlpParams), bL = pad(sizeof(float) * epochs);
+    DevBuf buf;
+    TRY(buf.alloc(bS + bI + 4 * bW + bL + pad(sizeof(unsigned))));
+    char* at = buf.as<char>();
+    float* dS = (float*)at;
+    int* dI = (int*)(at += bS);
+    float* dW = (float*)(at += bI);
+    float* dG = (float*)(at += bW);
+    float* dM1 = (float*)(at += bW);
+    float* dM2 = (float*)(at += bW);
+    float* dL = (float*)(at += bW);
+    unsigned* ticket = (unsigned*)(at += bL);
+    TRY(cudaMemcpy(dW, params, sizeof(float) * kMlpParams, cudaMemcpyHostToDevice));
+    TRY(cudaMemcpy(dS, samples, sizeof(float) * AST_RECORD_FLOATS * n, cudaMemcpyHostToDevice));
+    TRY(cudaMemcpy(dI, perm.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
+    TRY(cudaMemset(dG, 0, 3 * bW + bL + sizeof(unsigned)));
     std::vector<int64_t> order(nb);
     const float b1 = 0.9f, b2 = 0.999f;
     long long t = 0;
@@ -325,20 +373,17 @@ int ast_mlp_train(const float* samples, int64_t n, int epochs, int batch, float 
         for (int64_t i = 0; i < nb; i++) order[i] = i;
         std::shuffle(order.begin(), order.end(), gen);
         for (int64_t bi = 0; bi < nb; bi++) {
-            mlp_grad_kernel<<<batch / kB, kB, sizeof(GradSmem)>>>(dW.as<float>(), dS.as<float>(), dI.as<int>(),
-                                                                  order[bi] * batch, batch, 1.0f / (float)batch,
-                                                                  dG.as<float>(), dL.as<float>() + e);
             t++;
             const float c1 = 1.0f / (1.0f - std::pow(b1, (float)t));
             const float c2 = 1.0f / (1.0f - std::pow(b2, (float)t));
-            adam_kernel<<<(kMlpParams + 255) / 256, 256>>>(dW.as<float>(), dG.as<float>(), dM1.as<float>(),
-                                                          dM2.as<float>(), lr, b1, b2, 1e-8f, c1, c2);
+            mlp_grad_kernel<<<grad_blocks(batch), kT>>>(dW, dS, dI, order[bi] * batch, batch, 1.0f / (float)batch, dG,
+                                                        dL + e, Adam{dM1, dM2, ticket, lr, b1, b2, 1e-8f, c1, c2});
         }
         TRY(cudaGetLastError());
     }
-    TRY(cudaMemcpy(params, dW.p, sizeof(float) * kMlpParams, cudaMemcpyDeviceToHost));
+    TRY(cudaMemcpy(params, dW, sizeof(float) * kMlpParams, cudaMemcpyDeviceToHost));
     if (loss_per_epoch) {
-        TRY(cudaMemcpy(loss_per_epoch, dL.p, sizeof(float) * epochs, cudaMemcpyDeviceToHost));
+        TRY(cudaMemcpy(loss_per_epoch, dL, sizeof(float) * epochs, cudaMemcpyDeviceToHost));
         for (int e = 0; e < epochs; e++) loss_per_epoch[e] /= (float)(nb * batch);
     }
     return AST_OK;
