@@ -11,7 +11,7 @@
 // tensor-core tiles to pay; everything is FP32 SIMT.  A batch of 16384 is
 // bound by the latency of a CTA's phases: with one thread a sample, 256 samples
 // a CTA and the Adam step as a second launch it took 34 us on 64 SMs, as here
-// 21 us on all SMs.
+// 12 us on all SMs.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -55,6 +55,11 @@ struct GradSmem {
 
 // the Adam step that ends a training batch (shift/scale are fixed): the
 // moments and the CTAs' ticket (null: no step)
+// The CTAs' atomics on one address follow one another at some 10 ns each, so
+// in training they are spread over kSums copies of the gradient, which the
+// step adds up: a batch of 16384 20 -> 12 us with it
+// and with every load of the step in flight at once.
+constexpr int kSums = 4, kSumPitch = (kMlpParams + 3) / 4 * 4;
 struct Adam {
     float *m1, *m2;
     unsigned* ticket;
@@ -63,15 +68,36 @@ struct Adam {
 
 // samples: n records of AST_RECORD_FLOATS (x[6], target, ...); idx: optional
 // permutation (sample i of this pass is samples[idx[i]]).  grad (1325 floats,
-// the shift/scale slots stay zero) and loss_sum are accumulated; with Adam,
-// W_g is updated and grad zeroed.
+// the shift/scale slots stay zero; with Adam kSums of them) and loss_sum are
+// accumulated; with Adam, W_g is updated and grad zeroed.  W_g and grad lie on
+// 16 bytes and W_g has kSumPitch floats.
 __global__ void __launch_bounds__(kT) mlp_grad_kernel(float* __restrict__ W_g, const float* __restrict__ samples,
                                                       const int* __restrict__ idx, long long first, long long count,
                                                       float inv_count, float* grad, float* loss_sum, Adam adam)
 {
     __shared__ GradSmem s;
     const int t = threadIdx.x, q = t % kB, j0 = t / kB * kU;   // a warp's threads: one group of units
-    for (int i = t; i < kMlpParams; i += kT) s.W[i] = W_g[i];
+    // the mapped inputs of sample base + q; its target
+    auto features = [&](long long base) {
+        const bool valid = base + q < count;
+        const float* rec = samples;
+        if (valid) rec += (idx ? (long long)idx[first + base + q] : first + base + q) * AST_RECORD_FLOATS;
+        for (int i = t / kB; i < kI; i += kG)
+            s.X[q][i] = valid ? (mlp_map(i, rec[i]) - __ldcg(&W_g[kOffShift + i])) * __ldcg(&W_g[kOffScale + i]) : 0.0f;
+        return valid ? rec[6] : 0.0f;
+    };
+    // In training a launch may begin while the batch before it still runs:
+    // up to the wait it reads only what no launch writes (the samples and
+    // their order, shift and scale) and writes only shared memory.  The
+    // weights are read past L1, where the early reads may have left old ones.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const long long base0 = (long long)blockIdx.x * kB;
+    float target = features(base0);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+#pragma unroll
+    for (int r = 0; r < kSumPitch / 4; r += kT)
+        if (r + t < kSumPitch / 4)
+            reinterpret_cast<float4*>(s.W)[r + t] = __ldcg(reinterpret_cast<const float4*>(W_g) + r + t);
     // this thread's gradient entries: W2[k0..k0+1][l0..l0+1], then the others in turn
     const int k0 = t / (kH / 2) * 2, l0 = t % (kH / 2) * 2;
     constexpr int kRest = kH * kI + 3 * kH + 1, kR = (kRest + kT - 1) / kT;
@@ -79,15 +105,13 @@ __global__ void __launch_bounds__(kT) mlp_grad_kernel(float* __restrict__ W_g, c
 #pragma unroll
     for (int r = 0; r < kR; r++) gr[r] = 0.0f;
     float loss = 0.0f;
-    for (long long base = (long long)blockIdx.x * kB; base < count; base += (long long)gridDim.x * kB) {
-        __syncthreads();   // the weights; the last block's activations are read
-        const long long gi = base + q;
-        const bool valid = gi < count;
-        const float* rec = samples;
-        if (valid) rec += (idx ? (long long)idx[first + gi] : first + gi) * AST_RECORD_FLOATS;
-        for (int i = t / kB; i < kI; i += kG)
-            s.X[q][i] = valid ? (mlp_map(i, rec[i]) - s.W[kOffShift + i]) * s.W[kOffScale + i] : 0.0f;
+    for (long long base = base0; base < count; base += (long long)gridDim.x * kB) {
+        if (base != base0) {
+            __syncthreads();   // the last block's activations are read
+            target = features(base);
+        }
         __syncthreads();
+        const bool valid = base + q < count;
         // forward
         float z1[kU], z2[kU];
 #pragma unroll
@@ -122,7 +146,7 @@ __global__ void __launch_bounds__(kT) mlp_grad_kernel(float* __restrict__ W_g, c
         __syncthreads();
         // backward through the output and the second layer
         y = s.W[kOffB3] + ((s.Y[0][q] + s.Y[1][q]) + (s.Y[2][q] + s.Y[3][q]));
-        const float err = valid ? y - rec[6] : 0.0f;
+        const float err = valid ? y - target : 0.0f;
         const float dy = 2.0f * err * inv_count;
         if (t < kB) {
             s.DY[q] = dy;
@@ -184,18 +208,14 @@ __global__ void __launch_bounds__(kT) mlp_grad_kernel(float* __restrict__ W_g, c
     }
     for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
     if ((t & 31) == 0 && loss != 0.0f) atomicAdd(loss_sum, loss);
-    auto give = [&](int o, float v) {
-        if (v != 0.0f) atomicAdd(&grad[o], v);
-    };
-    give(kOffW2 + k0 * kH + l0, g2[0]);
-    give(kOffW2 + k0 * kH + l0 + 1, g2[1]);
-    give(kOffW2 + (k0 + 1) * kH + l0, g2[2]);
-    give(kOffW2 + (k0 + 1) * kH + l0 + 1, g2[3]);
+    if (adam.ticket) grad += blockIdx.x % kSums * kSumPitch;
+    atomicAdd(reinterpret_cast<float2*>(&grad[kOffW2 + k0 * kH + l0]), make_float2(g2[0], g2[1]));
+    atomicAdd(reinterpret_cast<float2*>(&grad[kOffW2 + (k0 + 1) * kH + l0]), make_float2(g2[2], g2[3]));
 #pragma unroll
     for (int r = 0; r < kR; r++) {
         // W1 and b1 lie before W2, then b2, w3 and b3 after it
         const int o = t + r * kT, lo = kH * kI + kH;
-        if (o < kRest) give(o < lo ? kOffW1 + o : kOffB2 + o - lo, gr[r]);
+        if (o < kRest) atomicAdd(&grad[o < lo ? kOffW1 + o : kOffB2 + o - lo], gr[r]);
     }
     if (!adam.ticket) return;
     // the CTA that gives last takes the step
@@ -206,17 +226,33 @@ __global__ void __launch_bounds__(kT) mlp_grad_kernel(float* __restrict__ W_g, c
     if (!s.last) return;
     __threadfence();
     if (t == 0) *adam.ticket = 0u;
-    for (int i = kOffW1 + t; i < kMlpParams; i += kT) {
-        const float g = __ldcg(&grad[i]);
-        grad[i] = 0.0f;
-        const float a = adam.b1 * adam.m1[i] + (1.0f - adam.b1) * g;
-        const float v = adam.b2 * adam.m2[i] + (1.0f - adam.b2) * g * g;
-        adam.m1[i] = a;
-        adam.m2[i] = v;
-        W_g[i] = s.W[i] - adam.lr * (a * adam.c1) / (sqrtf(v * adam.c2) + adam.eps);
+    grad -= blockIdx.x % kSums * kSumPitch;
+    constexpr int kP = (kMlpParams - kOffW1 + kT - 1) / kT;
+    float g[kP], a[kP], v[kP];
+#pragma unroll
+    for (int r = 0; r < kP; r++) {     // every load in flight before the first is used
+        const int i = kOffW1 + t + r * kT;
+        if (i >= kMlpParams) continue;
+        g[r] = 0.0f;
+#pragma unroll
+        for (int c = 0; c < kSums; c++) g[r] += __ldcg(&grad[c * kSumPitch + i]);
+        a[r] = __ldcg(&adam.m1[i]);
+        v[r] = __ldcg(&adam.m2[i]);
+    }
+#pragma unroll
+    for (int r = 0; r < kP; r++) {
+        const int i = kOffW1 + t + r * kT;
+        if (i >= kMlpParams) continue;
+#pragma unroll
+        for (int c = 0; c < kSums; c++) grad[c * kSumPitch + i] = 0.0f;
+        a[r] = adam.b1 * a[r] + (1.0f - adam.b1) * g[r];
+        v[r] = adam.b2 * v[r] + (1.0f - adam.b2) * g[r] * g[r];
+        adam.m1[i] = a[r];
+        adam.m2[i] = v[r];
+        W_g[i] = s.W[i] - adam.lr * (a[r] * adam.c1) / (sqrtf(v[r] * adam.c2) + adam.eps);
     }
 }
-static_assert(kOffW1 + kH * kI == kOffB1 && kOffB1 + kH == kOffW2 && kOffB2 + kH == kOffW3 && kOffW3 + kH == kOffB3,
+static_assert(kOffW1 + kH * kI == kOffB1 && kOffB1 + kH == kOffW2 && kOffB2 + kH == kOffW3 && kOffW3 + kH == kOffB3 && kOffW2 % 2 == 0,
               "the parameter block's order");
 
 // CTAs of a pass over count samples: at most two per SM of a GB300
@@ -297,7 +333,7 @@ int ast_mlp_grad(const float* params, const float* samples, int64_t n, float* gr
 {
     if (!params || !samples || !grad || n < 1) return AST_ERR_INVALID;
     DevBuf dW, dS, dG, dL;
-    TRY(dW.alloc(sizeof(float) * kMlpParams));
+    TRY(dW.alloc(sizeof(float) * kSumPitch));
     TRY(dS.alloc(sizeof(float) * AST_RECORD_FLOATS * n));
     TRY(dG.alloc(sizeof(float) * kMlpParams));
     TRY(dL.alloc(sizeof(float)));
@@ -350,22 +386,22 @@ int ast_mlp_train(const float* samples, int64_t n, int epochs, int batch, float 
     // losses, ticket)
     auto pad = [](size_t b) { return (b + 255) / 256 * 256; };
     const size_t bS = pad(sizeof(float) * AST_RECORD_FLOATS * n), bI = pad(sizeof(int) * n);
-    const size_t bW = pad(sizeof(float) * kMlpParams), bL = pad(sizeof(float) * epochs);
+    const size_t bW = pad(sizeof(float) * kSumPitch), bL = pad(sizeof(float) * epochs);
     DevBuf buf;
-    TRY(buf.alloc(bS + bI + 4 * bW + bL + pad(sizeof(unsigned))));
+    TRY(buf.alloc(bS + bI + (3 + kSums) * bW + bL + pad(sizeof(unsigned))));
     char* at = buf.as<char>();
     float* dS = (float*)at;
     int* dI = (int*)(at += bS);
     float* dW = (float*)(at += bI);
     float* dG = (float*)(at += bW);
-    float* dM1 = (float*)(at += bW);
+    float* dM1 = (float*)(at += kSums * bW);
     float* dM2 = (float*)(at += bW);
     float* dL = (float*)(at += bW);
     unsigned* ticket = (unsigned*)(at += bL);
     TRY(cudaMemcpy(dW, params, sizeof(float) * kMlpParams, cudaMemcpyHostToDevice));
     TRY(cudaMemcpy(dS, samples, sizeof(float) * AST_RECORD_FLOATS * n, cudaMemcpyHostToDevice));
     TRY(cudaMemcpy(dI, perm.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
-    TRY(cudaMemset(dG, 0, 3 * bW + bL + sizeof(unsigned)));
+    TRY(cudaMemset(dG, 0, (2 + kSums) * bW + bL + sizeof(unsigned)));
     std::vector<int64_t> order(nb);
     const float b1 = 0.9f, b2 = 0.999f;
     long long t = 0;
@@ -376,10 +412,18 @@ int ast_mlp_train(const float* samples, int64_t n, int epochs, int batch, float 
             t++;
             const float c1 = 1.0f / (1.0f - std::pow(b1, (float)t));
             const float c2 = 1.0f / (1.0f - std::pow(b2, (float)t));
-            mlp_grad_kernel<<<grad_blocks(batch), kT>>>(dW, dS, dI, order[bi] * batch, batch, 1.0f / (float)batch, dG,
-                                                        dL + e, Adam{dM1, dM2, ticket, lr, b1, b2, 1e-8f, c1, c2});
+            cudaLaunchConfig_t lc{};
+            lc.gridDim = grad_blocks(batch);
+            lc.blockDim = kT;
+            cudaLaunchAttribute early{};
+            early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            early.val.programmaticStreamSerializationAllowed = 1;
+            lc.attrs = &early;
+            lc.numAttrs = t > 1;   // the first one waits for the copies above
+            TRY(cudaLaunchKernelEx(&lc, mlp_grad_kernel, dW, (const float*)dS, (const int*)dI,
+                                   (long long)(order[bi] * batch), (long long)batch, 1.0f / (float)batch, dG, dL + e,
+                                   Adam{dM1, dM2, ticket, lr, b1, b2, 1e-8f, c1, c2}));
         }
-        TRY(cudaGetLastError());
     }
     TRY(cudaMemcpy(params, dW, sizeof(float) * kMlpParams, cudaMemcpyDeviceToHost));
     if (loss_per_epoch) {
