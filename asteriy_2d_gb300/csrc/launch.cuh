@@ -48,6 +48,34 @@ inline int sm_count()
     return v;
 }
 
+// early: the kernel may start while the one before it in the stream still runs:
+// its CTAs take free places on the SMs, do what needs none of its results and
+// wait (after_previous_step).  That saves the launch, but the CTAs are placed
+// around the last step's.  So it is for persistent kernels with more tiles than
+// CTAs, which fill every place all the same (FP32 HLLC wind 1537x771 41.2 ->
+// 36.9 us per step with the CTA's own first tile, HLL blast 4096x2048 75.5 ->
+// 73.8), and for grids (start_early) of many CTAs a place (FP64 exact solver
+// 1021x509 178 -> 173 us) or so few that each has an SM of its own (FP64 HLL
+// 64x32, 10 steps and the copies, 256 -> 236 us).  In between two CTAs shared an
+// SM while others stood empty: FP64 HLL 256x128 (128 CTAs) 23.0 -> 32.3 us per
+// step.  Not for the batch kernels: no gain over a batch's many tiles.
+inline bool start_early(long long ctas) { return 2 * ctas <= sm_count() || ctas >= 8 * sm_count(); }
+template <typename... P, typename... A>
+cudaError_t launch_after(bool early, void (*k)(P...), dim3 grid, size_t smem, cudaStream_t st, const A&... args)
+{
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = grid;
+    lc.blockDim = kThreads;
+    lc.dynamicSmemBytes = smem;
+    lc.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = &at;
+    lc.numAttrs = early ? 1 : 0;
+    return cudaLaunchKernelEx(&lc, k, args...);
+}
+
 // launch=false only raises the kernel's dynamic shared-memory limit, which
 // must happen outside stream capture (ast_create, ast_step_raw).  The FP64
 // solver on a small grid (fewer 32x16 tiles than two per SM) steps with
@@ -86,16 +114,14 @@ int launch_step_t(const StepParams& P, cudaStream_t st, bool launch)
         if (tiles < (FLUX == 2 ? 8LL : 2LL) * sm_count()) {
             dim3 grid((P.N + kSZ - 1) / kSZ, band);
             if (P.band_hi > 0) Q.units = (int)grid.x * rows;
-            step_kernel<R, FLUX, RECON, LAYOUT, kSZ, kSR>
-                <<<grid, kThreads, tile_smem_bytes<R, FLUX, kSZ, kSR>(), st>>>(Q);
-            e = cudaGetLastError();
+            e = launch_after(start_early((long long)grid.x * grid.y), step_kernel<R, FLUX, RECON, LAYOUT, kSZ, kSR>, grid,
+                             tile_smem_bytes<R, FLUX, kSZ, kSR>(), st, Q);
             return e == cudaSuccess ? AST_OK : cuda_fail(e, "step kernel launch");
         }
     }
     dim3 grid((P.N + kTZ - 1) / kTZ, band);
     if (P.band_hi > 0) Q.units = (int)grid.x * rows;
-    k<<<grid, kThreads, smem, st>>>(Q);
-    e = cudaGetLastError();
+    e = launch_after(start_early((long long)grid.x * grid.y), k, grid, smem, st, Q);
     return e == cudaSuccess ? AST_OK : cuda_fail(e, "step kernel launch");
 }
 
@@ -115,8 +141,8 @@ int launch_tma_t(const StepParams& P, const CUtensorMap& tin, const CUtensorMap&
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k, kThreads, smem);
         return e == cudaSuccess ? AST_OK : cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
     }
-    k<<<grid, kThreads, smem, st>>>(P, tin, tout);
-    e = cudaGetLastError();
+    const long long tiles = (long long)((P.N + kTmaTZ - 1) / kTmaTZ) * ((P.M + kTmaTR - 1) / kTmaTR);
+    e = launch_after(tiles > grid || 2 * grid <= sm_count(), k, grid, smem, st, P, tin, tout);
     return e == cudaSuccess ? AST_OK : cuda_fail(e, "persistent step kernel launch");
 }
 

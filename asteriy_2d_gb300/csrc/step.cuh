@@ -1734,7 +1734,7 @@ __device__ __forceinline__ void cta_epilogue(const StepParams& P, TileAcc<R>& ac
 {
     __shared__ R red_r[2][kThreads / 32];
     __shared__ int red_i[4][kThreads / 32];
-    __shared__ int s_last;
+    bool last = false;   // in thread 0
     const int tid = threadIdx.x;
     const int lane = tid & 31, wid = tid >> 5;
     RiemannCount& rc = acc.rc;
@@ -1789,7 +1789,7 @@ __device__ __forceinline__ void cta_epilogue(const StepParams& P, TileAcc<R>& ac
             if (st) atomicOr(&C->status, st);
             __threadfence();
             const unsigned int ticket = atomicAdd(&C->done, weight);
-            s_last = (ticket + weight == units) ? 1 : 0;
+            last = ticket + weight == units;
         } else {
             // raw mode: this CTA's dt candidate, min-reduced into *T_min
             double dt = P.dt_cap;
@@ -1797,11 +1797,9 @@ __device__ __forceinline__ void cta_epilogue(const StepParams& P, TileAcc<R>& ac
             if (b > 0.0) dt = fmin(dt, P.krit_dy / b);
             atomicMin((unsigned long long*)P.T_min, (unsigned long long)__double_as_longlong(dt));
             if (st && P.status_ptr) atomicOr(P.status_ptr, st);
-            s_last = 0;
         }
     }
-    __syncthreads();
-    if (s_last && tid == 0) {
+    if (last) {
         // funk_time (kernel.cu:1525-1536): T_do <- min dt, TT += T_do, i++
         __threadfence();
         DevClock* C = P.clock;
@@ -1816,8 +1814,16 @@ __device__ __forceinline__ void cta_epilogue(const StepParams& P, TileAcc<R>& ac
         C->step = C->step + 1;
         C->done = 0u;
         if (reset_tiles) C->next_tile = 0u;
-        __threadfence();
     }
+}
+
+// The start of a step's kernel that may have been launched while the step
+// before it still runs (launch_after): nothing that a kernel writes is touched
+// before it.  The step after this one may take its CTAs' places as they leave.
+__device__ __forceinline__ void after_previous_step()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // Tile (bx, by) of the problem P; `tiles` is the number of tiles of that
@@ -1863,6 +1869,7 @@ constexpr int min_ctas() { return sizeof(R) == 8 ? 2 : 4; }
 template <typename R, int FLUX, bool RECON, int LAYOUT, int TZ, int TR>
 __global__ void __launch_bounds__(kThreads, min_ctas<R, FLUX>()) step_kernel(const __grid_constant__ StepParams P)
 {
+    after_previous_step();
     step_tile<R, FLUX, RECON, LAYOUT, TZ, TR>(P, blockIdx.x, blockIdx.y + P.band_lo,
                                               P.units > 0 ? (unsigned)P.units : gridDim.x * gridDim.y);
 }
@@ -1935,7 +1942,8 @@ __global__ void __launch_bounds__(kThreads, min_ctas<R, 2>())
 }
 
 // The FP32 solver's persistent kernel: as many CTAs as fit on the GPU at
-// once, each taking tiles from a counter in the clock until none are left.
+// once, each taking its own tile and then tiles from a counter in the clock
+// until none are left.
 // A tile and its halo arrive by one bulk-tensor copy of the box (x = z
 // cells n0-4 .. n0+TZ+3, y = rows m0-2 .. m0+TR+1, all four planes) into
 // one of two buffers; the copy of the CTA's next tile runs while the current
@@ -1970,26 +1978,26 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == 4 ? 4 : 2)
     const int tiles_z = (P.N + TZ - 1) / TZ;
     const int t_lo = P.band_lo * tiles_z;   // this launch's tiles: t_lo <= t < tiles
     const int tiles = tiles_z * (P.band_hi > 0 ? P.band_hi : (P.M + TR - 1) / TR);
+    const int t_more = t_lo + (int)gridDim.x;   // the counter's tiles: those after every CTA's first
     if (copier) {
         tma::prefetch_map(&tin);
         tma::prefetch_map(&tout);
         tma::mbar_init(&bar[0], 1);
         tma::mbar_init(&bar[1], 1);
         tma::fence_async_shared();
-        step_consts<R>(P, sK);
         s_late = 0;
         sm.uni_known = 0;
         sm.uni_max[0] = sm.uni_max[1] = R(0);
         sm.uni_out[0] = sm.uni_out[1] = -2;
         s_pend = make_int2(-1, -1);
         sm.qn = 0u;   // later tiles: reset after the previous tile's queue
-        // the first two tiles: the first is copied now, the second at the
-        // start of the first tile's face pass
-        const int t0 = t_lo + (int)atomicAdd(&P.clock->next_tile, 1u);
-        const int t1 = (t0 < tiles) ? t_lo + (int)atomicAdd(&P.clock->next_tile, 1u) : tiles;
+    }
+    after_previous_step();
+    if (copier) {
+        // the CTA's own tile is copied now, the next at the start of this
+        // one's face pass
+        const int t0 = t_lo + (int)blockIdx.x;
         s_tile[0] = t0;
-        s_tile[1] = t1;
-        s_org[1] = make_int2((t1 % tiles_z) * TZ, (t1 / tiles_z) * TR);
         if (t0 < tiles) {
             s_org[0] = make_int2((t0 % tiles_z) * TZ, (t0 / tiles_z) * TR);
             tma::mbar_expect(&bar[0], kBoxBytes);
@@ -1997,6 +2005,14 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == 4 ? 4 : 2)
         }
     }
     __syncthreads();
+    if (copier) {
+        // while the copy runs (ordered before their use by the barrier after
+        // its arrival): the next tile's number, the step's constants
+        const int t1 = (s_tile[0] < tiles) ? t_more + (int)atomicAdd(&P.clock->next_tile, 1u) : tiles;
+        step_consts<R>(P, sK);
+        s_tile[1] = t1;
+        s_org[1] = make_int2((t1 % tiles_z) * TZ, (t1 / tiles_z) * TR);
+    }
     phase_mark(kPhaseStart);
     TileAcc<R> acc;
     acc.clear();
@@ -2049,7 +2065,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(R) == 4 ? 4 : 2)
                 tma::mbar_expect(&bar[b ^ 1], kBoxBytes);
                 tma::load_3d(&tin, &sm.qb[b ^ 1][0][0][0], &bar[b ^ 1], s_org[b ^ 1].x - 4, s_org[b ^ 1].y - 2,
                              0);
-                tnn = t_lo + (int)atomicAdd(&P.clock->next_tile, 1u);
+                tnn = t_more + (int)atomicAdd(&P.clock->next_tile, 1u);
             }
             // the previous tile's cells (sm.out is not written again before
             // the store has read it: see tile_body)
