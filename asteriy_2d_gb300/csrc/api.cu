@@ -105,7 +105,6 @@ struct ast_solver {
     StepParams P;
     cudaStream_t stream = nullptr;
     size_t elem = 8;                 // bytes per state value
-    int kflux = 0;                   // the kernels' FLUX
     long long ld = 0, plane = 0;
     void* buf[2] = {nullptr, nullptr};
     int cur = 0;
@@ -166,7 +165,6 @@ int ast_create(const ast_config* cfg, ast_solver** out)
     if (!S) return fail(AST_ERR_NOMEM, "host allocation");
     S->cfg = *cfg;
     S->elem = (cfg->precision == AST_PREC_FP32) ? 4 : 8;
-    S->kflux = kernel_flux(*cfg);
     // rows padded to 128 bytes: aligned, coalesced row starts
     const long long align = 128 / (long long)S->elem;
     S->ld = ((long long)cfg->N + align - 1) / align * align;
@@ -195,8 +193,8 @@ int ast_create(const ast_config* cfg, ast_solver** out)
         ast_destroy(S);
         return cuda_fail(e, "cudaMemcpy clock");
     }
-    rc = (S->elem == 8) ? launch_step_r<double, kSoA>(S->P, S->kflux, cfg->recon, nullptr, false)
-                        : launch_step_r<float, kSoA>(S->P, S->kflux, cfg->recon, nullptr, false);
+    rc = (S->elem == 8) ? launch_step_r<double, kSoA>(S->P, cfg->flux, cfg->recon, nullptr, false)
+                        : launch_step_r<float, kSoA>(S->P, cfg->flux, cfg->recon, nullptr, false);
     // FP32: the strip kernel (persistent = 2) or the persistent tile kernel (1)
     const bool want_sweep = S->elem == 4 && cfg->persistent == 2;
     if (rc == AST_OK && want_sweep) {
@@ -223,7 +221,7 @@ int ast_create(const ast_config* cfg, ast_solver** out)
         }
         int per_sm = 0, dev = 0, sms = 0;
         if (rc == AST_OK)
-            rc = launch_step_tma_e(S->elem, S->P, S->tin[0], S->tout[1], S->kflux, cfg->recon, 0, nullptr, false,
+            rc = launch_step_tma_e(S->elem, S->P, S->tin[0], S->tout[1], cfg->flux, cfg->recon, 0, nullptr, false,
                                    &per_sm);
         if (rc == AST_OK && (e = cudaGetDevice(&dev)) != cudaSuccess) rc = cuda_fail(e, "cudaGetDevice");
         if (rc == AST_OK && (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
@@ -463,11 +461,11 @@ static int enqueue_one(ast_solver* S)
     if (S->sweep)
         rc = launch_step_sweep(P, S->cfg.flux, S->cfg.recon, S->sweep_grid, S->stream, true, nullptr);
     else if (S->tma)
-        rc = launch_step_tma_e(S->elem, P, S->tin[S->cur], S->tout[S->cur ^ 1], S->kflux, S->cfg.recon,
+        rc = launch_step_tma_e(S->elem, P, S->tin[S->cur], S->tout[S->cur ^ 1], S->cfg.flux, S->cfg.recon,
                                S->tma_grid, S->stream, true, nullptr);
     else
-        rc = (S->elem == 8) ? launch_step_r<double, kSoA>(P, S->kflux, S->cfg.recon, S->stream, true)
-                            : launch_step_r<float, kSoA>(P, S->kflux, S->cfg.recon, S->stream, true);
+        rc = (S->elem == 8) ? launch_step_r<double, kSoA>(P, S->cfg.flux, S->cfg.recon, S->stream, true)
+                            : launch_step_r<float, kSoA>(P, S->cfg.flux, S->cfg.recon, S->stream, true);
     if (rc == AST_OK && S->elem == 4 && P.nsrc) {
         // the FP32 form's neutral-coupling source, after the step
         const long long K = (long long)S->cfg.N * S->cfg.M;
@@ -683,11 +681,11 @@ static int host_steps(ast_solver* S, int nsteps, double* s_a, double* u_a, doubl
                 // each band hands out its tiles from a counter set to zero
                 P.units = units;
                 if (b > 0) AST_CUDA(cudaMemsetAsync(&S->clock->next_tile, 0, sizeof(unsigned int), cst));
-                rc = launch_step_tma_e(S->elem, P, S->tin[S->cur], S->tout[S->cur ^ 1], S->kflux, S->cfg.recon,
+                rc = launch_step_tma_e(S->elem, P, S->tin[S->cur], S->tout[S->cur ^ 1], S->cfg.flux, S->cfg.recon,
                                        std::min((bd[b].t1 - bd[b].t0) * tiles_z, S->tma_grid), cst, true, nullptr);
             } else {
-                rc = (S->elem == 8) ? launch_step_r<double, kSoA>(P, S->kflux, S->cfg.recon, cst, true)
-                                    : launch_step_r<float, kSoA>(P, S->kflux, S->cfg.recon, cst, true);
+                rc = (S->elem == 8) ? launch_step_r<double, kSoA>(P, S->cfg.flux, S->cfg.recon, cst, true)
+                                    : launch_step_r<float, kSoA>(P, S->cfg.flux, S->cfg.recon, cst, true);
             }
             if (rc != AST_OK) break;
             const int nb = (int)((bd[b].k1 - bd[b].k0 + 255) / 256);

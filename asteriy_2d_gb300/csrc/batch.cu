@@ -41,7 +41,6 @@ static_assert(kNumSchedules == AST_BATCH_SCHEDULES, "schedule count");
 
 struct BatchClass {
     int flux, recon;
-    int kflux;                    // the kernels' FLUX
     int first, count;             // slots [first, first + count) of the parameter arrays
     int shape;                    // schedule in use
     int tiles[kNumSchedules];     // work-list length per schedule
@@ -148,15 +147,7 @@ int launch_problem(ast_batch* B, const BatchClass& c, int s, cudaStream_t st)
 {
     const size_t n = (size_t)B->nprob;
     return launch_step_tma(B->hPp[B->cur][s], B->hmaps[(2 * B->cur) * n + s], B->hmaps[(2 * B->cur + 1) * n + s],
-                           c.kflux, c.recon, B->pgrid[s], st, true, nullptr);
-}
-
-// the kernels' FLUX of the problem in slot s: its class's
-int slot_kflux(const ast_batch* B, int s)
-{
-    for (const BatchClass& k : B->cls)
-        if (s >= k.first && s < k.first + k.count) return k.kflux;
-    return 0;
+                           c.flux, c.recon, B->pgrid[s], st, true, nullptr);
 }
 
 int launch_class(ast_batch* B, BatchClass& c, int shape, cudaStream_t st, bool launch)
@@ -168,7 +159,7 @@ int launch_class(ast_batch* B, BatchClass& c, int shape, cudaStream_t st, bool l
             // the kernel's shared-memory limit, and each problem's CTAs
             int per_sm = 0, dev = 0, sms = 0;
             const size_t n = (size_t)B->nprob;
-            int rc = launch_step_tma(B->hPp[0][c.first], B->hmaps[c.first], B->hmaps[n + c.first], c.kflux, c.recon, 0,
+            int rc = launch_step_tma(B->hPp[0][c.first], B->hmaps[c.first], B->hmaps[n + c.first], c.flux, c.recon, 0,
                                      st, false, &per_sm);
             if (rc != AST_OK) return rc;
             BATCH_CUDA(cudaGetDevice(&dev));
@@ -199,7 +190,7 @@ int launch_class(ast_batch* B, BatchClass& c, int shape, cudaStream_t st, bool l
         const CUtensorMap* tout = B->maps + (size_t)(2 * B->cur + 1) * B->nprob;
         if (!launch) {
             int per_sm = 0, dev = 0, sms = 0;
-            int rc = launch_batch_tma(nullptr, nullptr, nullptr, nullptr, 0, 0, 0, nullptr, 0, c.kflux, c.recon, 0,
+            int rc = launch_batch_tma(nullptr, nullptr, nullptr, nullptr, 0, 0, 0, nullptr, 0, c.flux, c.recon, 0,
                                       st, false, &per_sm);
             if (rc != AST_OK) return rc;
             BATCH_CUDA(cudaGetDevice(&dev));
@@ -208,9 +199,9 @@ int launch_class(ast_batch* B, BatchClass& c, int shape, cudaStream_t st, bool l
             return AST_OK;
         }
         return launch_batch_tma(B->dP[B->cur], tin, tout, B->work + c.work0, c.tiles[shape], c.first, c.count,
-                                B->counters + 2 * ci, B->wait_polls, c.kflux, c.recon, c.grid, st, true, nullptr);
+                                B->counters + 2 * ci, B->wait_polls, c.flux, c.recon, c.grid, st, true, nullptr);
     }
-    return launch_batch(B->elem, shape, Ps, ts, c.count, c.tiles[shape], c.kflux, c.recon, st, launch);
+    return launch_batch(B->elem, shape, Ps, ts, c.count, c.tiles[shape], c.flux, c.recon, st, launch);
 }
 
 // `count` steps of every class; classes beyond the first run on their own
@@ -373,14 +364,10 @@ int ast_batch_create(const ast_config* cfgs, int nprob, ast_batch** out)
             BatchClass k;
             std::memset(&k, 0, sizeof k);
             k.flux = c.flux;
-            k.kflux = kernel_flux(c);
             k.recon = c.recon;
             k.first = s;
             B->cls.push_back(k);
         }
-        // one problem with the learned start value: its whole class steps with
-        // the kernel that has it
-        if (kernel_flux(c) != kExactInline) B->cls.back().kflux = c.flux;
         B->cls.back().count++;
         B->slot[order[s]] = s;
     }
@@ -459,7 +446,8 @@ int ast_batch_create(const ast_config* cfgs, int nprob, ast_batch** out)
             k.work0 = (int)work.size();
             for (int s = k.first; s < k.first + k.count; s++) {
                 const ast_config& c = B->cfg[order[s]];
-                const int fk = slot_kflux(B, s);
+                const int fk = (c.flux == AST_FLUX_HLL) ? 0 : (c.flux == AST_FLUX_HLLC) ? 1
+                                                          : (c.flux == AST_FLUX_HLLC_A) ? 3 : 2;
                 const int tz = (c.N + kTmaTZ - 1) / kTmaTZ;
                 const int nt = tz * ((c.M + kTmaTR - 1) / kTmaTR);
                 for (int t = 0; t < nt; t++) {
@@ -519,7 +507,8 @@ int ast_batch_create(const ast_config* cfgs, int nprob, ast_batch** out)
         for (int s = 0; s < nprob; s++) {
             const ast_config& c = B->cfg[order[s]];
             ms[s + 1] = ms[s] + tiles_of(c, 0);
-            ms[nprob + 1 + s] = slot_kflux(B, s);
+            ms[nprob + 1 + s] =
+                (c.flux == AST_FLUX_HLL) ? 0 : (c.flux == AST_FLUX_HLLC) ? 1 : (c.flux == AST_FLUX_HLLC_A) ? 3 : 2;
         }
         B->mix_tiles = ms[nprob];
         B->mix_recon = cfgs[0].recon;

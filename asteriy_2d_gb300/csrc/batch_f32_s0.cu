@@ -13,13 +13,11 @@ int launch_batch_tma(const StepParams* Ps, const CUtensorMap* tin, const CUtenso
         if (flux == AST_FLUX_HLL) AST_BTMA(0, true);
         if (flux == AST_FLUX_HLLC) AST_BTMA(1, true);
         if (flux == AST_FLUX_HLLC_A) AST_BTMA(3, true);
-        if (flux == kExactInline) AST_BTMA(kExactInline, true);
         AST_BTMA(2, true);
     }
     if (flux == AST_FLUX_HLL) AST_BTMA(0, false);
     if (flux == AST_FLUX_HLLC) AST_BTMA(1, false);
     if (flux == AST_FLUX_HLLC_A) AST_BTMA(3, false);
-    if (flux == kExactInline) AST_BTMA(kExactInline, false);
     AST_BTMA(2, false);
 #undef AST_BTMA
 }

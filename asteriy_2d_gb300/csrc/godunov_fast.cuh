@@ -447,38 +447,14 @@ __device__ __forceinline__ double godunov_sample64(const Gas<double>& g, const R
 // whose lanes need different ones), and the Newton iteration keeps each side's
 // 1/(rho c) and 1/p.  A step of the disturbed 4096x2048 wind: 458 us with
 // physics.cuh's code, 410 with this.
-namespace r32 {
-// Explicit roundings: several kernels inline this code and have to give the
-// same bits, which the compiler's own choice of fused operations does not.
-__device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ float sub(float a, float b) { return __fsub_rn(a, b); }
-}  // namespace r32
-
-__device__ __forceinline__ RPre<float> godunov_sides32(const Gas<float>& g, float rL, float pL, float unL, float utL,
-                                                       float rR, float pR, float unR, float utR)
-{
-    RPre<float> q;
-    q.swap = pL > pR;
-    q.enI = q.swap ? -unR : unL; q.teI = q.swap ? utR : utL; q.pI = q.swap ? pR : pL; q.rI = q.swap ? rR : rL;
-    q.enII = q.swap ? -unL : unR; q.teII = q.swap ? utL : utR; q.pII = q.swap ? pL : pR; q.rII = q.swap ? rL : rR;
-    q.cI = (q.rI != 0.0f) ? sqrtf(r32::mul(g.ga, q.pI) / q.rI) : 0.0f;
-    q.cII = (q.rII != 0.0f) ? sqrtf(r32::mul(g.ga, q.pII) / q.rII) : 0.0f;
-    q.Udf = r32::sub(q.enI, q.enII);
-    q.Urz = q.Uvk = 0.0f;
-    q.pattern = 4;
-    return q;
-}
-
 __device__ __forceinline__ RPre<float> godunov_pre32(const Gas<float>& g, float rL, float pL, float unL, float utL,
                                                      float rR, float pR, float unR, float utR)
 {
-    using namespace r32;
-    RPre<float> q = godunov_sides32(g, rL, pL, unL, utL, rR, pR, unR, utR);
-    const float Uud = mul(sub(q.pII, q.pI), rsqrtf(mul(q.rI, fmaf(g.hg2, q.pII, mul(g.hg1, q.pI)))));
+    RPre<float> q = godunov_sides(g, rL, pL, unL, utL, rR, pR, unR, utR);
+    const float Uud = (q.pII - q.pI) * rsqrtf(q.rI * (g.hg2 * q.pII + g.hg1 * q.pI));
     if (!(q.Udf > 0.0f)) {
-        q.Urz = mul(mul(-g.k2, q.cII), sub(1.0f, powf(q.pI / q.pII, g.gm)));
-        q.Uvk = mul(-g.k2, add(q.cII, q.cI));
+        q.Urz = -2.0f * q.cII * g.inv_g1 * (1.0f - powf(q.pI / q.pII, g.gm));
+        q.Uvk = -2.0f * (q.cII + q.cI) * g.inv_g1;
         if (q.Udf < q.Uvk) { q.pattern = 0; return q; }
         if (q.Udf <= q.Urz) { q.pattern = 1; return q; }
     }
@@ -487,51 +463,41 @@ __device__ __forceinline__ RPre<float> godunov_pre32(const Gas<float>& g, float 
     return q;
 }
 
-// pvrs_guess (physics.cuh), both terms divided by the impedances' product
-// (kK = 1/(rho_K c_K))
-__device__ __forceinline__ float pvrs_guess32(const RPre<float>& q)
-{
-    using namespace r32;
-    const float kI = 1.0f / mul(q.rI, q.cI), kII = 1.0f / mul(q.rII, q.cII);
-    const float p0 = fmaf(q.pI, kI, fmaf(q.pII, kII, q.Udf)) / add(kI, kII);
-    return q.pattern == 2 ? fminf(fmaxf(p0, q.pI), q.pII) : fmaxf(p0, q.pII);
-}
-
 // solve_p_newton (physics.cuh) in FP32
 __device__ __forceinline__ float solve_newton32(const Gas<float>& g, const RPre<float>& q, float p0, RiemannCount& rc)
 {
-    using namespace r32;
     float lo = (q.pattern == 2) ? q.pI : q.pII;
     float hi = (q.pattern == 2) ? q.pII : INFINITY;
-    const float tol = newton_tol(g.tol);
-    const float kI = 1.0f / mul(q.rI, q.cI), kII = 1.0f / mul(q.rII, q.cII), iI = 1.0f / q.pI, iII = 1.0f / q.pII;
+    const float dU = q.enI - q.enII, tol = newton_tol(g.tol);
+    const float kI = 1.0f / (q.rI * q.cI), kII = 1.0f / (q.rII * q.cII), iI = 1.0f / q.pI, iII = 1.0f / q.pII;
+    const float ga4 = 0.25f / g.ga, gp1 = g.ga + 1.0f, b = 3.0f * g.ga - 1.0f, k2 = 2.0f * g.inv_g1;
     float p = p0, prev_step = INFINITY;
     int k = 0;
     for (;;) {
         k++;
-        float f = -q.Udf, df = 0.0f;
+        float f = -dU, df = 0.0f;
 #pragma unroll
         for (int side = 0; side < 2; side++) {
             const float pK = side ? q.pII : q.pI, cK = side ? q.cII : q.cI, kK = side ? kII : kI;
-            const float x = mul(p, side ? iII : iI);
+            const float x = p * (side ? iII : iI);
             if (p > pK) {
-                const float is = rsqrtf(fmaf(g.gp, x, g.gm));
-                f = fmaf(mul(sub(p, pK), kK), is, f);
-                df = fmaf(mul(mul(fmaf(g.g2, x, g.n1), g.q4), kK), mul(mul(is, is), is), df);
+                const float is = rsqrtf(g.gp * x + g.gm);
+                f += (p - pK) * kK * is;
+                df += (gp1 * x + b) * ga4 * kK * (is * is * is);
             } else {
                 const float t = powf(x, g.gm);
-                f = fmaf(mul(g.k2, cK), sub(t, 1.0f), f);
-                df = add(df, mul(t, kK) / x);
+                f += k2 * cK * (t - 1.0f);
+                df += t * kK / x;
             }
         }
         if (f < 0.0f) lo = fmaxf(lo, p); else hi = fminf(hi, p);
-        float pn = sub(p, f / df);
-        if (fabsf(sub(pn, p)) <= mul(tol, p)) {
+        float pn = p - f / df;
+        if (fabsf(pn - p) <= tol * p) {
             p = pn;
             break;
         }
-        if (!(pn > lo && pn < hi)) pn = (pn >= hi) ? hi : mul(0.5f, add(lo, fminf(hi, mul(2.0f, p))));
-        const float step = fabsf(sub(pn, p));
+        if (!(pn > lo && pn < hi)) pn = (pn >= hi) ? hi : 0.5f * (lo + fminf(hi, 2.0f * p));
+        const float step = fabsf(pn - p);
         const bool done = k > 2 && step >= prev_step;
         prev_step = step;
         p = pn;
@@ -542,15 +508,6 @@ __device__ __forceinline__ float solve_newton32(const Gas<float>& g, const RPre<
     rc.newton_iters += k;
     if (k > rc.newton_max) rc.newton_max = k;
     return p;
-}
-
-// rare_coef<float> (physics.cuh)
-__device__ __forceinline__ float rare_coef32(const Gas<float>& g, float rc, float p, float pK)
-{
-    using namespace r32;
-    const float x = p / pK, d = sub(1.0f, x);
-    if (fabsf(d) < 0.02f) return mul(rc, fmaf(d, fmaf(d, fmaf(d, g.rs[2], g.rs[1]), g.rs[0]), 1.0f));
-    return mul(mul(g.gm, rc), d) / sub(1.0f, powf(x, g.gm));
 }
 
 struct WildSample32 {
@@ -572,36 +529,36 @@ template <int MODE>
 __device__ __forceinline__ float godunov_sample32(const Gas<float>& g, const RPre<float>& q, float p, float F[4],
                                                   RiemannCount& rc)
 {
-    const bool two_raref = MODE == kSampleAll ? q.pattern == 1 : MODE == kSampleClosed;
-    if (MODE == kSampleAll ? (q.pattern == 0 || q.pattern == 4) : (two_raref && q.pattern != 1)) {
+    constexpr bool two_raref = MODE == kSampleClosed;
+    if (two_raref && q.pattern != 1) {
         // vacuum, or no pattern
         const WildSample32 w = sample_wild32(g, q);
         rc.status |= w.status;
         for (int k = 0; k < 4; k++) F[k] = w.F[k];
         return w.S;
     }
-    using namespace r32;
     const bool shockII = !two_raref && q.pattern == 3;
-    const float zI = mul(q.rI, q.cI), zII = mul(q.rII, q.cII);
     float aI, aII;
     if (two_raref) {
-        p = mul(q.pI, powf(sub(q.Udf, q.Uvk) / sub(q.Urz, q.Uvk), g.inv_gm));
-        aI = rare_coef32(g, zI, p, q.pI);
+        p = q.pI * powf((q.Udf - q.Uvk) / (q.Urz - q.Uvk), 1.0f / g.gm);
+        aI = rare_coef(g, q.rI, q.cI, p, q.pI);
+        aII = rare_coef(g, q.rII, q.cII, p, q.pII);
     } else {
-        aI = sqrtf(mul(q.rI, fmaf(g.hg2, p, mul(g.hg1, q.pI))));
+        aI = sqrtf(q.rI * (g.hg2 * p + g.hg1 * q.pI));
+        if (shockII) aII = sqrtf(q.rII * (g.hg2 * p + g.hg1 * q.pII));
+        else aII = rare_coef(g, q.rII, q.cII, p, q.pII);
     }
-    if (shockII) aII = sqrtf(mul(q.rII, fmaf(g.hg2, p, mul(g.hg1, q.pII))));
-    else aII = rare_coef32(g, zII, p, q.pII);
-    const float u = fmaf(aI, q.enI, fmaf(aII, q.enII, sub(q.pI, q.pII))) / add(aI, aII);
+    const float u = (aI * q.enI + aII * q.enII + (q.pI - q.pII)) / (aI + aII);
     // heads (d) and tails (dd) of the two waves; a shock is both
-    const float wI = sub(q.enI, u), wII = sub(q.enII, u);
-    const float dI = sub(q.enI, two_raref ? q.cI : aI / q.rI);
-    const float ddI = two_raref ? fmaf(-g.hg1, wI, sub(u, q.cI)) : dI;
-    const float dII = add(q.enII, shockII ? aII / q.rII : q.cII);
-    const float ddII = shockII ? dII : fmaf(-g.hg1, wII, add(u, q.cII));
+    const float wI = q.enI - u, wII = q.enII - u;
+    const float dI = two_raref ? q.enI - q.cI : q.enI - aI / q.rI;
+    const float ddI = two_raref ? u - q.cI - g.hg1 * wI : dI;
+    const float dII = shockII ? q.enII + aII / q.rII : q.enII + q.cII;
+    const float ddII = shockII ? dII : u + q.cII - g.hg1 * wII;
     const float UU = fmaxf(fmaxf(fabsf(dI), fabsf(dII)), fmaxf(fabsf(ddI), fabsf(ddII)));
     // the interval that holds w = 0, side II mirrored
     const bool left = u >= 0.0f;
+    const float sg = left ? 1.0f : -1.0f;
     const float d = left ? dI : -dII, dd = left ? ddI : -ddII, w = left ? wI : -wII, a = left ? aI : aII;
     const float r0 = left ? q.rI : q.rII, c0 = left ? q.cI : q.cII;
     const float te = left ? q.teI : q.teII;
@@ -610,14 +567,14 @@ __device__ __forceinline__ float godunov_sample32(const Gas<float>& g, const RPr
     if (d < 0.0f) {
         if (dd > 0.0f) {
             // inside a rarefaction fan
-            const float ce = fmaf(g.g1, left ? en : -en, mul(2.0f, c0)) / g.g2;
-            ps = mul(ps, powf(ce / c0, g.inv_gm));
-            r = mul(g.ga, ps) / mul(ce, ce);
-            en = left ? ce : -ce;
+            const float ce = (g.g1 * (sg * en) + 2.0f * c0) / g.g2;
+            ps = ps * powf(ce / c0, 1.0f / g.gm);
+            r = g.ga * ps / (ce * ce);
+            en = sg * ce;
         } else {
             // between the wave and the contact
-            const float ce = fmaf(g.hg1, w, c0);
-            r = (shock ? mul(r0, a) : mul(g.ga, p)) / (shock ? fmaf(-r0, w, a) : mul(ce, ce));
+            const float ce = c0 + g.hg1 * w;
+            r = (shock ? r0 * a : g.ga * p) / (shock ? a - r0 * w : ce * ce);
             en = u;
             ps = p;
         }
@@ -625,11 +582,11 @@ __device__ __forceinline__ float godunov_sample32(const Gas<float>& g, const RPr
         ps = NAN;   // a state that is not a number
     }
     if (q.swap) en = -en;
-    const float m = mul(r, en), k = mul(mul(0.5f, r), fmaf(en, en, mul(te, te)));
+    const float m = r * en;
     F[0] = m;
-    F[1] = fmaf(m, en, ps);
-    F[2] = mul(m, te);
-    F[3] = mul(en, add(fmaf(ps, g.inv_g1, k), ps));
+    F[1] = m * en + ps;
+    F[2] = m * te;
+    F[3] = en * (ps * g.inv_g1 + 0.5f * r * (en * en + te * te) + ps);
     return fmaxf(UU, g.eps8);
 }
 
@@ -651,7 +608,7 @@ __device__ __forceinline__ RPre<double> face_pre(const Gas<double>& g, double rL
 __device__ __forceinline__ RPre<float> face_sides_of(const Gas<float>& g, float rL, float pL, float unL, float utL,
                                                      float rR, float pR, float unR, float utR)
 {
-    return godunov_sides32(g, rL, pL, unL, utL, rR, pR, unR, utR);
+    return godunov_sides(g, rL, pL, unL, utL, rR, pR, unR, utR);
 }
 __device__ __forceinline__ RPre<double> face_sides_of(const Gas<double>& g, double rL, double pL, double unL,
                                                       double utL, double rR, double pR, double unR, double utR)
@@ -660,8 +617,6 @@ __device__ __forceinline__ RPre<double> face_sides_of(const Gas<double>& g, doub
         return godunov_sides64(g, rL, pL, unL, utL, rR, pR, unR, utR);
     return sides_wild(g, rL, pL, unL, utL, rR, pR, unR, utR);
 }
-__device__ __forceinline__ float face_guess(const RPre<float>& q) { return pvrs_guess32(q); }
-__device__ __forceinline__ double face_guess(const RPre<double>& q) { return pvrs_guess(q); }
 // the safeguarded Newton from p0
 __device__ __forceinline__ float face_newton(const Gas<float>& g, const RPre<float>& q, float p0, RiemannCount& rc)
 {

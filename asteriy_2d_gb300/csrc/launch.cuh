@@ -226,13 +226,6 @@ int launch_step_r(const StepParams& P, int flux, int recon, cudaStream_t st, boo
         else
             return set_error(AST_ERR_UNSUPPORTED, "HLLCQ is an FP64 flux");
     }
-    if (flux == kExactInline) {
-        if constexpr (sizeof(R) == 4)
-            return recon ? launch_step_t<R, kExactInline, true, LAYOUT>(P, st, launch)
-                         : launch_step_t<R, kExactInline, false, LAYOUT>(P, st, launch);
-        else
-            return set_error(AST_ERR_UNSUPPORTED, "an FP32 kernel");
-    }
     if (recon) {
         if (flux == AST_FLUX_HLL) return launch_step_t<R, 0, true, LAYOUT>(P, st, launch);
         if (flux == AST_FLUX_HLLC) return launch_step_t<R, 1, true, LAYOUT>(P, st, launch);
@@ -275,17 +268,11 @@ int launch_batch_r(const StepParams* Ps, const int* tile_start, int nprob, int t
         if (flux == AST_FLUX_HLLC) return launch_batch_t<R, 1, true, TZ, TR>(Ps, tile_start, nprob, tiles, st, launch);
         if (flux == AST_FLUX_HLLC_A)
             return launch_batch_t<R, 3, true, TZ, TR>(Ps, tile_start, nprob, tiles, st, launch);
-        if constexpr (sizeof(R) == 4)
-            if (flux == kExactInline)
-                return launch_batch_t<R, kExactInline, true, TZ, TR>(Ps, tile_start, nprob, tiles, st, launch);
         return launch_batch_t<R, 2, true, TZ, TR>(Ps, tile_start, nprob, tiles, st, launch);
     }
     if (flux == AST_FLUX_HLL) return launch_batch_t<R, 0, false, TZ, TR>(Ps, tile_start, nprob, tiles, st, launch);
     if (flux == AST_FLUX_HLLC) return launch_batch_t<R, 1, false, TZ, TR>(Ps, tile_start, nprob, tiles, st, launch);
     if (flux == AST_FLUX_HLLC_A) return launch_batch_t<R, 3, false, TZ, TR>(Ps, tile_start, nprob, tiles, st, launch);
-    if constexpr (sizeof(R) == 4)
-        if (flux == kExactInline)
-            return launch_batch_t<R, kExactInline, false, TZ, TR>(Ps, tile_start, nprob, tiles, st, launch);
     return launch_batch_t<R, 2, false, TZ, TR>(Ps, tile_start, nprob, tiles, st, launch);
 }
 
@@ -333,13 +320,6 @@ int launch_batch_tma_mixed(const StepParams* Ps, const CUtensorMap* tin, const C
 // -> q2, before the gas step of the same time level
 int launch_scalar(const StepParams& P, const double* q, double* q2, int flux, int recon, double q_fixed,
                   cudaStream_t st);
-
-// the kernels' FLUX of a configuration
-inline int kernel_flux(const ast_config& c)
-{
-    return c.flux == AST_FLUX_GODUNOV && c.precision == AST_PREC_FP32 && c.guess != AST_GUESS_MLP ? kExactInline
-                                                                                                  : c.flux;
-}
 
 // kernel parameters of a configuration (grid spacing, constants, boundaries)
 inline void fill_step_params(StepParams& P, const ast_config& c)

@@ -34,8 +34,6 @@ struct Gas {
     R eps;                    // 10e-10: degenerate rarefaction test (Header.h:62)
     R eps8;                   // 10e-8: smallest wave speed for dt (Header.h:63)
     R hg1, hg2;               // (gamma-1)/2, (gamma+1)/2
-    R k2, inv_gm, q4, n1;     // 2/(gamma-1), 1/gm, 1/(4 gamma), 3 gamma - 1
-    R rs[3];                  // the series of a rarefaction's coefficient about p = p_K (rare_coef)
     int max_iter;
     int n;                    // 1/gm when it is a whole number from 2 to 16, else 0
     int zero;                 // 0, unknown to the compiler (d64::Pipe)
@@ -57,16 +55,6 @@ __host__ __device__ inline Gas<R> make_gas(double gamma, double tol, int max_ite
     g.eps8 = (R)10e-8;
     g.hg1 = (R)(0.5 * g1);
     g.hg2 = (R)(0.5 * g2);
-    g.k2 = (R)(2.0 / g1);
-    g.inv_gm = (R)(2.0 * gamma / g1);
-    g.q4 = (R)(0.25 / gamma);
-    g.n1 = (R)(3.0 * gamma - 1.0);
-    {
-        const double e = (g1 / gamma) / 2.0, a = 0.5 * (e - 1.0), b = (e - 1.0) * (e - 2.0) / 6.0;
-        g.rs[0] = (R)a;
-        g.rs[1] = (R)(a * a - b);
-        g.rs[2] = (R)(a * a * a - 2.0 * a * b + (e - 1.0) * (e - 2.0) * (e - 3.0) / 24.0);
-    }
     g.max_iter = max_iter;
     const double n = 2.0 * gamma / g1;
     const int ni = (n > 1.5 && n < 16.5) ? (int)(n + 0.5) : 0;

@@ -94,14 +94,6 @@ __device__ __forceinline__ void phase_mark(int, DevClock* = nullptr) {}
 
 enum Layout { kSoA = 0, kAoS = 1 };
 
-// The kernels' FLUX: enum ast_flux, or the FP32 exact solver without the
-// learned start value.  It solves every face where it is met: with the queue,
-// its shared memory and its code in the kernel the disturbed 4096x2048 wind
-// took 406 us a step, without 348, the grown blast 98 and 91 (the queue's
-// full warps pay for recomputing a face's states where iterations are long:
-// FP64; in FP32 the safeguarded Newton takes one or two).
-constexpr int kExactInline = 5;
-
 struct __align__(16) StepParams {
     int N, M;
     long long ld;                  // SoA row pitch in elements
@@ -642,10 +634,10 @@ __device__ __forceinline__ R solve_queued(const StepParams& P, const Gas<R>& g, 
         p0 = p0_mlp;
         if (!in_basin(q, p0)) {
             fallback++;
-            p0 = face_guess(q);
+            p0 = pvrs_guess(q);
         }
     } else {
-        p0 = face_guess(q);
+        p0 = pvrs_guess(q);
     }
     const int k0 = rc.newton_iters;
     const R p = face_newton(g, q, p0, rc);
@@ -751,14 +743,13 @@ __device__ __forceinline__ bool face_states(const StepParams& P, const S& sm, in
 // the exact solver's flux and wave speed of a face whose sides hold one state
 __device__ __forceinline__ float exact_same_state(const Gas<float>& g, float r, float p, float un, float ut, float F[4])
 {
-    using namespace r32;
-    const float cs = sqrtf(mul(g.ga, p) / r);
-    const float m = mul(r, un);
+    const float cs = sqrt(g.ga * p / r);
+    const float m = r * un;
     F[0] = m;
-    F[1] = fmaf(m, un, p);
-    F[2] = mul(m, ut);
-    F[3] = mul(un, add(fmaf(p, g.inv_g1, mul(mul(0.5f, r), fmaf(un, un, mul(ut, ut)))), p));
-    return fmaxf(add(fabsf(un), cs), g.eps8);
+    F[1] = m * un + p;
+    F[2] = m * ut;
+    F[3] = un * (p * g.inv_g1 + 0.5f * r * (un * un + ut * ut) + p);
+    return fmax(fabs(un) + cs, g.eps8);
 }
 __device__ __forceinline__ double exact_same_state(const Gas<double>& g, double r, double p, double un, double ut,
                                                    double F[4])
@@ -807,17 +798,6 @@ __device__ __forceinline__ void face_meta(const StepParams& P, const S& sm, int 
     }
 }
 
-// Face (a, c) of orientation ZF into the exact solver's queue (room for every
-// face of the tile); its flux is written by queue_pass.
-template <bool ZF, int TZ, int TR, typename S>
-__device__ __forceinline__ void push_face(S& sm, int a, int c, bool active, int pattern, bool front)
-{
-    const unsigned old = atomicAdd(&sm.qn, front ? 1u : 0x10000u);
-    const int slot = front ? (int)(old & 0xffffu) : S::kQueueCap - 1 - (int)(old >> 16);
-    const int f = ZF ? a * (TZ + 1) + c : TR * (TZ + 1) + a * TZ + c;
-    sm.qcode[slot] = (unsigned short)(f | (active ? 1 << 12 : 0) | (pattern << 14));
-}
-
 // The flux of face (a, c) from its reconstructed states L (lower cell) and U
 // (upper cell): written, in (mass, mom_z, mom_r, energy) order, to sm.Fz /
 // sm.Fr, and smax raised to its wave speed when the face is active.
@@ -827,11 +807,13 @@ __device__ __forceinline__ void face_flux(const StepParams& P, S& sm, const Gas<
                                           bool hi, const R L[4], const R U[4], RiemannCount& rc, R& smax,
                                           bool same_sides = false)
 {
+    constexpr int NFZ = TR * (TZ + 1);
+    constexpr int W = ZF ? TZ + 1 : TZ;      // faces per row of the face array
     constexpr int NN = ZF ? 2 : 3;           // normal velocity component
     constexpr int TT = ZF ? 3 : 2;           // tangential velocity component
     R F[4];
     R Sp;
-    if constexpr (FLUX == 2 || FLUX == kExactInline) {
+    if constexpr (FLUX == 2) {
         if (!active) {
             // no updated cell uses this face (both cells outside the grid or
             // held fixed): not solved, so the solver's counters see the same
@@ -852,26 +834,20 @@ __device__ __forceinline__ void face_flux(const StepParams& P, S& sm, const Gas<
             return;
         } else if (hi) {
             const RPre<R> q = face_pre(g, L[0], L[1], L[NN], L[TT], U[0], U[1], U[NN], U[TT]);
-            const bool iterative = q.pattern == 2 || q.pattern == 3;
-            if constexpr (FLUX == kExactInline) {
-                R p = R(0);
-                if (iterative) {
-                    int none = 0;
-                    p = solve_queued(P, g, q, gate_used(P) && wave_strength(q) > P.mlp_gate, R(0), rc, none);
-                }
-                Sp = face_sample<kSampleAll>(g, q, p, F, rc);
-            } else {
-                if (iterative) {
-                    // to the queue; front: the faces above the learned start's
-                    // gate where it is used or counted, else those of pattern
-                    // 3 (the two patterns' iterations take other branches:
-                    // other warps)
-                    push_face<ZF, TZ, TR>(sm, a, c, active, q.pattern,
-                                          gate_used(P) ? wave_strength(q) > P.mlp_gate : q.pattern == 3);
-                    return;
-                }
-                Sp = face_sample<kSampleClosed>(g, q, R(0), F, rc);
+            if (q.pattern == 2 || q.pattern == 3) {
+                // the iterative faces go to the queue (room for every face
+                // of the tile); their flux is written by queue_pass
+                // front: the faces above the learned start's gate where the gate
+                // is used or counted, else those of pattern 3 (the two patterns'
+                // iterations take other branches: kept in other warps)
+                const bool front = gate_used(P) ? wave_strength(q) > P.mlp_gate : q.pattern == 3;
+                const unsigned old = atomicAdd(&sm.qn, front ? 1u : 0x10000u);
+                const int slot = front ? (int)(old & 0xffffu) : S::kQueueCap - 1 - (int)(old >> 16);
+                const int f = a * W + c;
+                sm.qcode[slot] = (unsigned short)((ZF ? f : NFZ + f) | (active ? 1 << 12 : 0) | (q.pattern << 14));
+                return;
             }
+            Sp = face_sample<kSampleClosed>(g, q, R(0), F, rc);
         } else {
             Sp = flux_hll(g, L[0], L[1], L[NN], L[TT], U[0], U[1], U[NN], U[TT], F);
         }
@@ -1060,7 +1036,7 @@ __device__ __forceinline__ void face_pass(const StepParams& P, S& sm, int b, con
 {
     // every cell the tile's faces touch lies inside the grid
     const bool interior = n0 >= 1 && n0 + TZ < P.N && m0 >= 1 && m0 + TR < P.M;
-    if constexpr (FLUX != 2 && FLUX != kExactInline) {
+    if constexpr (FLUX != 2) {
         static_assert(TZ % 2 == 0 && TR % 2 == 0, "faces in pairs");
         constexpr int NZP = TR * (TZ / 2);          // z face pairs
         constexpr int NP = NZP + (TR / 2) * TZ;     // + r face pairs
@@ -1395,7 +1371,7 @@ __device__ __forceinline__ void patch_tile(const StepParams& P, S& sm, int b, in
 template <typename R, int FLUX>
 __device__ __forceinline__ R uniform_face(const Gas<R>& g, R r, R p, R un, R ut, R F[4])
 {
-    if constexpr (FLUX == 2 || FLUX == kExactInline) {
+    if constexpr (FLUX == 2) {
         return exact_same_state(g, r, p, un, ut, F);
     } else if constexpr (FLUX == 1) {
         return flux_hllc(g, r, p, un, ut, r, p, un, ut, F);
@@ -1907,7 +1883,7 @@ __global__ void __launch_bounds__(kThreads, min_ctas<R, FLUX>())
 // Many problems of any fluxes (one reconstruction) in one launch: as
 // batch_kernel, each CTA then steps its tile with the tile code of its
 // problem's flux, flux_of[j] = the kernels' FLUX (0 HLL, 1 HLLC, 2 exact
-// Godunov, 3 HLLC_Aleksashov, kExactInline); a CTA runs one of them, and the dynamic
+// Godunov, 3 HLLC_Aleksashov); a CTA runs one of the four, and the dynamic
 // shared memory is the largest of their tile spaces
 template <typename R, bool RECON, int TZ, int TR>
 __global__ void __launch_bounds__(kThreads, min_ctas<R, 2>())
@@ -1936,7 +1912,6 @@ __global__ void __launch_bounds__(kThreads, min_ctas<R, 2>())
     case 0: step_tile<R, 0, RECON, kSoA, TZ, TR>(sP, t % tz, t / tz, tiles); break;
     case 1: step_tile<R, 1, RECON, kSoA, TZ, TR>(sP, t % tz, t / tz, tiles); break;
     case 3: step_tile<R, 3, RECON, kSoA, TZ, TR>(sP, t % tz, t / tz, tiles); break;
-    case kExactInline: step_tile<R, kExactInline, RECON, kSoA, TZ, TR>(sP, t % tz, t / tz, tiles); break;
     default: step_tile<R, 2, RECON, kSoA, TZ, TR>(sP, t % tz, t / tz, tiles); break;
     }
 }
@@ -2333,7 +2308,6 @@ __global__ void __launch_bounds__(kThreads, 4)
                 case 0: uni = uniform_tile<R, 0, TZ, TR, false, S>(P, b, w.w != 0, false, 0); break;
                 case 1: uni = uniform_tile<R, 1, TZ, TR, false, S>(P, b, w.w != 0, false, 0); break;
                 case 3: uni = uniform_tile<R, 3, TZ, TR, false, S>(P, b, w.w != 0, false, 0); break;
-                // (the wave speeds of 2 and kExactInline are the same)
                 default: uni = uniform_tile<R, 2, TZ, TR, false, S>(P, b, w.w != 0, false, 0); break;
                 }
             } else {
@@ -2350,9 +2324,6 @@ __global__ void __launch_bounds__(kThreads, 4)
             case 0: tile_body<R, 0, RECON, kSoA, TZ, TR, true, true>(P, sm, b, P.gf, n0, m0, sK[b], acc, one); break;
             case 1: tile_body<R, 1, RECON, kSoA, TZ, TR, true, true>(P, sm, b, P.gf, n0, m0, sK[b], acc, one); break;
             case 3: tile_body<R, 3, RECON, kSoA, TZ, TR, true, true>(P, sm, b, P.gf, n0, m0, sK[b], acc, one); break;
-            case kExactInline:
-                tile_body<R, kExactInline, RECON, kSoA, TZ, TR, true, true>(P, sm, b, P.gf, n0, m0, sK[b], acc, one);
-                break;
             default: tile_body<R, 2, RECON, kSoA, TZ, TR, true, true>(P, sm, b, P.gf, n0, m0, sK[b], acc, one); break;
             }
         } else {

@@ -11,13 +11,11 @@ int launch_step_tma(const StepParams& P, const CUtensorMap& tin, const CUtensorM
         if (flux == AST_FLUX_HLL) return launch_tma_t<float, 0, true>(P, tin, tout, grid, st, launch, per_sm);
         if (flux == AST_FLUX_HLLC) return launch_tma_t<float, 1, true>(P, tin, tout, grid, st, launch, per_sm);
         if (flux == AST_FLUX_HLLC_A) return launch_tma_t<float, 3, true>(P, tin, tout, grid, st, launch, per_sm);
-        if (flux == kExactInline) return launch_tma_t<float, kExactInline, true>(P, tin, tout, grid, st, launch, per_sm);
         return launch_tma_t<float, 2, true>(P, tin, tout, grid, st, launch, per_sm);
     }
     if (flux == AST_FLUX_HLL) return launch_tma_t<float, 0, false>(P, tin, tout, grid, st, launch, per_sm);
     if (flux == AST_FLUX_HLLC) return launch_tma_t<float, 1, false>(P, tin, tout, grid, st, launch, per_sm);
     if (flux == AST_FLUX_HLLC_A) return launch_tma_t<float, 3, false>(P, tin, tout, grid, st, launch, per_sm);
-    if (flux == kExactInline) return launch_tma_t<float, kExactInline, false>(P, tin, tout, grid, st, launch, per_sm);
     return launch_tma_t<float, 2, false>(P, tin, tout, grid, st, launch, per_sm);
 }
 
