@@ -1,4 +1,4 @@
-// godunov_fast.cuh - the exact Riemann solver with few operations: FP64, then FP32.
+// godunov64.cuh - the exact Riemann solver's FP64 path with few FP64 operations.
 //
 // The same solver as physics.cuh's (kernel.cu:128-570, newton :635-680, devtwo
 // :682-749): the same wave patterns, the same p* and the same sampled states,
@@ -440,163 +440,13 @@ __device__ __forceinline__ double godunov_sample64(const Gas<double>& g, const R
     return max_pos(UU, g.eps8);
 }
 
-// ------------------------------------------------------------------ FP32
-// The FP32 form's exact solver: physics.cuh's formulas with fewer
-// instructions.  The sampled interval is selected before its state is formed
-// (the reference's independent tests run every interval's formulas in a warp
-// whose lanes need different ones), and the Newton iteration keeps each side's
-// 1/(rho c) and 1/p.  A step of the disturbed 4096x2048 wind: 458 us with
-// physics.cuh's code, 410 with this.
-__device__ __forceinline__ RPre<float> godunov_pre32(const Gas<float>& g, float rL, float pL, float unL, float utL,
-                                                     float rR, float pR, float unR, float utR)
-{
-    RPre<float> q = godunov_sides(g, rL, pL, unL, utL, rR, pR, unR, utR);
-    const float Uud = (q.pII - q.pI) * rsqrtf(q.rI * (g.hg2 * q.pII + g.hg1 * q.pI));
-    if (!(q.Udf > 0.0f)) {
-        q.Urz = -2.0f * q.cII * g.inv_g1 * (1.0f - powf(q.pI / q.pII, g.gm));
-        q.Uvk = -2.0f * (q.cII + q.cI) * g.inv_g1;
-        if (q.Udf < q.Uvk) { q.pattern = 0; return q; }
-        if (q.Udf <= q.Urz) { q.pattern = 1; return q; }
-    }
-    if (q.Udf <= Uud) q.pattern = 2;
-    else if (q.Udf > Uud) q.pattern = 3;
-    return q;
-}
-
-// solve_p_newton (physics.cuh) in FP32
-__device__ __forceinline__ float solve_newton32(const Gas<float>& g, const RPre<float>& q, float p0, RiemannCount& rc)
-{
-    float lo = (q.pattern == 2) ? q.pI : q.pII;
-    float hi = (q.pattern == 2) ? q.pII : INFINITY;
-    const float dU = q.enI - q.enII, tol = newton_tol(g.tol);
-    const float kI = 1.0f / (q.rI * q.cI), kII = 1.0f / (q.rII * q.cII), iI = 1.0f / q.pI, iII = 1.0f / q.pII;
-    const float ga4 = 0.25f / g.ga, gp1 = g.ga + 1.0f, b = 3.0f * g.ga - 1.0f, k2 = 2.0f * g.inv_g1;
-    float p = p0, prev_step = INFINITY;
-    int k = 0;
-    for (;;) {
-        k++;
-        float f = -dU, df = 0.0f;
-#pragma unroll
-        for (int side = 0; side < 2; side++) {
-            const float pK = side ? q.pII : q.pI, cK = side ? q.cII : q.cI, kK = side ? kII : kI;
-            const float x = p * (side ? iII : iI);
-            if (p > pK) {
-                const float is = rsqrtf(g.gp * x + g.gm);
-                f += (p - pK) * kK * is;
-                df += (gp1 * x + b) * ga4 * kK * (is * is * is);
-            } else {
-                const float t = powf(x, g.gm);
-                f += k2 * cK * (t - 1.0f);
-                df += t * kK / x;
-            }
-        }
-        if (f < 0.0f) lo = fmaxf(lo, p); else hi = fminf(hi, p);
-        float pn = p - f / df;
-        if (fabsf(pn - p) <= tol * p) {
-            p = pn;
-            break;
-        }
-        if (!(pn > lo && pn < hi)) pn = (pn >= hi) ? hi : 0.5f * (lo + fminf(hi, 2.0f * p));
-        const float step = fabsf(pn - p);
-        const bool done = k > 2 && step >= prev_step;
-        prev_step = step;
-        p = pn;
-        if (done) break;
-        if (k >= g.max_iter) { rc.status |= 0x04u; break; }
-    }
-    rc.newton_calls++;
-    rc.newton_iters += k;
-    if (k > rc.newton_max) rc.newton_max = k;
-    return p;
-}
-
-struct WildSample32 {
-    float F[4], S;
-    unsigned status;
-};
-static __device__ __noinline__ WildSample32 sample_wild32(const Gas<float>& g, RPre<float> q)
-{
-    RiemannCount rc;
-    rc.clear();
-    WildSample32 w;
-    w.S = godunov_sample(g, q, 0.0f, w.F, rc);
-    w.status = rc.status;
-    return w;
-}
-
-// godunov_sample (physics.cuh) at w = 0 in FP32; MODE as there
-template <int MODE>
-__device__ __forceinline__ float godunov_sample32(const Gas<float>& g, const RPre<float>& q, float p, float F[4],
-                                                  RiemannCount& rc)
-{
-    constexpr bool two_raref = MODE == kSampleClosed;
-    if (two_raref && q.pattern != 1) {
-        // vacuum, or no pattern
-        const WildSample32 w = sample_wild32(g, q);
-        rc.status |= w.status;
-        for (int k = 0; k < 4; k++) F[k] = w.F[k];
-        return w.S;
-    }
-    const bool shockII = !two_raref && q.pattern == 3;
-    float aI, aII;
-    if (two_raref) {
-        p = q.pI * powf((q.Udf - q.Uvk) / (q.Urz - q.Uvk), 1.0f / g.gm);
-        aI = rare_coef(g, q.rI, q.cI, p, q.pI);
-        aII = rare_coef(g, q.rII, q.cII, p, q.pII);
-    } else {
-        aI = sqrtf(q.rI * (g.hg2 * p + g.hg1 * q.pI));
-        if (shockII) aII = sqrtf(q.rII * (g.hg2 * p + g.hg1 * q.pII));
-        else aII = rare_coef(g, q.rII, q.cII, p, q.pII);
-    }
-    const float u = (aI * q.enI + aII * q.enII + (q.pI - q.pII)) / (aI + aII);
-    // heads (d) and tails (dd) of the two waves; a shock is both
-    const float wI = q.enI - u, wII = q.enII - u;
-    const float dI = two_raref ? q.enI - q.cI : q.enI - aI / q.rI;
-    const float ddI = two_raref ? u - q.cI - g.hg1 * wI : dI;
-    const float dII = shockII ? q.enII + aII / q.rII : q.enII + q.cII;
-    const float ddII = shockII ? dII : u + q.cII - g.hg1 * wII;
-    const float UU = fmaxf(fmaxf(fabsf(dI), fabsf(dII)), fmaxf(fabsf(ddI), fabsf(ddII)));
-    // the interval that holds w = 0, side II mirrored
-    const bool left = u >= 0.0f;
-    const float sg = left ? 1.0f : -1.0f;
-    const float d = left ? dI : -dII, dd = left ? ddI : -ddII, w = left ? wI : -wII, a = left ? aI : aII;
-    const float r0 = left ? q.rI : q.rII, c0 = left ? q.cI : q.cII;
-    const float te = left ? q.teI : q.teII;
-    const bool shock = left ? !two_raref : shockII;
-    float r = r0, en = left ? q.enI : q.enII, ps = left ? q.pI : q.pII;
-    if (d < 0.0f) {
-        if (dd > 0.0f) {
-            // inside a rarefaction fan
-            const float ce = (g.g1 * (sg * en) + 2.0f * c0) / g.g2;
-            ps = ps * powf(ce / c0, 1.0f / g.gm);
-            r = g.ga * ps / (ce * ce);
-            en = sg * ce;
-        } else {
-            // between the wave and the contact
-            const float ce = c0 + g.hg1 * w;
-            r = (shock ? r0 * a : g.ga * p) / (shock ? a - r0 * w : ce * ce);
-            en = u;
-            ps = p;
-        }
-    } else if (!(d >= 0.0f)) {
-        ps = NAN;   // a state that is not a number
-    }
-    if (q.swap) en = -en;
-    const float m = r * en;
-    F[0] = m;
-    F[1] = m * en + ps;
-    F[2] = m * te;
-    F[3] = en * (ps * g.inv_g1 + 0.5f * r * (en * en + te * te) + ps);
-    return fmaxf(UU, g.eps8);
-}
-
 // ------------------------------------------------------------------ by precision
 // The step's entry points: FP32 takes physics.cuh's code; FP64 the short forms
 // where the face allows them.
 __device__ __forceinline__ RPre<float> face_pre(const Gas<float>& g, float rL, float pL, float unL, float utL,
                                                 float rR, float pR, float unR, float utR)
 {
-    return godunov_pre32(g, rL, pL, unL, utL, rR, pR, unR, utR);
+    return godunov_pre(g, rL, pL, unL, utL, rR, pR, unR, utR);
 }
 __device__ __forceinline__ RPre<double> face_pre(const Gas<double>& g, double rL, double pL, double unL, double utL,
                                                  double rR, double pR, double unR, double utR)
@@ -617,15 +467,6 @@ __device__ __forceinline__ RPre<double> face_sides_of(const Gas<double>& g, doub
         return godunov_sides64(g, rL, pL, unL, utL, rR, pR, unR, utR);
     return sides_wild(g, rL, pL, unL, utL, rR, pR, unR, utR);
 }
-// the safeguarded Newton from p0
-__device__ __forceinline__ float face_newton(const Gas<float>& g, const RPre<float>& q, float p0, RiemannCount& rc)
-{
-    return solve_newton32(g, q, p0, rc);
-}
-__device__ __forceinline__ double face_newton(const Gas<double>& g, const RPre<double>& q, double p0, RiemannCount& rc)
-{
-    return solve_p_newton(g, q, p0, g.tol, rc);
-}
 // p* of a queued face by the reference's iteration
 __device__ __forceinline__ double face_solve(const Gas<double>& g, const RPre<double>& q, RiemannCount& rc)
 {
@@ -637,7 +478,7 @@ template <int MODE>
 __device__ __forceinline__ float face_sample(const Gas<float>& g, const RPre<float>& q, float p, float F[4],
                                              RiemannCount& rc)
 {
-    return godunov_sample32<MODE>(g, q, p, F, rc);
+    return godunov_sample<float, MODE>(g, q, p, F, rc);
 }
 template <int MODE>
 __device__ __forceinline__ double face_sample(const Gas<double>& g, const RPre<double>& q, double p, double F[4],

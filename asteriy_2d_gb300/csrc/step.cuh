@@ -21,7 +21,7 @@
 #include <cstddef>
 #include <type_traits>
 
-#include "godunov_fast.cuh"
+#include "godunov64.cuh"
 #include "mlp.cuh"
 #include "physics.cuh"
 #include "tma.cuh"
@@ -607,13 +607,6 @@ __device__ __forceinline__ float wave_strength(const RPre<R>& q)
     return fmaxf(lp, du);
 }
 
-// whether the faces above the learned start's gate are told from the others:
-// with the safeguarded Newton, for the learned start value or the counters
-__device__ __forceinline__ bool gate_used(const StepParams& P)
-{
-    return P.riemann_newton && (P.guess == 1 || P.collect_stats);
-}
-
 // p* of a queued (pattern 2 or 3) face: the reference's iteration, or the
 // safeguarded Newton.  Faces above the gate start from the learned value
 // p0_mlp when the learned form is on (when it leaves the basin: from the
@@ -640,7 +633,7 @@ __device__ __forceinline__ R solve_queued(const StepParams& P, const Gas<R>& g, 
         p0 = pvrs_guess(q);
     }
     const int k0 = rc.newton_iters;
-    const R p = face_newton(g, q, p0, rc);
+    const R p = solve_p_newton(g, q, p0, g.tol, rc);
     if (strong) {
         rc.strong_calls++;
         rc.strong_iters += rc.newton_iters - k0;
@@ -837,10 +830,10 @@ __device__ __forceinline__ void face_flux(const StepParams& P, S& sm, const Gas<
             if (q.pattern == 2 || q.pattern == 3) {
                 // the iterative faces go to the queue (room for every face
                 // of the tile); their flux is written by queue_pass
-                // front: the faces above the learned start's gate where the gate
-                // is used or counted, else those of pattern 3 (the two patterns'
-                // iterations take other branches: kept in other warps)
-                const bool front = gate_used(P) ? wave_strength(q) > P.mlp_gate : q.pattern == 3;
+                // front: the faces above the learned start's gate, or, with
+                // the reference's iterations, those of pattern 3 (another
+                // loop than pattern 2's: kept in other warps)
+                const bool front = P.riemann_newton ? wave_strength(q) > P.mlp_gate : q.pattern == 3;
                 const unsigned old = atomicAdd(&sm.qn, front ? 1u : 0x10000u);
                 const int slot = front ? (int)(old & 0xffffu) : S::kQueueCap - 1 - (int)(old >> 16);
                 const int f = a * W + c;
@@ -1173,10 +1166,10 @@ __device__ __forceinline__ void queue_pass(const StepParams& P, S& sm, int b, co
         __syncthreads();
     }
     // phase 2: p* (iteration), sampling and the flux of each queued face;
-    // threads 0..ns-1 take the front of the queue
+    // threads 0..ns-1 take the faces above the gate
     for (int t = threadIdx.x; t < ns + nw; t += kThreads) {
-        const bool front = t < ns, strong = front && gate_used(P);
-        const int i = front ? t : CAP - 1 - (t - ns);
+        const bool strong = t < ns;
+        const int i = strong ? t : CAP - 1 - (t - ns);
         const int code = sm.qcode[i];
         const bool active = (code >> 12) & 1;
         int a, c;

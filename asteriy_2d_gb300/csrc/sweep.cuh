@@ -191,7 +191,7 @@ __device__ __forceinline__ float sw_godunov_face(const StepParams& P, const Gas<
     const bool ident = hi && a[0] == b[0] && a[1] == b[1] && a[2] == b[2] && a[3] == b[3];
     RPre<float> q;
     q.pattern = 4;
-    if (hi && !ident) q = face_pre(g, a[0], a[1], a[2], a[3], b[0], b[1], b[2], b[3]);
+    if (hi && !ident) q = godunov_pre(g, a[0], a[1], a[2], a[3], b[0], b[1], b[2], b[3]);
     const bool iter = hi && !ident && (q.pattern == 2 || q.pattern == 3);
     const bool strong = iter && wave_strength(q) > P.mlp_gate;
     float p0m = 0.0f;
@@ -228,9 +228,9 @@ __device__ __forceinline__ float sw_godunov_face(const StepParams& P, const Gas<
     }
     if (iter) {
         const float p = solve_queued(P, g, q, strong, p0m, rc, fallback);
-        return face_sample<kSampleIterative>(g, q, p, F, rc);
+        return godunov_sample<float, kSampleIterative>(g, q, p, F, rc);
     }
-    return face_sample<kSampleClosed>(g, q, 0.0f, F, rc);
+    return godunov_sample<float, kSampleClosed>(g, q, 0.0f, F, rc);
 }
 
 // One strip: columns n0 .. n0+29 (lanes 1..30), rows [m0, m1).  Called by
