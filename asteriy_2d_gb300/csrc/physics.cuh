@@ -408,12 +408,12 @@ __device__ __forceinline__ void flux_hll_x2(const Gas<float>& g, float2 rL, floa
                                             float2 rR, float2 pR, float2 unR, float2 utR, float2 F[4], float2& S)
 {
     const float2 ga = pk(g.ga, g.ga), ig1 = pk(g.inv_g1, g.inv_g1), half = pk(0.5f, 0.5f);
-    // the larger sound speed from the larger p/r: one root a face
-    const float2 q = mul2(ga, pk(fmaxf((rL.x <= 0.0f) ? 0.0f : pL.x / rL.x, (rR.x <= 0.0f) ? 0.0f : pR.x / rR.x),
-                                 fmaxf((rL.y <= 0.0f) ? 0.0f : pL.y / rL.y, (rR.y <= 0.0f) ? 0.0f : pR.y / rR.y)));
-    const float2 mxc = pk(sqrtf(q.x), sqrtf(q.y));
+    const float2 gpL = mul2(ga, pL), gpR = mul2(ga, pR);
+    const float2 cL = pk((rL.x <= 0.0f) ? 0.0f : sqrtf(gpL.x / rL.x), (rL.y <= 0.0f) ? 0.0f : sqrtf(gpL.y / rL.y));
+    const float2 cR = pk((rR.x <= 0.0f) ? 0.0f : sqrtf(gpR.x / rR.x), (rR.y <= 0.0f) ? 0.0f : sqrtf(gpR.y / rR.y));
     const float2 eL = fma2(mul2(rL, fma2(utL, utL, mul2(unL, unL))), half, mul2(pL, ig1));
     const float2 eR = fma2(mul2(rR, fma2(utR, utR, mul2(unR, unR))), half, mul2(pR, ig1));
+    const float2 mxc = pk(fmaxf(cL.x, cR.x), fmaxf(cL.y, cR.y));
     const float2 DL = sub2(pk(fminf(unL.x, unR.x), fminf(unL.y, unR.y)), mxc);
     const float2 DR = add2(pk(fmaxf(unL.x, unR.x), fmaxf(unL.y, unR.y)), mxc);
     S = pk(fmaxf(fabsf(DL.x), fabsf(DR.x)), fmaxf(fabsf(DL.y), fabsf(DR.y)));
@@ -537,38 +537,10 @@ __device__ __forceinline__ R flux_hllc_ref(const Gas<R>& g, R rL, R pL, R u1, R 
     return S;
 }
 
-// FP32: the star state's own flux, as the FP64 short form below (fewer
-// operations than F_K + S_K (U* - U_K), and no difference of the large terms
-// S_K rho* and S_K rho_K); the larger sound speed from the larger p/r
-__device__ __forceinline__ float flux_hllc(const Gas<float>& g, float rL, float pL, float u1, float v1, float rR,
-                                           float pR, float u2, float v2, float F[4])
+template <typename R>
+__device__ __forceinline__ R flux_hllc(const Gas<R>& g, R rL, R pL, R u1, R v1, R rR, R pR, R u2, R v2, R F[4])
 {
-    const float c = sqrtf(g.ga * fmaxf(pL / rL, pR / rR));
-    const float SL = fminf(u1, u2) - c, SR = fmaxf(u1, u2) + c;
-    const float smax = fmaxf(fabsf(SL), fabsf(SR));
-    if (SL >= 0.0f || SR <= 0.0f) {
-        const bool l = SL >= 0.0f;
-        const float r = l ? rL : rR, p = l ? pL : pR, u = l ? u1 : u2, v = l ? v1 : v2;
-        const float m = r * u;
-        F[0] = m;
-        F[1] = m * u + p;
-        F[2] = m * v;
-        F[3] = (p * g.inv_g1 + r * (u * u + v * v) * 0.5f + p) * u;
-        return smax;
-    }
-    const float wL = SL - u1, wR = SR - u2, aL = rL * wL, aR = rR * wR;
-    const float SM = (aR * u2 - aL * u1 + (pL - pR)) / (aR - aL);
-    const float ps = 0.5f * ((aR * (SM - u2) + pR) + (aL * (SM - u1) + pL));
-    const bool l = SM >= 0.0f;
-    const float r = l ? rL : rR, p = l ? pL : pR, u = l ? u1 : u2, v = l ? v1 : v2;
-    const float w = l ? wL : wR, a = l ? aL : aR, S = l ? SL : SR;
-    const float inv = 1.0f / (S - SM);
-    const float e = p * g.inv_g1 + r * (u * u + v * v) * 0.5f;
-    F[0] = a * inv * SM;
-    F[1] = F[0] * SM + ps;
-    F[2] = F[0] * v;
-    F[3] = ((e * w + (ps * SM - p * u)) * inv + ps) * SM;
-    return smax;
+    return flux_hllc_ref(g, rL, pL, u1, v1, rR, pR, u2, v2, F);
 }
 static __device__ __noinline__ WildFlux flux_hllc_wild(const Gas<double>& g, double rL, double pL, double u1, double v1,
                                                         double rR, double pR, double u2, double v2)

@@ -439,36 +439,40 @@ __device__ __forceinline__ bool is_nan(double a)
 // Conservative update of one cell in FP32 from its state `in`
 // (rho, p, vz, vr) and its four face fluxes f[k][face] (k = mass, mom_z,
 // mom_r, energy; face = right, left, bottom, top, all oriented along +z/+r).
-// tz = T_do/dx and tr = T_do/dy multiply the flux differences, ty = T_do/r; the
-// momenta serve the energies.  Planar: Kernel_TVD, kernel.cu:3027-3073;
+// tdv = T_do/(dx dy), ty = T_do/r.  Planar: Kernel_TVD, kernel.cu:3027-3073;
 // axisymmetric with the cylindrical source: add_MK, kernel.cu:2480-2509.
-__device__ __forceinline__ void update_cell(const StepParams& P, float g1, float inv_g1, const float in[4],
-                                            const float f[4][4], float T_do, float tz, float tr, float ty, float Q2,
-                                            int& nrho, int& np, unsigned& status, float out[4], float& E2o,
+__device__ __forceinline__ void update_cell(const StepParams& P, float ga, float g1, float inv_g1, const float in[4],
+                                            const float f[4][4], float T_do, float tdv, float ty, float dx, float dy,
+                                            float Q2, int& nrho, int& np, unsigned& status, float out[4], float& E2o,
                                             float& KE2o)
 {
     const float r1 = in[0], p1 = in[1], vz1 = in[2], vr1 = in[3];
-    const float mz1 = r1 * vz1, mr1 = r1 * vr1;
-    const float E1 = p1 * inv_g1 + 0.5f * (mz1 * vz1 + mr1 * vr1);
-    float U[4] = {r1, mz1, mr1, E1};
+    float ps[4];
 #pragma unroll
-    for (int k = 0; k < 4; k++) U[k] = U[k] - tz * (f[k][0] - f[k][1]) - tr * (f[k][3] - f[k][2]);
+    for (int k = 0; k < 4; k++) {
+        const float f12 = f[k][0], f14 = -f[k][1], f13 = -f[k][2], f15 = f[k][3];
+        if (P.geom == 1) ps[k] = (f12 + f14) * dy + (f13 + f15) * dx;
+        else ps[k] = f12 * dy + f13 * dx + f14 * dy + f15 * dx;
+    }
+    const float Q3 = Q2 * vr1;
+    const float ke1 = r1 * (vz1 * vz1 + vr1 * vr1) * 0.5f;
+    float rho2, mz, mr, E2;
     if (P.geom == 1) {
-        const float w = ty * mr1;
-        U[0] -= w;
-        U[1] -= w * vz1;
-        U[2] -= w * vr1;
-        U[3] -= ty * vr1 * (E1 + p1);
+        rho2 = r1 - tdv * ps[0] - ty * r1 * vr1;
+        if (rho2 <= 0.0f) { nrho++; rho2 = r1; }
+        mz = r1 * vz1 - tdv * ps[1] - ty * r1 * vr1 * vz1;
+        mr = r1 * vr1 - tdv * ps[2] - ty * r1 * vr1 * vr1 + T_do * Q2;
+        E2 = (p1 * inv_g1 + ke1) - tdv * ps[3] - ty * vr1 * (ga * p1 * inv_g1 + ke1) + T_do * Q3;
+    } else {
+        rho2 = r1 - tdv * ps[0];
+        if (rho2 <= 0.0f) { nrho++; rho2 = r1; }
+        mz = r1 * vz1 - tdv * ps[1];
+        mr = r1 * vr1 - tdv * ps[2] + T_do * Q2;
+        E2 = (p1 * inv_g1 + ke1) - tdv * ps[3] + T_do * Q3;
     }
-    if (P.body_force) {
-        U[2] += T_do * Q2;
-        U[3] += T_do * Q2 * vr1;
-    }
-    float rho2 = U[0];
-    if (rho2 <= 0.0f) { nrho++; rho2 = r1; }
     const float irho = 1.0f / rho2;
-    const float vz2 = U[1] * irho, vr2 = U[2] * irho;
-    const float E2 = U[3], KE2 = 0.5f * (U[1] * vz2 + U[2] * vr2);
+    const float vz2 = mz * irho, vr2 = mr * irho;
+    const float KE2 = 0.5f * rho2 * (vz2 * vz2 + vr2 * vr2);
     float p2 = (E2 - KE2) * g1;
     if (p2 <= 0.0f) { np++; p2 = P.p_floorf; }
     // a non-finite flux or state reaches p2 through the energy or 1/rho
@@ -1217,7 +1221,6 @@ struct StepConsts {
     double T_do;           // the step's dt
     double ntz, ntr;       // -T_do / dx, -T_do / dy
     float tdv_f, T_f;      // T_do / (dx dy), T_do
-    float tz_f, tr_f;      // T_do / dx, T_do / dy
     int step;
 };
 
@@ -1231,8 +1234,6 @@ __device__ __forceinline__ void step_consts_of(const StepParams& P, double T_do,
     if constexpr (sizeof(R) == 4) {
         K.tdv_f = (float)(K.T_do / (P.dx * P.dy));
         K.T_f = (float)K.T_do;
-        K.tz_f = (float)-K.ntz;
-        K.tr_f = (float)-K.ntr;
     }
 }
 
@@ -1567,7 +1568,7 @@ __device__ __forceinline__ void tile_body(const StepParams& P, S& sm, int b, con
 
     // ---- conservative update of the tile's cells
     const float tdv_f = K.tdv_f, Tf = K.T_f, dxf = P.dxf, dyf = P.dyf;
-    const float g1f = P.gf.g1, ig1f = P.gf.inv_g1;
+    const float gaf = P.gf.ga, g1f = P.gf.g1, ig1f = P.gf.inv_g1;
     const auto& qv = sm.qb[b];
     // cell cidx of the tile: its staged state and its four face fluxes
     auto load_cell = [&](int row, int col, R in[4], R f[4][4]) {
@@ -1656,8 +1657,8 @@ __device__ __forceinline__ void tile_body(const StepParams& P, S& sm, int b, con
                 float ty, Q2;
                 sources_fp32(row, n, in, ty, Q2);
                 float E2, KE2;
-                update_cell(P, g1f, ig1f, in, f, Tf, K.tz_f, K.tr_f, ty, Q2, acc.nrho, acc.np, acc.rc.status, o, E2,
-                            KE2);
+                update_cell(P, gaf, g1f, ig1f, in, f, Tf, tdv_f, ty, dxf, dyf, Q2, acc.nrho, acc.np, acc.rc.status, o,
+                            E2, KE2);
                 // pressure recovery p = (g-1)(E - rho v^2/2) in FP64 where
                 // the kinetic energy is more than 99% of the total
                 if (KE2 > 0.99f * E2) deferred |= 2u << (2 * it);

@@ -303,7 +303,7 @@ __device__ __forceinline__ void sweep_strip(const StepParams& P, const StepConst
             acc.smr = fmaxf(acc.smr, Sp);
         }
     }
-    const float g1f = g.g1, ig1f = g.inv_g1;
+    const float gaf = g.ga, g1f = g.g1, ig1f = g.inv_g1;
 #pragma unroll 1
     for (int m = m0; m < m1; m++) {
         // row m+3 and the outer neighbour of row m+1, one step ahead
@@ -427,8 +427,8 @@ __device__ __forceinline__ void sweep_strip(const StepParams& P, const StepConst
                     }
                     const float ty = (P.geom == 1) ? K.T_f / y : 0.0f;
                     float E2, KE2;
-                    update_cell(P, g1f, ig1f, w0, f, K.T_f, K.tz_f, K.tr_f, ty, Q2, acc.nrho, acc.np, acc.rc.status,
-                                o, E2, KE2);
+                    update_cell(P, gaf, g1f, ig1f, w0, f, K.T_f, K.tdv_f, ty, P.dxf, P.dyf, Q2, acc.nrho, acc.np,
+                                acc.rc.status, o, E2, KE2);
                     // pressure recovery in FP64 where the kinetic energy is
                     // more than 99% of the total
                     if (KE2 > 0.99f * E2)
