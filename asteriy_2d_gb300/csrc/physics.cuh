@@ -408,12 +408,13 @@ __device__ __forceinline__ void flux_hll_x2(const Gas<float>& g, float2 rL, floa
                                             float2 rR, float2 pR, float2 unR, float2 utR, float2 F[4], float2& S)
 {
     const float2 ga = pk(g.ga, g.ga), ig1 = pk(g.inv_g1, g.inv_g1), half = pk(0.5f, 0.5f);
+    // the larger sound speed from the larger ga p/r: one root a face (a root
+    // keeps the order, so the same value, NaN and negative p included)
     const float2 gpL = mul2(ga, pL), gpR = mul2(ga, pR);
-    const float2 cL = pk((rL.x <= 0.0f) ? 0.0f : sqrtf(gpL.x / rL.x), (rL.y <= 0.0f) ? 0.0f : sqrtf(gpL.y / rL.y));
-    const float2 cR = pk((rR.x <= 0.0f) ? 0.0f : sqrtf(gpR.x / rR.x), (rR.y <= 0.0f) ? 0.0f : sqrtf(gpR.y / rR.y));
+    const float2 mxc = pk(sqrtf(fmaxf((rL.x <= 0.0f) ? 0.0f : gpL.x / rL.x, (rR.x <= 0.0f) ? 0.0f : gpR.x / rR.x)),
+                          sqrtf(fmaxf((rL.y <= 0.0f) ? 0.0f : gpL.y / rL.y, (rR.y <= 0.0f) ? 0.0f : gpR.y / rR.y)));
     const float2 eL = fma2(mul2(rL, fma2(utL, utL, mul2(unL, unL))), half, mul2(pL, ig1));
     const float2 eR = fma2(mul2(rR, fma2(utR, utR, mul2(unR, unR))), half, mul2(pR, ig1));
-    const float2 mxc = pk(fmaxf(cL.x, cR.x), fmaxf(cL.y, cR.y));
     const float2 DL = sub2(pk(fminf(unL.x, unR.x), fminf(unL.y, unR.y)), mxc);
     const float2 DR = add2(pk(fmaxf(unL.x, unR.x), fmaxf(unL.y, unR.y)), mxc);
     S = pk(fmaxf(fabsf(DL.x), fabsf(DR.x)), fmaxf(fabsf(DL.y), fabsf(DR.y)));
@@ -537,10 +538,42 @@ __device__ __forceinline__ R flux_hllc_ref(const Gas<R>& g, R rL, R pL, R u1, R 
     return S;
 }
 
-template <typename R>
-__device__ __forceinline__ R flux_hllc(const Gas<R>& g, R rL, R pL, R u1, R v1, R rR, R pR, R u2, R v2, R F[4])
+// FP32: the same values with one root (of the larger ga p/r) and one star
+// state: the side that the contact leaves behind is selected first (lanes of a
+// warp differ in it, so the two branches above ran one after the other)
+__device__ __forceinline__ float flux_hllc(const Gas<float>& g, float rL, float pL, float u1, float v1, float rR,
+                                           float pR, float u2, float v2, float F[4])
 {
-    return flux_hllc_ref(g, rL, pL, u1, v1, rR, pR, u2, v2, F);
+    const float mxc = sqrtf(fmaxf(g.ga * pL / rL, g.ga * pR / rR));
+    const float SL = fminf(u1, u2) - mxc, SR = fmaxf(u1, u2) + mxc;
+    const float smax = fmaxf(fabsf(SL), fabsf(SR));
+    const float eL = pL * g.inv_g1 + rL * (u1 * u1 + v1 * v1) * 0.5f;
+    const float eR = pR * g.inv_g1 + rR * (u2 * u2 + v2 * v2) * 0.5f;
+    if (SL >= 0.0f) {
+        const float m = rL * u1;
+        F[0] = m; F[1] = m * u1 + pL; F[2] = m * v1; F[3] = (eL + pL) * u1;
+        return smax;
+    }
+    if (SR <= 0.0f) {
+        const float m = rR * u2;
+        F[0] = m; F[1] = m * u2 + pR; F[2] = m * v2; F[3] = (eR + pR) * u2;
+        return smax;
+    }
+    const float suR = SR - u2, suL = SL - u1;
+    const float SM = (suR * rR * u2 - suL * rL * u1 - pR + pL) / (suR * rR - suL * rL);
+    const float ptz = (pR + rR * suR * (SM - u2) + pL + rL * suL * (SM - u1)) * 0.5f;
+    const bool l = SM >= 0.0f;
+    const float r = l ? rL : rR, p = l ? pL : pR, u = l ? u1 : u2, v = l ? v1 : v2;
+    const float e = l ? eL : eR, su = l ? suL : suR, S = l ? SL : SR;
+    const float inv = 1.0f / (S - SM);
+    const float rs = r * su * inv;
+    const float es = e * su * inv + (ptz * SM - p * u) * inv;
+    const float m = r * u;
+    F[0] = m + S * (rs - r);
+    F[1] = m * u + p + S * (rs * SM - m);
+    F[2] = m * v + S * (rs * v - r * v);
+    F[3] = (e + p) * u + S * (es - e);
+    return smax;
 }
 static __device__ __noinline__ WildFlux flux_hllc_wild(const Gas<double>& g, double rL, double pL, double u1, double v1,
                                                         double rR, double pR, double u2, double v2)
