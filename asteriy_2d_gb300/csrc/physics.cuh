@@ -140,7 +140,6 @@ __device__ __forceinline__ double max_abs(double a, double b)
     return from(x < y ? y : x);
 }
 __device__ __forceinline__ double max_pos(double a, double b) { return from(bits(a) < bits(b) ? bits(b) : bits(a)); }
-__device__ __forceinline__ bool finite(double a) { return (__double2hiint(a) & 0x7ff00000) != 0x7ff00000; }
 // The ranges the short forms take: positive with 2^-150 <= a < 2^150, and
 // |a| < 2^150 (so that no product or quotient of theirs leaves the normal
 // range); NaN and infinities are outside.

@@ -405,8 +405,6 @@ __device__ __forceinline__ S& tile_smem()
 // ------------------------------------------------------------------ sign and NaN tests
 // bitwise equality of two staged values
 __device__ __forceinline__ bool same_bits(float a, float b) { return __float_as_uint(a) == __float_as_uint(b); }
-// a > 0 or a positive NaN, on the bit pattern
-__device__ __forceinline__ bool positive_bits(float a) { return __float_as_int(a) > 0; }
 __device__ __forceinline__ bool same_bits(double a, double b)
 {
     return __double_as_longlong(a) == __double_as_longlong(b);
@@ -608,6 +606,13 @@ __device__ __forceinline__ float wave_strength(const RPre<R>& q)
     const float lp = __logf((float)(q.pII / q.pI));
     const float du = fabsf((float)(q.enI - q.enII)) / (float)fmin(q.cI, q.cII);
     return fmaxf(lp, du);
+}
+
+// whether the faces above the learned start's gate are told from the others:
+// with the safeguarded Newton, for the learned start value or the counters
+__device__ __forceinline__ bool gate_used(const StepParams& P)
+{
+    return P.riemann_newton && (P.guess == 1 || P.collect_stats);
 }
 
 // p* of a queued (pattern 2 or 3) face: the reference's iteration, or the
@@ -833,10 +838,11 @@ __device__ __forceinline__ void face_flux(const StepParams& P, S& sm, const Gas<
             if (q.pattern == 2 || q.pattern == 3) {
                 // the iterative faces go to the queue (room for every face
                 // of the tile); their flux is written by queue_pass
-                // front: the faces above the learned start's gate, or, with
-                // the reference's iterations, those of pattern 3 (another
-                // loop than pattern 2's: kept in other warps)
-                const bool front = P.riemann_newton ? wave_strength(q) > P.mlp_gate : q.pattern == 3;
+                // front: the faces above the learned start's gate where the gate
+                // is used or counted, else those of pattern 3 (the two patterns'
+                // iterations take other branches: kept in other warps; FP32
+                // wind 4096x2048 468 -> 455 us per step)
+                const bool front = gate_used(P) ? wave_strength(q) > P.mlp_gate : q.pattern == 3;
                 const unsigned old = atomicAdd(&sm.qn, front ? 1u : 0x10000u);
                 const int slot = front ? (int)(old & 0xffffu) : S::kQueueCap - 1 - (int)(old >> 16);
                 const int f = a * W + c;
@@ -980,27 +986,14 @@ __device__ __forceinline__ void face_two(const StepParams& P, S& sm, int b, cons
         }
     }
     if constexpr (FLUX == 0 && sizeof(R) == 4) {
-        // HLL in FP32: both faces in packed arithmetic; or, when both faces
-        // of every active lane of the warp hold one state on all four sides
-        // (one bit pattern, rho > 0, p > 0: undisturbed gas), that state's
-        // physical flux once for both (flux_physical: what the HLL formula
-        // gives up to rounding, its wave speed formed as the formula forms it)
+        // HLL in FP32: both faces in packed arithmetic.  (Warps of one state
+        // on all sides took flux_physical instead after a vote, other values
+        // in the last bits wherever a warp's faces were not all of one state
+        // and 2% of the blast's step: 76.5 against 74.9 us.)
         constexpr int NN = ZF ? 2 : 3, TT = ZF ? 3 : 2;
         float2 F[4], Sp;
-        bool one = two && positive_bits(L0[0]) && positive_bits(L0[1]);
-#pragma unroll
-        for (int k = 0; k < 4; k++)
-            one = one && same_bits(L0[k], U0[k]) && same_bits(L0[k], L1[k]) && same_bits(L0[k], U1[k]);
-        if (__all_sync(__activemask(), one)) {
-            float f[4];
-            const float s = flux_physical(g, L0[0], L0[1], L0[NN], L0[TT], f);
-#pragma unroll
-            for (int k = 0; k < 4; k++) F[k] = pk(f[k], f[k]);
-            Sp = pk(s, s);
-        } else {
-            flux_hll_x2(g, pk(L0[0], L1[0]), pk(L0[1], L1[1]), pk(L0[NN], L1[NN]), pk(L0[TT], L1[TT]),
-                        pk(U0[0], U1[0]), pk(U0[1], U1[1]), pk(U0[NN], U1[NN]), pk(U0[TT], U1[TT]), F, Sp);
-        }
+        flux_hll_x2(g, pk(L0[0], L1[0]), pk(L0[1], L1[1]), pk(L0[NN], L1[NN]), pk(L0[TT], L1[TT]), pk(U0[0], U1[0]),
+                    pk(U0[1], U1[1]), pk(U0[NN], U1[NN]), pk(U0[TT], U1[TT]), F, Sp);
         store(a, c, act0, F[0].x, F[1].x, F[2].x, F[3].x, Sp.x);
         if (two) store(a1, c1, act1, F[0].y, F[1].y, F[2].y, F[3].y, Sp.y);
     } else {
@@ -1185,10 +1178,10 @@ __device__ __forceinline__ void queue_pass(const StepParams& P, S& sm, int b, co
         __syncthreads();
     }
     // phase 2: p* (iteration), sampling and the flux of each queued face;
-    // threads 0..ns-1 take the faces above the gate
+    // threads 0..ns-1 take the front of the queue
     for (int t = threadIdx.x; t < ns + nw; t += kThreads) {
-        const bool strong = t < ns;
-        const int i = strong ? t : CAP - 1 - (t - ns);
+        const bool front = t < ns, strong = front && gate_used(P);
+        const int i = front ? t : CAP - 1 - (t - ns);
         const int code = sm.qcode[i];
         const bool active = (code >> 12) & 1;
         int a, c;
@@ -1477,7 +1470,10 @@ __device__ __forceinline__ bool uniform_speeds(const S& sm, int b, const Gas<R>&
 // whole tile whose cells all take the same update (no row of the FP32 form's
 // FP64 update, no force or source).  A barrier; out of line, so that the disturbed tiles'
 // code stays as it is without it (inlined it cost them up to 25%).
-// Undisturbed gas is most of a blast's grid: UNI_MEASURED
+// Undisturbed gas is most of a blast's grid: 4096x2048 per step, start of the
+// growth, FP32 HLL 144 us with every face computed, 72 with these tiles left
+// out (60 where every tile is; one pass over HBM takes 40), FP32 exact solver
+// with the learned start 162 -> 108, FP64 HLL 1.9 -> 0.40 ms.
 // Not used by the FP64 kernels' small tiles but for the exact solver (kSkip): a
 // grid that takes them waits for its disturbed tiles and for the code's fetch,
 // 256x128 HLL 22.7 us per step without the test, 26.2 with it.
@@ -1489,6 +1485,9 @@ template <typename R, int FLUX, int TZ, int TR, bool CACHE, typename S>
 __device__ __noinline__ int uniform_tile(const StepParams& P, int b, bool box, bool plain, int iter)
 {
     S& sm = tile_smem<S>();
+    // (the FP32 form's planar update sums the four faces in an order in which
+    // equal fluxes leave a rounding behind)
+    if (sizeof(R) == 4 && P.geom != 1) return kMixed;
     if (!tile_same<R, TZ, TR>(sm, b, box)) return kMixed;
     const auto& q = sm.qb[b];
     constexpr int QX = S::QX;

@@ -5,7 +5,8 @@ the full path, so the two runs have to agree bit for bit: blasts at rest and
 in moving gas (v_r too), a source, negative zeros, ragged tiles, every flux,
 both precisions, the per-tile and the persistent kernels, the batch.
 
-The FP32 exact solver's inline form against the FP64 one: the update's sixteen
+The FP32 exact solver (plain start value, its queue split by pattern) against
+the FP64 one: the update's sixteen
 products round to 2^-24 each and the pressure subtracts the kinetic energy
 (here at most four times it), p* is found to 1e-6, its flux moves a cell by at
 most half a wave crossing: 2e-5 of the largest value after one step."""
@@ -91,7 +92,7 @@ def test_batch_uniform_tiles_match_the_full_path(precision, flux):
 
 @pytest.mark.parametrize("gamma", [5.0 / 3.0, 1.4, 1.3, 3.0])
 @pytest.mark.parametrize("N,M,persistent", [(16, 16, 0), (65, 33, 0), (130, 70, 1)])
-def test_fp32_inline_exact_solver_matches_fp64(gamma, N, M, persistent):
+def test_fp32_exact_solver_matches_fp64(gamma, N, M, persistent):
     rng = np.random.default_rng(4)
     s = np.exp(rng.uniform(-0.5, 0.5, (N * M, 2)))
     u = rng.uniform(-1.0, 1.0, (N * M, 2))
