@@ -410,6 +410,9 @@ __device__ __forceinline__ bool same_bits(double a, double b)
     return __double_as_longlong(a) == __double_as_longlong(b);
 }
 
+// a > 0 or a positive NaN, on the bit pattern
+__device__ __forceinline__ bool positive_bits(float a) { return __float_as_int(a) > 0; }
+
 // a <= 0, and whether a is a NaN (FP64: on the bit pattern; an FP64
 // comparison holds the FP64 pipe as long as a sum)
 __device__ __forceinline__ bool le_zero(float a) { return a <= 0.0f; }
@@ -986,14 +989,27 @@ __device__ __forceinline__ void face_two(const StepParams& P, S& sm, int b, cons
         }
     }
     if constexpr (FLUX == 0 && sizeof(R) == 4) {
-        // HLL in FP32: both faces in packed arithmetic.  (Warps of one state
-        // on all sides took flux_physical instead after a vote, other values
-        // in the last bits wherever a warp's faces were not all of one state
-        // and 2% of the blast's step: 76.5 against 74.9 us.)
+        // HLL in FP32: both faces in packed arithmetic; or, when both faces
+        // of every active lane of the warp hold one state on all four sides
+        // (one bit pattern, rho > 0, p > 0: undisturbed gas), that state's
+        // physical flux once for both (flux_physical: what the HLL formula
+        // gives up to rounding, its wave speed formed as the formula forms it)
         constexpr int NN = ZF ? 2 : 3, TT = ZF ? 3 : 2;
         float2 F[4], Sp;
-        flux_hll_x2(g, pk(L0[0], L1[0]), pk(L0[1], L1[1]), pk(L0[NN], L1[NN]), pk(L0[TT], L1[TT]), pk(U0[0], U1[0]),
-                    pk(U0[1], U1[1]), pk(U0[NN], U1[NN]), pk(U0[TT], U1[TT]), F, Sp);
+        bool one = two && positive_bits(L0[0]) && positive_bits(L0[1]);
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            one = one && same_bits(L0[k], U0[k]) && same_bits(L0[k], L1[k]) && same_bits(L0[k], U1[k]);
+        if (__all_sync(__activemask(), one)) {
+            float f[4];
+            const float s = flux_physical(g, L0[0], L0[1], L0[NN], L0[TT], f);
+#pragma unroll
+            for (int k = 0; k < 4; k++) F[k] = pk(f[k], f[k]);
+            Sp = pk(s, s);
+        } else {
+            flux_hll_x2(g, pk(L0[0], L1[0]), pk(L0[1], L1[1]), pk(L0[NN], L1[NN]), pk(L0[TT], L1[TT]),
+                        pk(U0[0], U1[0]), pk(U0[1], U1[1]), pk(U0[NN], U1[NN]), pk(U0[TT], U1[TT]), F, Sp);
+        }
         store(a, c, act0, F[0].x, F[1].x, F[2].x, F[3].x, Sp.x);
         if (two) store(a1, c1, act1, F[0].y, F[1].y, F[2].y, F[3].y, Sp.y);
     } else {
@@ -1440,8 +1456,8 @@ __device__ __forceinline__ bool tile_same(const S& sm, int b, bool box)
 }
 
 // The wave speeds of a uniform tile's faces (valid in thread 0), and whether
-// its flux is finite: then every face of one orientation has the same flux
-// and the update's flux differences are exactly zero.  A barrier.
+// its flux is finite and one: then every face of one orientation has the same
+// flux and the update's flux differences are exactly zero.  A barrier.
 template <typename R, int FLUX, typename S>
 __device__ __forceinline__ bool uniform_speeds(const S& sm, int b, const Gas<R>& g, R& sz, R& sr)
 {
@@ -1451,8 +1467,20 @@ __device__ __forceinline__ bool uniform_speeds(const S& sm, int b, const Gas<R>&
     if (threadIdx.x == 0) {
         const R s0 = q[0][2][2 + QX], s1 = q[1][2][2 + QX], s2 = q[2][2][2 + QX], s3 = q[3][2][2 + QX];
         R F[4], G[4];
-        sz = uniform_face<R, FLUX>(g, s0, s1, s2, s3, F);   // z faces: normal v_z
-        sr = uniform_face<R, FLUX>(g, s0, s1, s3, s2, G);   // r faces: normal v_r
+        if constexpr (FLUX == 0 && sizeof(R) == 4) {
+            // face_two takes the physical flux or the HLL formula, warp by
+            // warp: one flux only where the two agree (.x z faces, .y r faces)
+            float2 H[4], sp;
+            flux_hll_x2(g, pk(s0, s0), pk(s1, s1), pk(s2, s3), pk(s3, s2), pk(s0, s0), pk(s1, s1), pk(s2, s3),
+                        pk(s3, s2), H, sp);
+            sz = flux_physical(g, s0, s1, s2, s3, F);
+            sr = flux_physical(g, s0, s1, s3, s2, G);
+            for (int k = 0; k < 4; k++) ok = ok && H[k].x == F[k] && H[k].y == G[k];
+            ok = ok && sp.x == sz && sp.y == sr;
+        } else {
+            sz = uniform_face<R, FLUX>(g, s0, s1, s2, s3, F);   // z faces: normal v_z
+            sr = uniform_face<R, FLUX>(g, s0, s1, s3, s2, G);   // r faces: normal v_r
+        }
         for (int k = 0; k < 4; k++) ok = ok && isfinite(F[k]) && isfinite(G[k]);
         ok = ok && isfinite(sz) && isfinite(sr);
     }
@@ -1470,10 +1498,10 @@ __device__ __forceinline__ bool uniform_speeds(const S& sm, int b, const Gas<R>&
 // whole tile whose cells all take the same update (no row of the FP32 form's
 // FP64 update, no force or source).  A barrier; out of line, so that the disturbed tiles'
 // code stays as it is without it (inlined it cost them up to 25%).
-// Undisturbed gas is most of a blast's grid: 4096x2048 per step, start of the
-// growth, FP32 HLL 144 us with every face computed, 72 with these tiles left
-// out (60 where every tile is; one pass over HBM takes 40), FP32 exact solver
-// with the learned start 162 -> 108, FP64 HLL 1.9 -> 0.40 ms.
+// Undisturbed gas is most of a blast's grid: 4096x2048 per step, with the full
+// path and without, FP32 HLL 148 -> 74 us (61 where every tile is uniform; one
+// pass over HBM takes 40), FP32 exact solver with the learned start 184 -> 109,
+// FP64 HLL 2.20 -> 0.40 ms, FP64 exact solver 2.20 -> 1.31 ms.
 // Not used by the FP64 kernels' small tiles but for the exact solver (kSkip): a
 // grid that takes them waits for its disturbed tiles and for the code's fetch,
 // 256x128 HLL 22.7 us per step without the test, 26.2 with it.

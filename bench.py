@@ -10,13 +10,12 @@ Forms measured (each from the same initial state, warm-up steps first):
   fp64_godunov   plain FP64 path (the reference's solver; the oracle-comparable form)
   fp32_pvrs      FP32 form, Newton for p* from the acoustic (PVRS-type) start value
   fp32_learned   FP32 form, Newton from the learned start value (the headline)
-  fp32_learned_skip  the same with skip_uniform = 1: tiles whose staged cells are
-                 all bit-identical skip the face pass (identical results, checked
-                 bit for bit against fp32_learned; not the headline)
+  fp32_learned_skip  the same with skip_uniform = 1 (no longer a difference: tiles
+                 whose staged cells are all bit-identical always skip the face
+                 pass), checked bit for bit against fp32_learned
   fp64_hll, fp32_hll  the HLL flux in FP64 and in the FP32 form
-  fp32_hll_skip  fp32_hll with skip_uniform = 1 (uniform tiles skip the face
-                 pass; face pairs of undisturbed gas skip the reconstruction),
-                 checked bit for bit against fp32_hll
+  fp32_hll_skip  fp32_hll with skip_uniform = 1, as above, checked bit for bit
+                 against fp32_hll
 The FP32 forms report their density and pressure L1 error against the FP64
 run after the same steps, and Newton statistics (mean/max iterations,
 fallback rate).  The headline `value` is the form named in config.form.

@@ -144,21 +144,19 @@ typedef struct ast_config {
        bulk-tensor copies, double-buffered; the learned start value by f16
        tensor-core tiles); 0 = one CTA per tile.  The same arithmetic per
        face and cell.  The FP64 solver with 1 runs the persistent tile
-       kernel for the HLL family on grids of at least two 32x16 tiles per
-       SM, one CTA per tile otherwise (the exact solver: one CTA per tile);
+       kernel on grids of at least two 32x16 tiles per SM (the exact solver:
+       eight), one CTA per tile otherwise;
        the raw entry points always use one CTA per tile (default 1)         */
     int32_t persistent;
-    /* 1: tiles whose staged cells (tile and two-cell halo, ghosts included)
-       all hold the same four values, bit for bit, skip the face pass: every
-       face of such a tile has the same flux, so the flux differences of the
-       update are exactly zero, and the update runs on zero fluxes; the wave
+    /* accepted (0 or 1) and without effect: tiles whose staged cells (tile and
+       two-cell halo, ghosts included) all hold the same four values, bit for
+       bit, always skip the face pass.  Every face of such a tile has the same
+       flux, so the flux differences of the update are exactly zero; the wave
        speeds come from one face of each orientation.  The results are
        identical to the full computation.  Tiles near the fixed region, runs
-       with region_select, and uniform states whose flux is not finite take
-       the full path.  With HLL in the FP32 form it also lets face pairs whose
-       five stencil cells are one state in a whole warp skip the
-       reconstruction (the same results; faster where the gas is undisturbed,
-       some per cent slower where every face is disturbed) (default 0)      */
+       with region_select, FP32 planar runs, and uniform states whose flux is
+       not finite (FP32 HLL: not the same by the formula and as the state's own
+       flux) take the full path (default 0)                                 */
     int32_t skip_uniform;
     /* polls of a bulk tile copy's barrier before the FP32 persistent kernels
        report AST_ST_TIMEOUT (the copy is then waited for with the long
