@@ -134,9 +134,12 @@ __device__ __forceinline__ RPre<double> godunov_pre64(const Gas<double>& g, doub
         return q;
     }
     // Urz = -2 cII/(gamma-1) (1 - x^gm), x = pI/pII: FP32 decides unless Udf
-    // lies within 1e-4 of it
+    // lies within 1e-4 of it.  ln x to FP32 precision over all of x: from x
+    // itself, near 1 (where FP32 no longer tells x from 1) from 1 - x (which
+    // in turn loses a small x)
     const double x = o.mul(q.pI, o.rcp(q.pII));
-    const float y = -expm1f((float)g.gm * log1pf(-low_float(o.sub(1.0, x))));
+    const float xf = low_float(x), lx = xf < 0.5f ? logf(xf) : log1pf(-low_float(o.sub(1.0, x)));
+    const float y = -expm1f((float)g.gm * lx);
     const float zf = -low_float(k2) * low_float(q.cII) * y, uf = low_float(q.Udf);
     const bool sure = fabsf(uf - zf) > 1e-4f * fabsf(zf) && y < 1.0f;
     if (sure && uf > zf) {

@@ -1,0 +1,109 @@
+"""The FP64 exact solver's wave patterns on single faces: the pattern decides
+the formulas, so faces are placed on both sides of its thresholds, at pressure
+ratios up to 1e12, in both orders of the sides and both orientations, and one
+step is compared with the oracle.
+
+Each test face is the middle one of four cells (A A B B) in a row of such
+groups, first order, so a cell next to it changes by this face's flux alone
+(its other neighbour equals it)."""
+import numpy as np
+import pytest
+
+import pyoracle as O
+from asteriy_2d_gb300 import abi as A
+from asteriy_2d_gb300 import problems, solver
+
+pytestmark = pytest.mark.gpu
+
+
+def line(faces, along_z):
+    """The groups of `faces` ((rho, p, un) of the lower and of the upper side)
+    along z or r, four cells wide across: a configuration and its state."""
+    n = 4 * len(faces)
+    cfg = problems.blast_config(n if along_z else 4, 4 if along_z else n, flux=A.FLUX_GODUNOV)
+    cfg.recon, cfg.geom = A.RECON_NONE, A.GEOM_PLANAR
+    cfg.x_min, cfg.x_max, cfg.y_max = 0.0, float(cfg.N - 1), float(cfg.M)   # dx = dy = 1
+    cfg.p_floor = 1e-300
+    for side in range(4):
+        A.set_bc(cfg, side, A.BC_OUTFLOW)
+    q = np.repeat(np.array(faces, dtype=np.float64).reshape(-1, 3), 2, axis=0)
+    k = np.arange(cfg.N * cfg.M)
+    q = q[k % cfg.N if along_z else k // cfg.N]
+    s, u = q[:, :2].copy(), np.zeros((len(k), 2))
+    u[:, 0 if along_z else 1] = q[:, 2]
+    return cfg, s, u
+
+
+def step(cfg, s, u, dt):
+    cfg.collect_stats = 1
+    with solver.Solver(cfg) as S:
+        S.set_state(s, u)
+        S.set_clock(dt)
+        S.step(1)
+        return (*S.get_state(), S.clock()[0], S.stats())
+
+
+def worst(cfg, s, u, dt):
+    """The largest difference from the oracle's step, each cell by its own
+    scales: rho, p + rho u^2, |u| + c."""
+    gs, gu, tdo, _ = step(cfg, s, u, dt)
+    os_, ou, otdo, _, _, _ = O.run(cfg, s, u, 1, T_do=dt)
+    q = np.sum(ou * ou, 1)
+    e = max(np.max(np.abs(gs[:, 0] - os_[:, 0]) / os_[:, 0]),
+            np.max(np.abs(gs[:, 1] - os_[:, 1]) / (os_[:, 1] + os_[:, 0] * q)),
+            np.max(np.abs(gu - ou) / (np.sqrt(q) + np.sqrt(cfg.gamma * os_[:, 1] / os_[:, 0]))[:, None]))
+    return e, abs(tdo - otdo) / otdo
+
+
+def threshold_faces(ga, cII):
+    """Faces at a fraction f beside the threshold between two rarefactions (f <
+    0) and shock and rarefaction, in the frame in which the sampled state is
+    the one between the low-pressure side's wave and the contact."""
+    g1, g2 = ga - 1.0, ga + 1.0
+    gm = g1 / (2 * ga)
+    out = []
+    for ratio in (1e2, 1e4, 1e6, 1e7, 1e8, 1e9, 1e10, 1e12):
+        for dens in (1.0, 30.0):
+            rI, rII = dens, 1.0
+            pII = cII * cII * rII / ga
+            pI = pII / ratio
+            cI = np.sqrt(ga * pI / rI)
+            Urz = -2 * cII / g1 * (1 - ratio ** -gm)
+            for f in (-3e-2, -3e-3, -3e-4, 3e-4, 7e-4, 1e-3, 3e-3, 6e-3, 1e-2, 1.5e-2, 2.5e-2, 5e-2):
+                U = Urz * (1 - f)
+
+                def res(p):    # rises with p
+                    fI = (p - pI) / np.sqrt(rI * (0.5 * g2 * p + 0.5 * g1 * pI)) if p > pI else \
+                        2 * cI / g1 * ((p / pI) ** gm - 1)
+                    return fI + 2 * cII / g1 * ((p / pII) ** gm - 1) - U
+
+                lo, hi = 1e-6 * pI, pII
+                for _ in range(200):
+                    p = np.sqrt(lo * hi)
+                    lo, hi = (lo, p) if res(p) > 0 else (p, hi)
+                a = np.sqrt(rI * (0.5 * g2 * p + 0.5 * g1 * pI))
+                if p > pI:
+                    u, edge = -(p - pI) / a, -a / rI
+                else:
+                    u = -2 * cI / g1 * ((p / pI) ** gm - 1)
+                    edge = u - cI * (p / pI) ** gm
+                w = 0.5 * (u + edge)            # (enI = 0 so far)
+                I, II = (rI, pI, -w), (rII, pII, -U - w)
+                out.append((I, II))
+                out.append(((rII, pII, U + w), (rI, pI, w)))
+    return out
+
+
+# p* is found to the tolerance in velocity, 1e-9 cII: relative to p_I that is
+# 1e-3 at most (c_I >= 1e-6 cII), and the low-pressure cell changes by at most
+# 1e-7 of itself here (dt c_I/dx): 1e-10.  A face in the wrong pattern is
+# off by tenths of the change of the cells, 1e-9 and more.
+@pytest.mark.parametrize("gamma", [5.0 / 3.0, 1.4, 4.0 / 3.0])
+@pytest.mark.parametrize("along_z", [True, False])
+def test_patterns_at_large_pressure_ratios(gamma, along_z):
+    cII = 10.0
+    cfg, s, u = line(threshold_faces(gamma, cII), along_z)
+    cfg.gamma, cfg.riemann_tol = gamma, 1e-9 * cII
+    err, terr = worst(cfg, s, u, 0.1 / (np.max(np.abs(u)) + cII))
+    assert err <= 1e-10, err
+    assert terr <= 1e-9, terr
