@@ -331,6 +331,8 @@ __device__ __forceinline__ double newton_p64(const Gas<double>& g, const RPre<do
         const double p = pn;
         k++;
         const double qI = fma(gI, p, g.gm), qII = fma(gII, p, g.gm);
+        // p far above both pressures (qII <= qI): FP32 does not hold the derivative's terms
+        if (__double2hiint(qI) >= ((1023 + 100) << 20)) return solve_exact(g, q, rc);
         const double sI = o.rsqrt(qI), sII = o.rsqrt(qII);
         const double f = fma(o.mul(o.sub(p, q.pI), kI), sI, fma(o.mul(o.sub(p, q.pII), kII), sII, flip(q.Udf)));
         const float uI = low_float(sI), uII = low_float(sII);
