@@ -133,6 +133,11 @@ __device__ __forceinline__ RPre<double> godunov_pre64(const Gas<double>& g, doub
         q.pattern = 0;
         return q;
     }
+    // equal pressures (a contact, or two equal rarefactions): Urz = 0 >= Udf
+    if (bits(dp) == 0) {
+        q.pattern = 1;
+        return q;
+    }
     // Urz = -2 cII/(gamma-1) (1 - x^gm), x = pI/pII: FP32 decides unless Udf
     // lies within 1e-4 of it.  ln x to FP32 precision over all of x: from x
     // itself, near 1 (where FP32 no longer tells x from 1) from 1 - x (which
@@ -146,7 +151,7 @@ __device__ __forceinline__ RPre<double> godunov_pre64(const Gas<double>& g, doub
         q.pattern = 2;
         return q;
     }
-    q.Urz = o.mul(o.mul(-k2, q.cII), o.sub(1.0, pow_gm(g, x)));
+    q.Urz = o.mul(o.mul(k2, q.cII), o.sub(pow_gm(g, x), 1.0));   // a zero is +0, as key() needs it
     q.pattern = (sure || key(q.Udf) <= key(q.Urz)) ? 1 : 2;
     return q;
 }

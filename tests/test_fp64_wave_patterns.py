@@ -121,3 +121,24 @@ def test_two_shocks_far_above_both_pressures(low, high, along_z):
     err, terr = worst(cfg, s, u, 0.05 / np.max(np.abs(u)))
     assert err <= 1e-12, err
     assert terr <= 1e-12, terr
+
+
+# faces with equal pressures and equal normal velocities (contacts) take the
+# closed form: nothing iterates, and the gas stays as it is but for the
+# density's advection (the oracle's step to a few roundings)
+@pytest.mark.parametrize("recon", [A.RECON_NONE, A.RECON_MINMOD])
+@pytest.mark.parametrize("p", [0.1, 1.0 / 3.0, 1.0, 7.3])
+@pytest.mark.parametrize("v", [0.0, 0.3])
+def test_contacts_take_the_closed_form(recon, p, v):
+    cfg = problems.blast_config(37, 21, flux=A.FLUX_GODUNOV)
+    cfg.recon, cfg.geom = recon, A.GEOM_PLANAR
+    for side in range(4):
+        A.set_bc(cfg, side, A.BC_OUTFLOW)
+    K = cfg.N * cfg.M
+    s = np.stack([np.exp(np.random.default_rng(1).uniform(-1.0, 1.0, K)), np.full(K, p)], 1)
+    u = np.stack([np.full(K, v), np.full(K, -v)], 1)
+    stats = step(cfg, s, u, 1e-4)[3]
+    assert stats["bisect_calls"] == stats["newton_calls"] == 0, stats
+    err, terr = worst(cfg, s, u, 1e-4)
+    assert err <= 1e-13, err
+    assert terr <= 1e-13, terr
