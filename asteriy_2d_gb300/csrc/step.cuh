@@ -762,14 +762,20 @@ __device__ __forceinline__ double exact_same_state(const Gas<double>& g, double 
     return is_nan(S) ? g.eps8 : larger_speed(S, g.eps8);
 }
 
-// whether the two sides of a face hold equal values (FP64: the same bits)
+// whether the two sides of a face hold equal values (FP64: the same bits, or a
+// zero velocity of either sign: gas at rest beside its mirror image)
 __device__ __forceinline__ bool same_state(const float L[4], const float U[4])
 {
     return L[0] == U[0] && L[1] == U[1] && L[2] == U[2] && L[3] == U[3];
 }
+__device__ __forceinline__ bool same_or_zero(double a, double b)
+{
+    const long long i = d64::bits(a), j = d64::bits(b);
+    return i == j || ((i | j) & ~d64::kSign) == 0;
+}
 __device__ __forceinline__ bool same_state(const double L[4], const double U[4])
 {
-    return same_bits(L[0], U[0]) && same_bits(L[1], U[1]) && same_bits(L[2], U[2]) && same_bits(L[3], U[3]);
+    return same_bits(L[0], U[0]) && same_bits(L[1], U[1]) && same_or_zero(L[2], U[2]) && same_or_zero(L[3], U[3]);
 }
 
 // Whether face (a, c) of orientation ZF belongs to an updated cell

@@ -142,3 +142,18 @@ def test_contacts_take_the_closed_form(recon, p, v):
     err, terr = worst(cfg, s, u, 1e-4)
     assert err <= 1e-13, err
     assert terr <= 1e-13, terr
+
+
+# gas at rest beside its mirror image at the axis (v_r = +0 and -0 on the two
+# sides of that face) stays at rest, exactly, and takes the identical-state path
+@pytest.mark.parametrize("recon", [A.RECON_NONE, A.RECON_MINMOD])
+@pytest.mark.parametrize("p", [0.1, 1.0, 7.3, 10.0])
+def test_gas_at_rest_at_a_reflecting_axis_stays_at_rest(recon, p):
+    cfg = problems.blast_config(37, 21, flux=A.FLUX_GODUNOV)
+    cfg.recon = recon
+    K = cfg.N * cfg.M
+    s, u = np.stack([np.ones(K), np.full(K, p)], 1), np.zeros((K, 2))
+    gs, gu, _, stats = step(cfg, s, u, 1e-3)
+    assert np.all(gu == 0.0), np.max(np.abs(gu))
+    assert len(np.unique(gs[:, 0])) == len(np.unique(gs[:, 1])) == 1
+    assert stats["bisect_calls"] == stats["newton_calls"] == 0, stats
