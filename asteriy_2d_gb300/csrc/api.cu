@@ -66,6 +66,8 @@ __global__ void funk_time_kernel(double* T, double* T_do, double* TT, int* i)
 int ast::cuda_fail(cudaError_t e, const char* what)
 {
     g_last_error = std::string(what) + ": " + cudaGetErrorString(e);
+    // reported here: the runtime's copy must not turn up in the next call's launch check
+    (void)cudaGetLastError();
     return AST_ERR_CUDA;
 }
 
