@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 
     // the planar update (kernel.cu:2201-2290)
     const double T_do = *T_do_p;
-    const double ntz = -T_do / P.dx, ntr = -T_do / P.dy;
+    const double ntz = -T_do / P.dx, zr = P.dx / P.dy;
     const bool body = P.body_force && x > P.body_lo && x < P.body_hi;
 #pragma unroll
     for (int it = 0; it < kCells; it++) {
@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(kThreads, 2)
         if (body) Q2 = (row_y(m) >= P.body_rsplit) ? -P.body_amp * c.rho : P.body_amp * c.rho;
         int nrho = 0, np = 0;
         unsigned status = 0;
-        update_cell64(P.g, P.p_floor, false, in, f, T_do, ntz, ntr, 0.0, body, Q2, false, 0.0, 0.0, nrho, np, status, o);
+        update_cell64(P.g, P.p_floor, false, in, f, T_do, ntz, zr, 0.0, body, Q2, false, 0.0, 0.0, nrho, np, status, o);
         s2[k] = make_double2(o[0], o[1]);
         u2[k] = make_double2(o[2], o[3]);
     }

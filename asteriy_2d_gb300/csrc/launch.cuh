@@ -333,6 +333,7 @@ inline void fill_step_params(StepParams& P, const ast_config& c)
     P.y_min = (c.y_max / (2.0 * c.M));
     P.krit_dx = c.cfl * P.dx;
     P.krit_dy = c.cfl * P.dy;
+    P.zr = P.dx / P.dy;
     P.dt_cap = c.dt_cap;
     P.p_floor = c.p_floor;
     P.gamma = c.gamma;
