@@ -50,16 +50,26 @@ inline int sm_count()
 
 // early: the kernel may start while the one before it in the stream still runs:
 // its CTAs take free places on the SMs, do what needs none of its results and
-// wait (after_previous_step).  That saves the launch, but the CTAs are placed
-// around the last step's.  So it is for persistent kernels with more tiles than
-// CTAs, which fill every place all the same (FP32 HLLC wind 1537x771 41.2 ->
-// 36.9 us per step with the CTA's own first tile, HLL blast 4096x2048 75.5 ->
-// 73.8), and for grids (start_early) of many CTAs a place (FP64 exact solver
-// 1021x509 178 -> 173 us) or so few that each has an SM of its own (FP64 HLL
-// 64x32, 10 steps and the copies, 256 -> 236 us).  In between two CTAs shared an
-// SM while others stood empty: FP64 HLL 256x128 (128 CTAs) 23.0 -> 32.3 us per
-// step.  Not for the batch kernels: no gain over a batch's many tiles.
-inline bool start_early(long long ctas) { return 2 * ctas <= sm_count() || ctas >= 8 * sm_count(); }
+// wait (after_previous_step).  That saves 1 to 2 us of launch, but the CTAs are
+// placed around the last step's, two on one SM while others stand empty.  So it
+// is for steps launched one by one only: under capture there is no launch to
+// save, and the placement alone made FP32 HLL 1024x512 18.5 -> 24.9 us per step,
+// FP64 HLL 192x96 22.6 -> 28.5, the 4096x2048 learned start 107.4 -> 109.5.  And
+// for grids of few or many CTAs a place (us per step, ten steps, without and with):
+//   small (at most 0.4 CTAs per SM): FP64 HLL 64x32 26.4 -> 24.4, 160x80 (50
+//   CTAs) 27.0 -> 24.8; 192x96 (72) 25.3 -> 26.8, 256x128 (128) 25.2 -> 34.0;
+//   from 8 CTAs per SM: FP64 exact solver 900x450 (1653) 174.9 -> 173.2,
+//   1024x512 (2048) 197.6 -> 193.4; 700x350 (968) 143 -> 150.
+// The persistent kernels' lines are in launch_tma_t.  Not for the batch kernels: no
+// gain over a batch's many tiles.
+inline bool start_early(long long ctas) { return 5 * ctas <= 2 * sm_count() || ctas >= 8 * sm_count(); }
+inline bool capturing(cudaStream_t st)
+{
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) == cudaSuccess) return cs != cudaStreamCaptureStatusNone;
+    (void)cudaGetLastError();   // the launch itself will report it
+    return true;
+}
 template <typename... P, typename... A>
 cudaError_t launch_after(bool early, void (*k)(P...), dim3 grid, size_t smem, cudaStream_t st, const A&... args)
 {
@@ -72,7 +82,7 @@ cudaError_t launch_after(bool early, void (*k)(P...), dim3 grid, size_t smem, cu
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     lc.attrs = &at;
-    lc.numAttrs = early ? 1 : 0;
+    lc.numAttrs = early && !capturing(st) ? 1 : 0;
     return cudaLaunchKernelEx(&lc, k, args...);
 }
 
@@ -141,8 +151,14 @@ int launch_tma_t(const StepParams& P, const CUtensorMap& tin, const CUtensorMap&
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k, kThreads, smem);
         return e == cudaSuccess ? AST_OK : cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
     }
-    const long long tiles = (long long)((P.N + kTmaTZ - 1) / kTmaTZ) * ((P.M + kTmaTR - 1) / kTmaTR);
-    e = launch_after(tiles > grid || 2 * grid <= sm_count(), k, grid, smem, st, P, tin, tout);
+    // early from 3.5 tiles a CTA, where a late CTA's tiles go to the others (FP32
+    // HLLC wind 1537x771, 3.9 tiles a CTA, 39.9 -> 39.5 us per step, FP64 HLL
+    // 1500x750, 7.3, 120.9 -> 118.0; but FP32 HLL blast 1280x640, 2.6, 23.5 ->
+    // 24.9, and 1024x512, 1.7, 22.0 -> 26.4), and on half the SMs at most (FP32 HLL
+    // 256x128, 64 CTAs, 18.8 -> 16.6; 512x256, 256 CTAs, 17.1 -> 17.9)
+    const int rows = P.band_hi > 0 ? P.band_hi - P.band_lo : (P.M + kTmaTR - 1) / kTmaTR;
+    const long long tiles = (long long)((P.N + kTmaTZ - 1) / kTmaTZ) * rows;
+    e = launch_after(2 * tiles >= 7LL * grid || 2 * grid <= sm_count(), k, grid, smem, st, P, tin, tout);
     return e == cudaSuccess ? AST_OK : cuda_fail(e, "persistent step kernel launch");
 }
 
