@@ -100,7 +100,6 @@ struct __align__(16) StepParams {
     long long plane;               // SoA plane size in elements
     double x_min, dx, y_min, dy;
     double krit_dx, krit_dy;       // cfl*dx and cfl*dy
-    double zr;                     // dx/dy
     double dt_cap, p_floor;
     double gamma, tol;
     int max_iter;
@@ -157,6 +156,7 @@ struct __align__(16) StepParams {
     long long rec_cap;
     int rec_every;                 // record on steps with step % rec_every == 0
     double rec_gate;               // record faces with wave strength above this
+    double zr;                     // dx/dy
 };
 
 // the gas constants of the arithmetic R
@@ -536,12 +536,11 @@ __device__ __forceinline__ void update_cell64(const Gas<double>& g, double p_flo
     out[0] = rho2; out[1] = p2; out[2] = vz2; out[3] = vr2;
 }
 
-// The FP32 kernels' FP64 update of the four cell rows next to the axis
-// (axisymmetric), the two orientations added one by one (ntr = -T_do/dy): its
-// results are rounded to FP32, where another form of the sums shows in one value
-// in some 1e8 (runs of the 1537x771 wind then part after 650 steps), so this one
-// stays as it is.
-__device__ __forceinline__ void update_cell_axis(const Gas<double>& g, double p_floor, const float in[4],
+// The FP32 kernels' FP64 update of the four cell rows next to the axis, the two
+// orientations added one by one (ntr = -T_do/dy): its results are rounded to FP32,
+// where another form of the sums shows in one value in some 1e8 (runs of the
+// 1537x771 wind then part after 650 steps), so this one stays as it is.
+__device__ __forceinline__ void update_cell_axis(const Gas<double>& g, double p_floor, bool axisym, const float in[4],
                                                  const float f[4][4], double T_do, double ntz, double ntr, double ty,
                                                  bool body, double Q2, int& nrho, int& np, unsigned& status,
                                                  float out[4])
@@ -557,11 +556,14 @@ __device__ __forceinline__ void update_cell_axis(const Gas<double>& g, double p_
         const double fz = o.sub((double)f[k][0], (double)f[k][1]), fr = o.sub((double)f[k][3], (double)f[k][2]);
         U[k] = fma(ntr, fr, fma(ntz, fz, U[k]));
     }
-    const double w = flip(o.mul(ty, mr1));
-    U[0] = o.add(w, U[0]);
-    U[1] = fma(w, vz1, U[1]);
-    U[2] = fma(w, vr1, U[2]);
-    U[3] = fma(flip(o.mul(ty, vr1)), o.add(E1, p1), U[3]);
+    if (axisym) {
+        branch();
+        const double w = flip(o.mul(ty, mr1));
+        U[0] = o.add(w, U[0]);
+        U[1] = fma(w, vz1, U[1]);
+        U[2] = fma(w, vr1, U[2]);
+        U[3] = fma(flip(o.mul(ty, vr1)), o.add(E1, p1), U[3]);
+    }
     if (body) {
         branch();
         U[2] = fma(T_do, Q2, U[2]);
@@ -1682,8 +1684,9 @@ __device__ __forceinline__ void tile_body(const StepParams& P, S& sm, int b, con
         const bool body = P.body_force && n >= P.body_nlo && n <= P.body_nhi;
         if (body) Q2 = (m0 + row >= P.body_mlo) ? -P.body_amp * (double)in[0] : P.body_amp * (double)in[0];
         if constexpr (sizeof(R) == 4) {
-            update_cell_axis(P.gd, P.p_floor, in, f, T_do, K.ntz, K.ntr, T_do / sm.ydrow[row], body, Q2, acc.nrho,
-                             acc.np, acc.rc.status, o);
+            const double ty = (P.geom == 1) ? T_do / sm.ydrow[row] : 0.0;
+            update_cell_axis(P.gd, P.p_floor, P.geom == 1, in, f, T_do, K.ntz, K.ntr, ty, body, Q2, acc.nrho, acc.np,
+                             acc.rc.status, o);
         } else {
             // the neutral-coupling source (the FP32 form adds it in
             // neutral_kernel after the step)

@@ -415,8 +415,8 @@ __device__ __forceinline__ void sweep_strip(const StepParams& P, const StepConst
                         if (x > P.body_lo && x < P.body_hi)
                             Q2 = (y >= P.body_rsplit) ? -P.body_amp * (double)w0[0] : P.body_amp * (double)w0[0];
                     }
-                    update_cell_axis(P.gd, P.p_floor, w0, f, T_do, K.ntz, K.ntr, T_do / y, P.body_force != 0, Q2,
-                                     acc.nrho, acc.np, acc.rc.status, o);
+                    update_cell_axis(P.gd, P.p_floor, true, w0, f, T_do, K.ntz, K.ntr, T_do / y, P.body_force != 0,
+                                     Q2, acc.nrho, acc.np, acc.rc.status, o);
                 } else {
                     const float y = P.y_minf + (float)m * P.dyf;
                     float Q2 = 0.0f;
