@@ -814,14 +814,18 @@ __device__ __forceinline__ bool same_state(const float L[4], const float U[4])
 {
     return L[0] == U[0] && L[1] == U[1] && L[2] == U[2] && L[3] == U[3];
 }
-__device__ __forceinline__ bool same_or_zero(double a, double b)
-{
-    const long long i = d64::bits(a), j = d64::bits(b);
-    return i == j || ((i | j) & ~d64::kSign) == 0;
-}
 __device__ __forceinline__ bool same_state(const double L[4], const double U[4])
 {
-    return same_bits(L[0], U[0]) && same_bits(L[1], U[1]) && same_or_zero(L[2], U[2]) && same_or_zero(L[3], U[3]);
+    // (one word, no branches: lanes that part here would not meet again before
+    // the solver)
+    unsigned long long d = 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const unsigned long long i = __double_as_longlong(L[k]), j = __double_as_longlong(U[k]);
+        const bool zeros = k >= 2 && ((i | j) << 1) == 0;
+        d |= zeros ? 0ull : i ^ j;
+    }
+    return d == 0;
 }
 
 // Whether face (a, c) of orientation ZF belongs to an updated cell
