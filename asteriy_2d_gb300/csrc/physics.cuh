@@ -640,9 +640,10 @@ __device__ __forceinline__ double flux_hllc(const Gas<double>& g, double rL, dou
 // HLLC_2d_Korolkov_b_s, Gas_Dinamic.cu:1660-1808, metod 2, W = 0): Q is a
 // density carried by the flow, its flux Q u on the upwind side and, in a
 // star region, the side's flux corrected by S (Q* - Q) with
-// Q* = Q (S - u)/(S - SM).  The wave speeds and the contact speed are
-// flux_hllc's, formed by the same expressions, so the scalar moves with
-// that solver's mass flux.
+// Q* = Q (S - u)/(S - SM).  The wave speeds and the contact speed are those
+// of flux_hllc_ref, by its expressions; the FP64 gas flux forms them otherwise
+// (sound_max, flux_star), so the scalar moves with that solver's mass flux to
+// rounding.
 template <typename R>
 __device__ __forceinline__ R flux_hllc_q(const Gas<R>& g, R rL, R pL, R u1, R QL, R rR, R pR, R u2, R QR)
 {

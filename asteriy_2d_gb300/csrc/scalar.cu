@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kScalarThreads) scalar_kernel(StepParams P, co
     const double f_l = face_q<FLUX, RECON, true>(P, g, zc[0], zc[1], zc[2], zc[3], zq[0], zq[1], zq[2], zq[3]);
     const double f_b = face_q<FLUX, RECON, false>(P, g, rc[0], rc[1], zc[2], rc[2], rq[0], rq[1], zq[2], rq[2]);
     const double f_t = face_q<FLUX, RECON, false>(P, g, rc[1], zc[2], rc[2], rc[3], rq[1], zq[2], rq[2], rq[3]);
-    // the density's update form (update_cell)
+    // the density's update, the reference's expressions
     const double T_do = (P.clock != nullptr) ? *(volatile double*)&P.clock->T_do : *P.T_do_ptr;
     const double tdv = T_do / (P.dx * P.dy);
     const double f12 = f_r, f14 = -f_l, f13 = -f_b, f15 = f_t;

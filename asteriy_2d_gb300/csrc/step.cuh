@@ -490,9 +490,9 @@ __device__ __forceinline__ void update_cell(const StepParams& P, float ga, float
 // the signs are read off the bit patterns.  Each conserved value is rounded once
 // at its own size (twice with the axisymmetric source), as by the expressions
 // above.  Rms error of a step against long double, relative to that of plain
-// FP64 sums: density 1.00, momenta 1.01, pressure 0.95 (HLLC, planar, Mach 1);
+// FP64 sums: density 1.01, velocities 1.01, pressure 0.91 (HLLC, planar, Mach 1);
 // 1.39, 1.32 and 1.15 with the two orientations added one after the other to
-// rounded momenta, at the same speed.  `body`, `source`: whether Q2, and Sz and
+// rounded momenta, 32000x400 HLLC 15.85 -> 15.67 ms for four steps.  `body`, `source`: whether Q2, and Sz and
 // Sr, are to be added.
 __device__ __forceinline__ void update_cell64(const Gas<double>& g, double p_floor, bool axisym, const double in[4],
                                               const double f[4][4], double T_do, double ntz, double zr, double ty,
@@ -726,16 +726,14 @@ __device__ __forceinline__ void record_face(const StepParams& P, const Gas<R>& g
 // ------------------------------------------------------------------ face passes
 // The reconstructed states on both sides of face (a, c) of orientation ZF
 // (minmod on the staged cells when RECON and the face is in the
-// high-order region `hi`; the cell values otherwise).  When the four
+// high-order region `hi`; the cell values otherwise).  FP64, when the four
 // stencil cells of every variable hold the same bits in all the warp's
-// active lanes (undisturbed gas), the limited slope is +0 (x - x = +0, and
-// minmod of zeros, or of the NaN of inf - inf, is +0), so the face values
-// are the cell's value plus +0 and the upper cell's value: taken without
-// the minmod arithmetic, the same bits.  (At step 1000 of the 4096x2048
-// blast about nine faces in ten are such: the exact-solver step 0.189 ->
-// 0.175 ms in FP32, 11.45 -> 10.44 ms in FP64; where the gas is disturbed
-// everywhere the test costs about 5%.)  Returns whether the warp took
-// that path (then the two sides of every lane's face are equal).
+// active lanes (undisturbed gas beside a disturbed tile's): the limited slope
+// is +0 (x - x = +0, and minmod of zeros, or of the NaN of inf - inf, is +0), so
+// the face values are the cell's value plus +0 and the upper cell's value:
+// taken without the minmod arithmetic, the same bits.  Returns whether the
+// warp took that path (then the two sides of every lane's face are equal);
+// FP32 never does (its uniform tiles skip the faces altogether).
 template <typename R, bool RECON, bool ZF, bool VOTE = true, typename S>
 __device__ __forceinline__ bool face_states(const StepParams& P, const S& sm, int b, int a, int c, bool hi, R L[4],
                                             R U[4])
@@ -1555,11 +1553,12 @@ __device__ __forceinline__ bool uniform_speeds(const S& sm, int b, const Gas<R>&
 // whole tile whose cells all take the same update (no row of the FP32 form's
 // FP64 update, no force or source).  A barrier; out of line, so that the disturbed tiles'
 // code stays as it is without it (inlined it cost them up to 25%).
-// Undisturbed gas is most of a blast's grid: 4096x2048 per step, with the full
-// path and without, FP32 HLL 148 -> 74 us (61 where every tile is uniform; one
-// pass over HBM takes 40), FP32 exact solver with the learned start 184 -> 109,
-// FP64 HLL 2.20 -> 0.40 ms, FP64 exact solver 2.20 -> 1.31 ms.
-// Not used by the FP64 kernels' small tiles but for the exact solver (kSkip): a
+// Undisturbed gas is most of a blast's grid: 4096x2048 grown to a third of the
+// radius, per step, with the full path and without, FP32 HLL 148 -> 73 us (62
+// where every tile is uniform; one pass over HBM takes 40), FP32 exact solver with
+// the learned start 184 -> 107, FP64 HLL 2.20 -> 0.40 ms, FP64 exact solver 2.20 ->
+// 1.26 ms.
+// Not used by the FP64 kernels' small tiles but for the exact solver (skips_uniform): a
 // grid that takes them waits for its disturbed tiles and for the code's fetch,
 // 256x128 HLL 22.7 us per step without the test, 26.2 with it.
 enum { kMixed = 0, kUniform = 1, kStored = 2 };

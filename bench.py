@@ -49,8 +49,8 @@ REF_BUDGET_S = 150.0    # reference arm: seconds of timed host work
 # (dram__bytes_read.sum + dram__bytes_write.sum); the default grid only
 MEASURED_TRAFFIC = {"fp32_learned": 134.40e6 + 94.28e6, "fp32_hll": 134.29e6 + 93.31e6}
 MEASURED_TRAFFIC_SOURCE = ("a constant, not measured in this run: ncu dram__bytes_read.sum + dram__bytes_write.sum "
-                           "of one launch (profiles/step_kernel_tma_fp32_learned_godunov_4096x2048.md, the capture "
-                           "of the current kernel)")
+                           "of one launch (profiles/step_kernel_tma_fp32_learned_godunov_4096x2048.md, captured "
+                           "before uniform tiles skipped their faces)")
 
 
 def peaks():
