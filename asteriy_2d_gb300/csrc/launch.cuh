@@ -52,17 +52,18 @@ inline int sm_count()
 // its CTAs take free places on the SMs, do what needs none of its results and
 // wait (after_previous_step).  That saves 1 to 2 us of launch, but the CTAs are
 // placed around the last step's, two on one SM while others stand empty.  So it
-// is for steps launched one by one only: under capture there is no launch to
-// save, and the placement alone made FP32 HLL 1024x512 18.5 -> 24.9 us per step,
-// FP64 HLL 192x96 22.6 -> 28.5, the 4096x2048 learned start 107.4 -> 109.5.  And
-// for grids of few or many CTAs a place (us per step, ten steps, without and with):
-//   small (at most 0.4 CTAs per SM): FP64 HLL 64x32 26.4 -> 24.4, 160x80 (50
-//   CTAs) 27.0 -> 24.8; 192x96 (72) 25.3 -> 26.8, 256x128 (128) 25.2 -> 34.0;
-//   from 8 CTAs per SM: FP64 exact solver 900x450 (1653) 174.9 -> 173.2,
-//   1024x512 (2048) 197.6 -> 193.4; 700x350 (968) 143 -> 150.
+// is for grids of few or many CTAs a place, and in captured blocks of steps, which
+// have no launch to save, for the smallest only.  Us per step without and with,
+// a CTA per tile:
+//   ten steps launched one by one: FP64 HLL blast 64x32 (8 CTAs) 26.4 -> 24.4,
+//   160x80 (50) 27.0 -> 24.8, wind 183x81 (72) 242.9 -> 227.5 for eight steps,
+//   blast 192x96 (72) 25.3 -> 26.8, 256x128 (128) 25.2 -> 34.0; FP64 exact solver
+//   700x350 (968) 143 -> 150, 900x450 (1653) 174.9 -> 173.2, 1024x512 (2048) 197.6 ->
+//   193.4: up to half the SMs and from 8 CTAs per SM;
+//   captured: FP64 HLLC wind 160x80 26.5 -> 26.0, 176x88 (66 CTAs) 25.5 -> 29.7, HLL
+//   192x96 22.6 -> 28.5; exact solver 900x450 202.4 -> 206.8: up to 0.4 per SM.
 // The persistent kernels' lines are in launch_tma_t.  Not for the batch kernels: no
 // gain over a batch's many tiles.
-inline bool start_early(long long ctas) { return 5 * ctas <= 2 * sm_count() || ctas >= 8 * sm_count(); }
 inline bool capturing(cudaStream_t st)
 {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -71,7 +72,8 @@ inline bool capturing(cudaStream_t st)
     return true;
 }
 template <typename... P, typename... A>
-cudaError_t launch_after(bool early, void (*k)(P...), dim3 grid, size_t smem, cudaStream_t st, const A&... args)
+cudaError_t launch_after(bool direct, bool captured, void (*k)(P...), dim3 grid, size_t smem, cudaStream_t st,
+                         const A&... args)
 {
     cudaLaunchConfig_t lc{};
     lc.gridDim = grid;
@@ -82,8 +84,15 @@ cudaError_t launch_after(bool early, void (*k)(P...), dim3 grid, size_t smem, cu
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     lc.attrs = &at;
-    lc.numAttrs = early && !capturing(st) ? 1 : 0;
+    lc.numAttrs = (direct != captured && capturing(st) ? captured : direct) ? 1 : 0;
     return cudaLaunchKernelEx(&lc, k, args...);
+}
+template <typename... P, typename... A>
+cudaError_t launch_tiles(void (*k)(P...), dim3 grid, size_t smem, cudaStream_t st, const A&... args)
+{
+    const long long ctas = (long long)grid.x * grid.y;
+    return launch_after(2 * ctas <= sm_count() || ctas >= 8 * sm_count(), 5 * ctas <= 2 * sm_count(), k, grid, smem, st,
+                        args...);
 }
 
 // launch=false only raises the kernel's dynamic shared-memory limit, which
@@ -124,14 +133,14 @@ int launch_step_t(const StepParams& P, cudaStream_t st, bool launch)
         if (tiles < (FLUX == 2 ? 8LL : 2LL) * sm_count()) {
             dim3 grid((P.N + kSZ - 1) / kSZ, band);
             if (P.band_hi > 0) Q.units = (int)grid.x * rows;
-            e = launch_after(start_early((long long)grid.x * grid.y), step_kernel<R, FLUX, RECON, LAYOUT, kSZ, kSR>, grid,
-                             tile_smem_bytes<R, FLUX, kSZ, kSR>(), st, Q);
+            e = launch_tiles(step_kernel<R, FLUX, RECON, LAYOUT, kSZ, kSR>, grid, tile_smem_bytes<R, FLUX, kSZ, kSR>(), st,
+                             Q);
             return e == cudaSuccess ? AST_OK : cuda_fail(e, "step kernel launch");
         }
     }
     dim3 grid((P.N + kTZ - 1) / kTZ, band);
     if (P.band_hi > 0) Q.units = (int)grid.x * rows;
-    e = launch_after(start_early((long long)grid.x * grid.y), k, grid, smem, st, Q);
+    e = launch_tiles(k, grid, smem, st, Q);
     return e == cudaSuccess ? AST_OK : cuda_fail(e, "step kernel launch");
 }
 
@@ -151,14 +160,18 @@ int launch_tma_t(const StepParams& P, const CUtensorMap& tin, const CUtensorMap&
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k, kThreads, smem);
         return e == cudaSuccess ? AST_OK : cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
     }
-    // early from 3.5 tiles a CTA, where a late CTA's tiles go to the others (FP32
-    // HLLC wind 1537x771, 3.9 tiles a CTA, 39.9 -> 39.5 us per step, FP64 HLL
-    // 1500x750, 7.3, 120.9 -> 118.0; but FP32 HLL blast 1280x640, 2.6, 23.5 ->
-    // 24.9, and 1024x512, 1.7, 22.0 -> 26.4), and on half the SMs at most (FP32 HLL
-    // 256x128, 64 CTAs, 18.8 -> 16.6; 512x256, 256 CTAs, 17.1 -> 17.9)
+    // early with more tiles than CTAs, whose places are all filled the same: FP64
+    // HLLC wind 712x327 1338 -> 1287 us for twelve steps, FP32 exact solver 800x400
+    // 28.3 -> 26.5 us per step, HLLC wind 1537x771 39.9 -> 39.5 (FP32 HLL blasts of 1 to
+    // 3 tiles a CTA lose: 1024x512 22.0 -> 26.4).  Captured, FP64 so too (700x350 HLL
+    // grown 84.5 -> 82.4, blast 74.5 -> 79.5), FP32 not: HLL 1024x512 18.5 -> 24.9, HLLC
+    // wind 1537x771 36.8 -> 37.8, learned start 4096x2048 107.4 -> 109.5.  On half the SMs
+    // at most, always: FP32 HLL 256x128 (64 CTAs) 18.8 -> 16.6, captured 64x32 15.1 ->
+    // 13.9, 512x256 (256 CTAs) 17.1 -> 17.9.
     const int rows = P.band_hi > 0 ? P.band_hi - P.band_lo : (P.M + kTmaTR - 1) / kTmaTR;
     const long long tiles = (long long)((P.N + kTmaTZ - 1) / kTmaTZ) * rows;
-    e = launch_after(2 * tiles >= 7LL * grid || 2 * grid <= sm_count(), k, grid, smem, st, P, tin, tout);
+    const bool small = 2 * grid <= sm_count(), many = tiles > grid;
+    e = launch_after(small || many, small || (many && sizeof(R) == 8), k, grid, smem, st, P, tin, tout);
     return e == cudaSuccess ? AST_OK : cuda_fail(e, "persistent step kernel launch");
 }
 
